@@ -754,149 +754,411 @@ __global__ void cholesky_kernel(int p, const double* __restrict__ sigma,
 struct ResampleHdr {
     int total;        // number of copied rows (Σ counts)
     int first_src;    // source row of output row 0
-    unsigned done;    // blocks of counts_rank_kernel finished
-    int pad;
+    int pad[2];
 };
 
-// sequential FP64 partial sums, as itertools.accumulate (COV.py:242-251)
-// The additions stay strictly sequential (the reference's accumulation order, so the edges
-// are bit-exact); one warp streams w through a shared-memory double buffer so that lane 0's
-// chain of dependent additions never waits on global-memory latency.
-constexpr int kCdfChunk = 1024;
-__global__ void __launch_bounds__(32) cdf_kernel(const double* __restrict__ w, int n,
-                                                 double* __restrict__ edges) {
-    __shared__ double buf[2][kCdfChunk];
-    if (blockIdx.x != 0) return;
-    const int lane = threadIdx.x;
-    const int nchunks = (n + kCdfChunk - 1) / kCdfChunk;
-    auto load = [&](int c) {
-        const int base = c * kCdfChunk;
-        for (int k = lane; k < kCdfChunk; k += 32) buf[c & 1][k] = (base + k < n) ? w[base + k] : 0.0;
-    };
-    double acc = 0.0;
-    if (lane == 0) edges[0] = 0.0;
-    if (nchunks > 0) load(0);
-    __syncwarp();
-    for (int c = 0; c < nchunks; ++c) {
-        if (c + 1 < nchunks) load(c + 1);            // the next chunk streams in meanwhile
-        if (lane == 0) {
-            const int base = c * kCdfChunk, len = min(kCdfChunk, n - base);
-            const double* b = buf[c & 1];
-            for (int k = 0; k < len; ++k) {
-                acc += b[k];
-                edges[base + k + 1] = acc;
-            }
-        }
-        __syncwarp();
-    }
+// Sequential FP64 partial sums, as itertools.accumulate (COV.py:242-251): edges[i + 1] =
+// fl(edges[i] + w[i]), bit for bit, without the chain of dependent additions (67 cycles each:
+// 1,326 µs for 32,768 weights, measured).
+//
+// While the running sum stays in one binade, [2^e, 2^(e+1)) with unit u = 2^(e-52) in the last
+// place, it is an integer multiple S u of u, 2^52 <= S < 2^53, and adding w rounds to S + q with
+// q = w/u rounded to the nearest integer: the same q whatever S, except when w/u lies exactly
+// between two integers, where the even sum is taken and q depends on the parity of S alone.
+// So an addition is a map S -> S + (S even ? a0 : a1), such maps compose into maps of the same
+// form, and a tile of additions is one parallel scan in 64-bit integers.  The first addition
+// that leaves the binade (or meets a negative or non-finite weight) is done in FP64 and the scan
+// starts again behind it; the binade then grows by at least one, so a sum of n positive
+// weights restarts about log2(n) times after the first kCdfHead weights, which one thread adds.
+// Below 2^-1021 (zeros and subnormals included) the unit is 2^-1074 and the same holds.
+// A tie needs the dropped bits of w to be exactly a half, once in 2^s weights for a shift of s
+// bits, so most warps see none and scan plain sums; the pair of increments is carried only by
+// the warps that do and between the warps.  What bounds the kernel is the integer work of the
+// restarts on one SM: short tiles by one warp up to kCdfWarpEnd weights, where most restarts
+// fall, then tiles of kCdfTile by the whole block.  Measured: 32,768
+// weights 71 µs (1,326 µs with the additions in a row), 1,024 weights 17 µs (43 µs).
+constexpr int kCdfThreads = 512;
+constexpr int kCdfPer = 8;
+constexpr int kCdfTile = kCdfThreads * kCdfPer;
+constexpr int kCdfHead = 16;
+constexpr int kCdfWarpPer = 4;
+constexpr int kCdfWarpEnd = 1024;
+constexpr uint64_t kCdfBig = 1ull << 58;       // saturation: anything >= 2^53 leaves the binade
+
+struct CdfAdd { uint64_t a0, a1; };            // increment of an even and of an odd sum
+
+__device__ __forceinline__ CdfAdd cdf_then(CdfAdd f, CdfAdd g) {
+    const uint64_t r0 = f.a0 + ((f.a0 & 1) ? g.a1 : g.a0);
+    const uint64_t r1 = f.a1 + ((f.a1 & 1) ? g.a0 : g.a1);
+    return {r0 < kCdfBig ? r0 : kCdfBig, r1 < kCdfBig ? r1 : kCdfBig};
 }
 
-// base[v] = Σ_{v' > v} v'·hist[v'] (reverse exclusive scan) then stable ranks within
-// equal counts: start_i = base[c_i] + c_i · #{k < i : c_k = c_i}.  One CTA of 1024 threads.
-constexpr int kRankCache = 4096;
-__device__ void rank_counts(int n, const int* __restrict__ counts, int* __restrict__ hist, int* __restrict__ base,
-                            int* __restrict__ seen, int* __restrict__ start, ResampleHdr* __restrict__ hdr) {
-    __shared__ int warp_tot[32];
-    __shared__ int carry;
-    __shared__ int s_seen[kRankCache];
-    if (threadIdx.x == 0) carry = 0;
-    for (int k = threadIdx.x; k < kRankCache; k += blockDim.x) s_seen[k] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // values n .. 0 in chunks of blockDim, processed from high to low
-    for (int top = n; top >= 0; top -= (int)blockDim.x) {
-        const int v = top - (int)threadIdx.x;
-        const int x = (v >= 1) ? v * __ldcg(hist + v) : 0;
-        // inclusive scan inside the block in thread order (= decreasing v)
-        int s = x;
+// the addition of weight w to a sum of binade e (e = -1022 also covers the subnormals)
+__device__ __forceinline__ CdfAdd cdf_add(double w, int e) {
+    const uint64_t bits = (uint64_t)__double_as_longlong(w);
+    if ((bits << 1) == 0) return {0, 0};
+    const int x = (int)(bits >> 52);           // sign and exponent
+    if (x >= 0x7ff) return {kCdfBig, kCdfBig};
+    const uint64_t m = (bits & 0xFFFFFFFFFFFFFull) | (x ? 1ull << 52 : 0ull);
+    const int s = e - (x ? x - 1023 : -1022);
+    if (s < 0) return {kCdfBig, kCdfBig};
+    if (s == 0) return {m, m};
+    if (s > 53) return {0, 0};                 // below half a unit
+    const uint64_t q = m >> s, rem = m & ((1ull << s) - 1), half = 1ull << (s - 1);
+    if (rem == half) return {q + (q & 1), q + ((q + 1) & 1)};
+    return {q + (rem > half), q + (rem > half)};
+}
+
+// S u as a double (S < 2^53; S >= 2^52 unless e = -1022)
+__device__ __forceinline__ double cdf_value(uint64_t S, int e) {
+    return __longlong_as_double((long long)(S >> 52 ? ((uint64_t)(e + 1023) << 52) | (S & 0xFFFFFFFFFFFFFull) : S));
+}
+
+// the sum acc as S and e; false if it is negative or not finite
+__device__ __forceinline__ bool cdf_split(double acc, uint64_t& S, int& e) {
+    const uint64_t bits = (uint64_t)__double_as_longlong(acc);
+    const int x = (int)(bits >> 52);
+    if (x >= 0x7ff && bits != 1ull << 63) return false;
+    e = (x & 0x7ff) ? x - 1023 : -1022;
+    S = (bits & 0xFFFFFFFFFFFFFull) | ((x & 0x7ff) ? 1ull << 52 : 0ull);
+    return true;
+}
+
+// this lane's PER additions (f), the map of the lanes before it (pre) and of the whole warp (all)
+template <int PER>
+__device__ __forceinline__ void cdf_warp_scan(const double (&v)[PER], int e, int lane, CdfAdd (&f)[PER], CdfAdd& pre,
+                                              CdfAdd& all) {
+    CdfAdd tot{0, 0};
+    bool tie = false;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        f[k] = cdf_add(v[k], e);
+        tie |= f[k].a0 != f[k].a1;
+    }
+    if (!__any_sync(0xffffffffu, tie)) {
+        // 32 PER increments below 2^53 stay below 2^61; a saturated one (2^58) may be among them
+        uint64_t t = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) t += f[k].a0;
+        t = t < kCdfBig ? t : kCdfBig;
+        uint64_t s = t;
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += t;
+            const uint64_t p = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += p;
         }
-        if (lane == 31) warp_tot[warp] = s;
-        __syncthreads();
-        if (warp == 0) {
-            int wt = warp_tot[lane];
-            for (int o = 1; o < 32; o <<= 1) {
-                int t = __shfl_up_sync(0xffffffffu, wt, o);
-                if (lane >= o) wt += t;
+        pre.a0 = pre.a1 = s - t < kCdfBig ? s - t : kCdfBig;
+        s = __shfl_sync(0xffffffffu, s, 31);
+        all.a0 = all.a1 = s < kCdfBig ? s : kCdfBig;
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) tot = cdf_then(tot, f[k]);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const CdfAdd p{__shfl_up_sync(0xffffffffu, tot.a0, o), __shfl_up_sync(0xffffffffu, tot.a1, o)};
+        if (lane >= o) tot = cdf_then(p, tot);
+    }
+    pre = CdfAdd{__shfl_up_sync(0xffffffffu, tot.a0, 1), __shfl_up_sync(0xffffffffu, tot.a1, 1)};
+    if (lane == 0) pre = CdfAdd{0, 0};
+    all = CdfAdd{__shfl_sync(0xffffffffu, tot.a0, 31), __shfl_sync(0xffffffffu, tot.a1, 31)};
+}
+
+// this thread's edges from the sum S before its first weight (index i0): those inside the binade
+// (the sums only grow, so the others come after them).  True where this thread holds the tile's
+// new position and sum: behind the first addition that leaves the binade, or at the tile's end.
+template <int PER>
+__device__ __forceinline__ bool cdf_apply(const double (&v)[PER], const CdfAdd (&f)[PER], uint64_t S, int e, int i0,
+                                          int end, double* __restrict__ edges, int& pos, double& acc) {
+    int last = -1;                             // the first of my sums outside the binade
+    uint64_t at = 0;
+    double left = 0.0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        if (i0 + k >= end) break;
+        const uint64_t next = S + ((S & 1) ? f[k].a1 : f[k].a0);
+        if ((next >> 53) == 0) {
+            edges[i0 + k + 1] = cdf_value(next, e);
+        } else if ((S >> 53) == 0) {
+            last = k;
+            at = S;
+            left = v[k];
+        }
+        S = next;
+    }
+    if (last >= 0) {
+        pos = i0 + last + 1;
+        acc = cdf_value(at, e) + left;
+        edges[pos] = acc;
+        return true;
+    }
+    if ((S >> 53) || i0 >= end || i0 + PER < end) return false;
+    pos = end;
+    acc = cdf_value(S, e);
+    return true;
+}
+
+// one CTA; also clears the counts that the next kernel adds to
+__global__ void __launch_bounds__(kCdfThreads) cdf_kernel(const double* __restrict__ w, int n,
+                                                          double* __restrict__ edges, int* __restrict__ counts) {
+    __shared__ CdfAdd s_warp[kCdfThreads / 32];
+    __shared__ double s_w[kCdfWarpEnd];
+    __shared__ double s_acc;
+    __shared__ int s_pos;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int stop = n < kCdfWarpEnd ? n : kCdfWarpEnd;
+    for (int i = tid; i < stop; i += kCdfThreads) s_w[i] = w[i];
+    __syncthreads();
+    if (warp == 0) {
+        int pos = n < kCdfHead ? n : kCdfHead;
+        double acc = 0.0;
+        if (lane == 0) {
+            edges[0] = 0.0;
+            for (int i = 0; i < pos; ++i) {
+                acc += s_w[i];
+                edges[i + 1] = acc;
             }
-            warp_tot[lane] = wt;
         }
+        acc = __shfl_sync(0xffffffffu, acc, 0);
+        uint64_t S;
+        int e;
+        while (pos < stop && cdf_split(acc, S, e)) {
+            const int end = stop - pos < 32 * kCdfWarpPer ? stop : pos + 32 * kCdfWarpPer;
+            const int i0 = pos + lane * kCdfWarpPer;
+            double v[kCdfWarpPer];
+            CdfAdd f[kCdfWarpPer], pre, all;
+#pragma unroll
+            for (int k = 0; k < kCdfWarpPer; ++k) v[k] = i0 + k < end ? s_w[i0 + k] : 0.0;
+            cdf_warp_scan(v, e, lane, f, pre, all);
+            const bool mine = cdf_apply(v, f, S + ((S & 1) ? pre.a1 : pre.a0), e, i0, end, edges, pos, acc);
+            const int from = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+            pos = __shfl_sync(0xffffffffu, pos, from);
+            acc = __shfl_sync(0xffffffffu, acc, from);
+        }
+        if (lane == 0) {
+            s_acc = acc;
+            s_pos = pos;
+        }
+    } else {
+        for (int i = tid - 32; i < n; i += kCdfThreads - 32) counts[i] = 0;
+    }
+    __syncthreads();
+    for (;;) {
+        int pos = s_pos;
+        double acc = s_acc;
+        if (pos >= n) return;
+        uint64_t S;
+        int e;
+        if (!cdf_split(acc, S, e)) {           // a negative or non-finite sum: plain additions
+            if (tid == 0) {
+                for (int i = pos; i < n; ++i) {
+                    acc += w[i];
+                    edges[i + 1] = acc;
+                }
+            }
+            return;
+        }
+        const int end = n - pos < kCdfTile ? n : pos + kCdfTile;
+        const int i0 = pos + tid * kCdfPer;
+        double v[kCdfPer];
+        CdfAdd f[kCdfPer], pre, all;
+#pragma unroll
+        for (int k = 0; k < kCdfPer; ++k) v[k] = i0 + k < end ? __ldg(w + i0 + k) : 0.0;
+        cdf_warp_scan(v, e, lane, f, pre, all);
+        if (lane == 0) s_warp[warp] = all;
         __syncthreads();
-        const int before = carry + (warp > 0 ? warp_tot[warp - 1] : 0) + s - x;
-        if (v >= 0) base[v] = before;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += warp_tot[31];
+        if (warp > 0) {
+            // the warps before this one, in order: lane l takes warp l's map
+            CdfAdd t = lane < warp ? s_warp[lane] : CdfAdd{0, 0};
+#pragma unroll
+            for (int o = 1; o < kCdfThreads / 32; o <<= 1) {
+                const CdfAdd p{__shfl_up_sync(0xffffffffu, t.a0, o), __shfl_up_sync(0xffffffffu, t.a1, o)};
+                if (lane >= o) t = cdf_then(p, t);
+            }
+            t = CdfAdd{__shfl_sync(0xffffffffu, t.a0, kCdfThreads / 32 - 1),
+                       __shfl_sync(0xffffffffu, t.a1, kCdfThreads / 32 - 1)};
+            pre = cdf_then(t, pre);
+        }
+        if (cdf_apply(v, f, S + ((S & 1) ? pre.a1 : pre.a0), e, i0, end, edges, pos, acc)) {
+            s_acc = acc;
+            s_pos = pos;
+        }
         __syncthreads();
     }
-    if (threadIdx.x == 0) hdr->total = carry;
-    // stable ranks: warp 0 walks the chains in order
-    if (warp != 0) return;
-    int first = -1;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
-        const int c = (i < n) ? __ldcg(counts + i) : 0;
-        const unsigned peers = __match_any_sync(0xffffffffu, c);
-        const int leader = __ffs(peers) - 1;
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        int old = 0;
-        if (lane == leader && c > 0) {
-            if (c < kRankCache) { old = s_seen[c]; s_seen[c] = old + __popc(peers); }
-            else { old = seen[c]; seen[c] = old + __popc(peers); }
-        }
-        old = __shfl_sync(0xffffffffu, old, leader);
-        if (c > 0) {
-            const int st = base[c] + c * (old + rank);
-            start[i] = st;
-            if (st == 0) first = i;
-        } else if (i < n) {
-            start[i] = -1;
-        }
-        __syncwarp();
-    }
-    for (int o = 16; o > 0; o >>= 1) first = max(first, __shfl_xor_sync(0xffffffffu, first, o));
-    if (lane == 0) hdr->first_src = first;
 }
 
 // counts[i] = #{j : edges[i] <= r_j < edges[i+1]}; r_j >= edges[n] dropped (gsl_histogram).
-// One thread per uniform; the last block to finish (threadfence reduction: the block count is
-// cleared before the launch) forms the histogram of the counts and the ranks.
-__global__ void __launch_bounds__(1024) counts_rank_kernel(int n, uint64_t seed, const uint32_t* __restrict__ epoch,
-                                                           const double* __restrict__ edges, int* __restrict__ counts,
-                                                           int* __restrict__ hist, int* __restrict__ base,
-                                                           int* __restrict__ seen, int* __restrict__ start,
-                                                           ResampleHdr* __restrict__ hdr, unsigned* __restrict__ done) {
+// One thread per uniform.
+__global__ void __launch_bounds__(256) counts_kernel(int n, uint64_t seed, const uint32_t* __restrict__ epoch,
+                                                     const double* __restrict__ edges, int* __restrict__ counts) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) {
-        u32x4 r = draw(seed, (uint32_t)j, 0u, STREAM_RESAMPLE, 0u, *epoch);
-        const double x = u01_closed_open(r.x, r.y);
-        if (x >= edges[0] && x < edges[n]) {
-            // largest i with edges[i] <= x
-            int lo = 0, hi = n;          // edges[lo] <= x < edges[hi]
-            while (hi - lo > 1) {
-                int mid = (lo + hi) >> 1;
-                if (x >= edges[mid]) lo = mid; else hi = mid;
-            }
-            atomicAdd(&counts[lo], 1);
-        }
+    if (j >= n) return;
+    u32x4 r = draw(seed, (uint32_t)j, 0u, STREAM_RESAMPLE, 0u, *epoch);
+    const double x = u01_closed_open(r.x, r.y);
+    if (!(x >= edges[0] && x < edges[n])) return;
+    // largest i with edges[i] <= x
+    int lo = 0, hi = n;          // edges[lo] <= x < edges[hi]
+    while (hi - lo > 1) {
+        int mid = (lo + hi) >> 1;
+        if (x >= edges[mid]) lo = mid; else hi = mid;
     }
-    __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int c = __ldcg(counts + i);
-        if (c > 0) atomicAdd(&hist[c], 1);
-    }
-    __threadfence_block();
-    __syncthreads();
-    rank_counts(n, counts, hist, base, seen, start, hdr);
+    atomicAdd(&counts[lo], 1);
 }
 
+// start[i] = first output row of chain i's copies: rows in order of decreasing count, ties by
+// increasing index.  One CTA; each thread owns kRankPer consecutive chains of a chunk and one
+// column of counters per small count (s_col[c][thread], column 0 for the counts of kRankSmall
+// and more), so a thread's chains come in order, a scan over the threads of each column gives the
+// stable ranks, and no two threads share a counter.  The few chains with large counts (at most
+// n/kRankSmall, since the counts add up to at most n) are ranked against each other.  Counts
+// and results pass through shared memory so that global accesses are coalesced, and only as many
+// columns as the chains need are cleared and scanned.  Measured:
+// 32,768 chains 22 µs (375 µs with one warp walking the chains in order), 1,024 chains 9 µs.
+constexpr int kRankThreads = 1024;
+constexpr int kRankPer = 32;
+constexpr int kRankSmall = 32;
+constexpr int kRankChunk = kRankThreads * kRankPer;
+constexpr size_t kRankSmem = (size_t)kRankChunk * sizeof(int) + (size_t)kRankSmall * kRankThreads * sizeof(uint16_t);
+
+__global__ void __launch_bounds__(kRankThreads) rank_kernel(int n, const int* __restrict__ counts,
+                                                            int* __restrict__ big_row, int* __restrict__ big_cnt,
+                                                            int* __restrict__ start, ResampleHdr* __restrict__ hdr) {
+    extern __shared__ int s_chunk[];               // [kRankThreads][kRankPer]
+    uint16_t* s_col = reinterpret_cast<uint16_t*>(s_chunk + kRankChunk);     // [kRankSmall][kRankThreads]
+    __shared__ int s_tot[kRankSmall], s_base[kRankSmall], s_seen[kRankSmall];
+    __shared__ int s_bigsum;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int threads = n < kRankChunk ? ((n + kRankPer - 1) / kRankPer + 31) / 32 * 32 : kRankThreads;
+    const bool owner = tid < threads;
+    uint16_t* col = s_col + tid;
+    // chain k of thread t lies at word t kRankPer + (k ^ (t mod 32)): no bank conflicts by row or column
+    auto word = [](int i) { return (i & ~31) | ((i ^ (i >> 5)) & 31); };
+    auto clear = [&]() {
+        for (int v = warp; v < kRankSmall; v += 32)
+            for (int k = lane * 2; k < threads; k += 64) *reinterpret_cast<uint32_t*>(s_col + v * kRankThreads + k) = 0u;
+    };
+    int c[kRankPer];
+    auto load = [&](long c0) {
+        const int len = n - c0 < kRankChunk ? (int)(n - c0) : kRankChunk;
+        for (int i = tid; i < threads * kRankPer; i += kRankThreads) s_chunk[word(i)] = i < len ? counts[c0 + i] : 0;
+        __syncthreads();
+        if (owner) {
+#pragma unroll
+            for (int k = 0; k < kRankPer; ++k) c[k] = s_chunk[word(tid * kRankPer + k)];
+        }
+    };
+    auto tally = [&]() {
+        int big = 0;
+        if (owner) {
+#pragma unroll
+            for (int k = 0; k < kRankPer; ++k) {
+                if (c[k] <= 0) continue;
+                const int v = c[k] < kRankSmall ? c[k] : 0;
+                col[v * kRankThreads] += 1;
+                if (v == 0) big += c[k];
+            }
+        }
+        return big;
+    };
+    int total = 0;                                 // warp v: chains with count v so far
+    auto add_columns = [&]() {
+        int t = 0;
+        for (int k = lane; k < threads; k += 32) t += s_col[warp * kRankThreads + k];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        total += t;
+    };
+    clear();
+    if (tid == 0) {
+        s_bigsum = 0;
+        hdr->first_src = -1;
+    }
+    // totals per count over all chunks, each thread in its own column
+    for (long c0 = 0; c0 < n; c0 += kRankChunk) {
+        if (c0 > 0) {
+            __syncthreads();
+            clear();
+        }
+        load(c0);
+        const int big = tally();
+        if (big) atomicAdd(&s_bigsum, big);
+        __syncthreads();
+        add_columns();
+    }
+    if (lane == 0) s_tot[warp] = total;
+    __syncthreads();
+    if (warp == 0) {
+        // base[v] = Σ_{v' > v} v' chains(v') (lane v), behind the large counts
+        int x = lane * s_tot[lane], s = x;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_down_sync(0xffffffffu, s, o);
+            if (lane + o < 32) s += t;
+        }
+        s_base[lane] = s_bigsum + s - x;
+        s_seen[lane] = 0;
+        if (lane == 0) hdr->total = s_bigsum + s;
+    }
+    for (long c0 = 0; c0 < n; c0 += kRankChunk) {
+        if (n > kRankChunk) {
+            // the columns hold the last chunk's counts: this chunk's alone again
+            __syncthreads();
+            clear();
+            load(c0);
+            tally();
+        }
+        __syncthreads();
+        // exclusive scan of column `warp` over the threads, behind the earlier chunks' chains
+        int carry = 0;
+        for (int k = 0; k < threads; k += 32) {
+            uint16_t* at = s_col + warp * kRankThreads + k + lane;
+            const int v = *at;
+            int s = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, s, o);
+                if (lane >= o) s += t;
+            }
+            *at = (uint16_t)(carry + s - v);
+            carry += __shfl_sync(0xffffffffu, s, 31);
+        }
+        __syncthreads();
+        if (owner) {
+            const long i0 = c0 + tid * kRankPer;
+#pragma unroll
+            for (int k = 0; k < kRankPer; ++k) {
+                int st = -1;
+                if (c[k] > 0) {
+                    const int v = c[k] < kRankSmall ? c[k] : 0;
+                    const int rank = s_seen[v] + col[v * kRankThreads]++;
+                    if (v == 0) {
+                        big_row[rank] = (int)(i0 + k);
+                        big_cnt[rank] = c[k];
+                    } else {
+                        st = s_base[v] + v * rank;
+                        if (st == 0) hdr->first_src = (int)(i0 + k);
+                    }
+                }
+                s_chunk[word(tid * kRankPer + k)] = st;
+            }
+        }
+        __syncthreads();
+        const int len = n - c0 < kRankChunk ? (int)(n - c0) : kRankChunk;
+        for (int i = tid; i < len; i += kRankThreads) start[c0 + i] = s_chunk[word(i)];
+        if (lane == 0) s_seen[warp] += carry;
+    }
+    __syncthreads();
+    const int nbig = s_tot[0];
+    for (int a = tid; a < nbig; a += kRankThreads) {
+        const int ca = big_cnt[a];
+        int st = 0;
+        for (int b = 0; b < nbig; ++b) {
+            const int cb = big_cnt[b];
+            st += (cb > ca || (cb == ca && b < a)) ? cb : 0;
+        }
+        start[big_row[a]] = st;
+        if (st == 0) hdr->first_src = big_row[a];
+    }
+}
+
+// one thread per element of θ, so that consecutive threads copy consecutive parameters
 __global__ void gather_kernel(int n, int p, const double* __restrict__ beta,
                               const int* __restrict__ counts, const int* __restrict__ start,
                               const ResampleHdr* __restrict__ hdr,
@@ -904,29 +1166,26 @@ __global__ void gather_kernel(int n, int p, const double* __restrict__ beta,
                               const double* __restrict__ da_in, double* __restrict__ th_out,
                               double* __restrict__ pr_out, double* __restrict__ da_out,
                               double* __restrict__ po_out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(t / p), j = (int)(t - (long)i * p);
     if (i >= n) return;
     const double b = *beta;
-    const int c = counts[i];
-    if (c > 0) {
-        const int s0 = start[i];
+    auto copy = [&](int src, int d0, int c) {
+        const double v = th_in[(size_t)src * p + j];
+        for (int k = 0; k < c; ++k) th_out[(size_t)(d0 + k) * p + j] = v;
+        if (j != 0) return;
+        const double pr = pr_in[src], da = da_in[src];
+        const double po = pr + b * da;
         for (int k = 0; k < c; ++k) {
-            const int d = s0 + k;
-            for (int j = 0; j < p; ++j) th_out[(size_t)d * p + j] = th_in[(size_t)i * p + j];
-            pr_out[d] = pr_in[i];
-            da_out[d] = da_in[i];
-            po_out[d] = pr_in[i] + b * da_in[i];
+            pr_out[d0 + k] = pr;
+            da_out[d0 + k] = da;
+            po_out[d0 + k] = po;
         }
-    }
+    };
+    const int c = counts[i];
+    if (c > 0) copy(i, start[i], c);
     // rows left over when uniforms fell beyond the last edge repeat the first group's row
-    const int d = i;
-    if (d >= hdr->total && hdr->first_src >= 0) {
-        const int src = hdr->first_src;
-        for (int j = 0; j < p; ++j) th_out[(size_t)d * p + j] = th_in[(size_t)src * p + j];
-        pr_out[d] = pr_in[src];
-        da_out[d] = da_in[src];
-        po_out[d] = pr_in[src] + b * da_in[src];
-    }
+    if (i >= hdr->total && hdr->first_src >= 0) copy(hdr->first_src, i, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1187,14 +1446,14 @@ extern "C" int ag_cholesky_scaled(const ag_stage_state* st, int32_t p, void* str
     return launch_status("cholesky_kernel");
 }
 
-// workspace layout: hdr (with the block count of counts_rank_kernel) | edges[n+1] |
-// counts[n] (if not given) | hist[n+1] | base[n+1] | seen[n+1] | start[n]
+// workspace layout: hdr | edges[n+1] | counts[n] (if not given) | rows and counts of the
+// chains with large counts | start[n]
 static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 extern "C" size_t ag_resample_workspace_bytes(int32_t n) {
     if (n <= 0) return 0;
     size_t b = align256(sizeof(ResampleHdr));
     b += align256((size_t)(n + 1) * sizeof(double));
-    b += 5 * align256((size_t)(n + 1) * sizeof(int));
+    b += 4 * align256((size_t)(n + 1) * sizeof(int));
     return b;
 }
 
@@ -1219,24 +1478,19 @@ extern "C" int ag_resample(const ag_stage_state* st, int32_t n, int32_t p, uint6
     ws += align256((size_t)(n + 1) * sizeof(double));
     const size_t ib = align256((size_t)(n + 1) * sizeof(int));
     int* cnt_ws = reinterpret_cast<int*>(ws); ws += ib;
-    int* hist = reinterpret_cast<int*>(ws); ws += ib;
-    int* base = reinterpret_cast<int*>(ws); ws += ib;
-    int* seen = reinterpret_cast<int*>(ws); ws += ib;
+    int* big_row = reinterpret_cast<int*>(ws); ws += ib;
+    int* big_cnt = reinterpret_cast<int*>(ws); ws += ib;
     int* start = reinterpret_cast<int*>(ws); ws += ib;
     int* cnt = counts ? counts : cnt_ws;
-    rc = cuda_status(cudaMemsetAsync(cnt, 0, (size_t)n * sizeof(int), s), "memset counts");
+    rc = cuda_status(cudaFuncSetAttribute(rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRankSmem),
+                     "cudaFuncSetAttribute(rank_kernel)");
     if (rc) return rc;
-    rc = cuda_status(cudaMemsetAsync(hist, 0, (size_t)(n + 1) * sizeof(int), s), "memset hist");
-    if (rc) return rc;
-    rc = cuda_status(cudaMemsetAsync(seen, 0, (size_t)(n + 1) * sizeof(int), s), "memset seen");
-    if (rc) return rc;
-    rc = cuda_status(cudaMemsetAsync(&hdr->done, 0, sizeof(unsigned), s), "memset block count");
-    if (rc) return rc;
-    cdf_kernel<<<1, 32, 0, s>>>(st->w, n, edges);
-    counts_rank_kernel<<<blocks(n, 1024), 1024, 0, s>>>(n, seed, st->epoch, edges, cnt, hist, base, seen, start,
-                                                         hdr, &hdr->done);
-    gather_kernel<<<blocks(n, 128), 128, 0, s>>>(n, p, st->beta, cnt, start, hdr, theta_in, prior_in,
-                                                 data_in, theta_out, prior_out, data_out, post_out);
+    cdf_kernel<<<1, kCdfThreads, 0, s>>>(st->w, n, edges, cnt);
+    counts_kernel<<<blocks(n, 256), 256, 0, s>>>(n, seed, st->epoch, edges, cnt);
+    rank_kernel<<<1, kRankThreads, kRankSmem, s>>>(n, cnt, big_row, big_cnt, start, hdr);
+    gather_kernel<<<(unsigned)(((long)n * p + 255) / 256), 256, 0, s>>>(n, p, st->beta, cnt, start, hdr, theta_in,
+                                                                        prior_in, data_in, theta_out, prior_out,
+                                                                        data_out, post_out);
     return launch_status("resample kernels");
 }
 
