@@ -210,7 +210,7 @@ struct CovState {
     double llk_max;
     double beta0;          // β at the start of the stage
     double low, high, step;
-    double pts[kGridPoints];
+    double pts[2];         // points of the next round (round 0, Brent)
     double cov_high;       // COV at the full remaining δβ
     double dbeta;          // chosen δβ
     double cov;            // COV at dbeta
@@ -225,6 +225,20 @@ struct CovState {
     int phase;             // 0: evaluating the initial point, 1: iterating
 };
 
+// blocks of the schedule kernel for n chains, and the partial sums one round of it writes
+constexpr int kCovBlocks = 152;
+__host__ __device__ constexpr int cov_blocks(int n) {
+    return (n + 255) / 256 < kCovBlocks ? (n + 255) / 256 : kCovBlocks;
+}
+__host__ __device__ constexpr size_t cov_round_partials(int n) {
+    // a grid level's moments per block, or Brent's two points per chunk
+    const size_t level = (size_t)2 * kGridPoints * cov_blocks(n), brent = 4 * (size_t)((n + kEvalChunk - 1) / kEvalChunk);
+    return level > brent ? level : brent;
+}
+__host__ __device__ constexpr size_t cov_part_doubles(int n) {
+    return 2 * cov_round_partials(n) + 2 * (size_t)((n + kEvalChunk - 1) / kEvalChunk);
+}
+
 // order-preserving map of a double onto uint64
 __device__ inline uint64_t dkey(double x) {
     uint64_t b = (uint64_t)__double_as_longlong(x);
@@ -235,58 +249,152 @@ __device__ inline double dkey_inv(uint64_t k) {
     return __longlong_as_double((long long)b);
 }
 
-// k-th smallest (0-based) key of llk by 8-bit radix select; one CTA
-__device__ uint64_t block_select(const double* __restrict__ llk, int n, int k, int* hist,
-                                 int* sh) {
-    uint64_t prefix = 0ull, mask = 0ull;
-    for (int pass = 0; pass < 8; ++pass) {
-        const int shift = 56 - 8 * pass;
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            uint64_t key = dkey(llk[i]);
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255], 1);
+// Median and maximum of llk, one CTA.  The range of the keys that can hold the wanted rank is
+// cut into 2^11 buckets of equal width (in key space), counted in shared memory, and narrowed to
+// one bucket; once a bucket holds at most kMedianList keys they are collected and ranked against
+// each other.  Starting from the keys' own range, the log-likelihoods of a stage take one or two
+// counting passes (a radix select over the fixed bytes of the key took 16): 32,768 values in
+// 23 µs (129 µs), 1,024 in 11 µs (50 µs).  The passes are bound by the latency of reading llk from L2 on one SM.
+constexpr int kMedianThreads = 1024;
+constexpr int kMedianBits = 11;
+constexpr int kMedianList = 128;        // 8 threads rank each key
+
+template <class F>
+__device__ __forceinline__ void median_each(const double* __restrict__ llk, int n, F f) {
+    for (long i0 = threadIdx.x; i0 < n; i0 += 8 * kMedianThreads) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const long i = i0 + (long)q * kMedianThreads;
+            v[q] = i < n ? __ldg(llk + i) : 0.0;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int acc = 0, d = 0;
-            for (; d < 256; ++d) {
-                if (acc + hist[d] > k) break;
-                acc += hist[d];
-            }
-            sh[0] = d;
-            sh[1] = k - acc;
-        }
-        __syncthreads();
-        const int d = sh[0];
-        k = sh[1];
-        prefix |= (uint64_t)d << shift;
-        mask |= 255ull << shift;
-        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (i0 + (long)q * kMedianThreads < n) f(dkey(v[q]));
     }
-    return prefix;
 }
 
-__global__ void __launch_bounds__(1024) cov_median_kernel(const double* __restrict__ llk, int n,
-                                                          const double* __restrict__ beta,
-                                                          CovState* __restrict__ S) {
-    __shared__ int hist[256];
-    __shared__ int sh[2];
-    __shared__ double smax[32];
-    // maximum
-    double mx = -INFINITY;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, llk[i]);
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = mx;
+__device__ inline uint64_t u64_min(uint64_t a, uint64_t b) { return a < b ? a : b; }
+__device__ inline uint64_t u64_max(uint64_t a, uint64_t b) { return a > b ? a : b; }
+
+__global__ void __launch_bounds__(kMedianThreads) cov_median_kernel(const double* __restrict__ llk, int n,
+                                                                    const double* __restrict__ beta,
+                                                                    CovState* __restrict__ S) {
+    __shared__ int s_hist[1 << kMedianBits];
+    __shared__ uint64_t s_list[kMedianList];
+    __shared__ uint64_t s_a[32], s_b[32];
+    __shared__ double s_max[32];
+    __shared__ int s_warp[32];
+    __shared__ uint64_t s_key[2];
+    __shared__ int s_bucket, s_before, s_count, s_fill;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // smallest and largest key; the maximum as fmax has it (NaN left out)
+    uint64_t mn = ~0ull, mx = 0ull;
+    uint64_t big = dkey(-INFINITY);
+    median_each(llk, n, [&](uint64_t k) {
+        mn = u64_min(mn, k);
+        mx = u64_max(mx, k);
+        if (k <= dkey(INFINITY)) big = u64_max(big, k);
+    });
+    double top = dkey_inv(big);
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = u64_min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = u64_max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    if (lane == 0) {
+        s_a[warp] = mn;
+        s_b[warp] = mx;
+        s_max[warp] = top;
+    }
     __syncthreads();
-    // median as gsl_stats_median_from_sorted_data: mean of elements (n-1)/2 and n/2
-    const uint64_t klo = block_select(llk, n, (n - 1) / 2, hist, sh);
-    const uint64_t khi = (n % 2) ? klo : block_select(llk, n, n / 2, hist, sh);
-    if (threadIdx.x == 0) {
-        double m = smax[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, smax[w]);
-        const double lo = dkey_inv(klo), hi = dkey_inv(khi);
-        S->median = (n % 2) ? lo : (lo + hi) / 2.0;
+    uint64_t lo = s_a[lane], hi = s_b[lane];
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = u64_min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = u64_max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    // rank k among the `count` keys in [lo, lo + range]
+    uint64_t range = hi - lo;
+    int k = (n - 1) / 2, count = n;
+    while (range > 0 && count > kMedianList) {
+        const int width = 64 - __clzll((long long)range);
+        const int shift = width > kMedianBits ? width - kMedianBits : 0;
+        for (int b = tid; b < 1 << kMedianBits; b += kMedianThreads) s_hist[b] = 0;
+        __syncthreads();
+        median_each(llk, n, [&](uint64_t key) {
+            if (key - lo <= range) atomicAdd(&s_hist[(key - lo) >> shift], 1);
+        });
+        __syncthreads();
+        // the bucket of rank k: two buckets per thread
+        const int h0 = s_hist[2 * tid], h1 = s_hist[2 * tid + 1];
+        int s = h0 + h1;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        if (lane == 31) s_warp[warp] = s;
+        __syncthreads();
+        int w = lane < warp ? s_warp[lane] : 0;
+        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        const int before = w + s - h0 - h1;
+        if (k >= before && k < before + h0 + h1) {
+            const bool second = k >= before + h0;
+            s_bucket = 2 * tid + second;
+            s_before = before + (second ? h0 : 0);
+            s_count = second ? h1 : h0;
+        }
+        __syncthreads();
+        lo += (uint64_t)s_bucket << shift;
+        range = (1ull << shift) - 1;           // may reach past hi: no keys lie there
+        k -= s_before;
+        count = s_count;
+        __syncthreads();
+    }
+    // klo, the key of rank (n-1)/2; khi, the next one of rank n/2 (gsl_stats_median_from_sorted_data)
+    if (tid == 0) {
+        s_fill = 0;
+        s_key[0] = s_key[1] = lo;
+    }
+    __syncthreads();
+    if (range > 0) {
+        median_each(llk, n, [&](uint64_t key) {
+            if (key - lo <= range) s_list[atomicAdd(&s_fill, 1)] = key;
+        });
+        __syncthreads();
+        const int c = tid >> 3;
+        const uint64_t key = s_list[c < count ? c : 0];
+        int rank = 0;
+        for (int j = tid & 7; j < count; j += 8) {
+            const uint64_t other = s_list[j];
+            rank += other < key || (other == key && j < c);
+        }
+        for (int o = 4; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+        if (c < count) {
+            if (rank == k) s_key[0] = key;
+            if (rank == k + 1) s_key[1] = key;
+        }
+        __syncthreads();
+    }
+    if (n % 2 == 0 && k + 1 >= count) {
+        // the next key lies beyond the bucket
+        uint64_t next = ~0ull;
+        const uint64_t last = lo + range < lo ? ~0ull : lo + range;
+        median_each(llk, n, [&](uint64_t key) {
+            if (key > last) next = u64_min(next, key);
+        });
+        for (int o = 16; o > 0; o >>= 1) next = u64_min(next, __shfl_xor_sync(0xffffffffu, next, o));
+        if (lane == 0) s_a[warp] = next;
+        __syncthreads();
+        if (tid == 0) {
+            for (int j = 1; j < 32; ++j) next = u64_min(next, s_a[j]);
+            s_key[1] = next;
+        }
+    }
+    if (tid == 0) {
+        double m = s_max[0];
+        for (int w = 1; w < 32; ++w) m = fmax(m, s_max[w]);
+        const double vlo = dkey_inv(s_key[0]), vhi = dkey_inv(s_key[1]);
+        S->median = (n % 2) ? vlo : (vlo + vhi) / 2.0;
         S->llk_max = m;
         S->beta0 = *beta;
         S->low = 0.0;
@@ -300,18 +408,16 @@ __global__ void __launch_bounds__(1024) cov_median_kernel(const double* __restri
     }
 }
 
-// shifted weight moments Σe and Σe², e = exp(g (llk − median) − g (llk_max − median)), of one
-// chunk of kEvalChunk chains: 256 threads each sum their chains in index order, then the warps'
-// sums are added in warp order
-__device__ void chunk_moments(const double* __restrict__ llk, int n, double g, double med, double llk_max,
-                              int chunk, double* __restrict__ out) {
+// Σe and Σe² over one chunk of kEvalChunk chains (in thread 0's out): 256 threads each sum their
+// chains in index order, then the warps' sums are added in warp order
+template <class F>
+__device__ void chunk_sums(int n, int chunk, F value, double (&out)[2]) {
     __shared__ double r1[8], r2[8];
-    const double mx = g * (llk_max - med);
     double s1 = 0.0, s2 = 0.0;
     const int begin = chunk * kEvalChunk;
     const int end = min(n, begin + kEvalChunk);
     for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const double e = exp(g * (llk[i] - med) - mx);
+        const double e = value(i);
         s1 += e;
         s2 = fma(e, e, s2);
     }
@@ -334,11 +440,20 @@ __device__ void chunk_moments(const double* __restrict__ llk, int n, double g, d
     __syncthreads();      // r1 and r2 are reused by the next chunk
 }
 
+// the shifted weight moments, e = exp(g (llk − median) − g (llk_max − median)), of one chunk
+__device__ void chunk_moments(const double* __restrict__ llk, int n, double g, double med, double llk_max, int chunk,
+                              double (&out)[2]) {
+    const double mx = g * (llk_max - med);
+    chunk_sums(n, chunk, [&](int i) { return exp(g * (llk[i] - med) - mx); }, out);
+}
+
 // COV of the normalised weights from the shifted moments, with the reference's
 // convention that a non-finite COV counts as 1e100 (COV.cc:355-364)
 __device__ double cov_from_moments(double s1, double s2, double mx, int n) {
-    // an infinite weight in the reference (exp overflow) or an infinite weight sum
-    if (isinf(exp(mx)) || !(s1 > 0.0) || isinf(exp(mx) * s1)) return 1e100;
+    // an infinite weight in the reference (exp overflow) or an infinite weight sum (the sum is at
+    // most n: neither is possible for the small exponents)
+    if (!(s1 > 0.0)) return 1e100;
+    if (mx > 600.0 && (isinf(exp(mx)) || isinf(exp(mx) * s1))) return 1e100;
     double v = (s2 / (s1 * s1) - 1.0 / n) / (double)(n - 1);
     if (v < 0.0) v = 0.0;
     double c = (double)n * sqrt(v);
@@ -346,50 +461,54 @@ __device__ double cov_from_moments(double s1, double s2, double mx, int n) {
     return c;
 }
 
-// One level of the grid search (COV.cc:240-326) given the COVs of this round's points: round 0
-// evaluated the full remaining step, later rounds the kGridPoints points of a level.
-__device__ void grid_step(CovState& S, const double* cov, double target, double tol) {
+// Where the COV of a point lies against the target: 0 at most target - tol, 1 within tol of the
+// target, 2 above.  COV = n sqrt((Σe²/(Σe)² − 1/n)/(n − 1)) >= c is Σe² >= X(c) (Σe)² with
+// X(c) = (c/n)² (n − 1) + 1/n, so a decision takes a product and a comparison where the COV itself
+// takes two divisions and a square root (~4,000 cycles of dependent FP64).
+__device__ double cov_threshold(double c, int n) {
+    const double r = c / (double)n;
+    return c < 0.0 ? -1.0 : r * r * (double)(n - 1) + 1.0 / n;
+}
+
+__device__ int cov_class(double s1, double s2, double mx, double below, double above) {
+    // the reference's 1e100: no weights, an infinite weight or weight sum, a NaN
+    if (!(s1 > 0.0)) return 2;
+    if (mx > 600.0 && (isinf(exp(mx)) || isinf(exp(mx) * s1))) return 2;
+    const double q = s1 * s1;
+    return s2 <= below * q ? 0 : s2 < above * q ? 1 : 2;
+}
+
+// One level of the grid search (COV.cc:240-326): round 0 evaluated the full remaining step (cls is
+// its class), later rounds the kGridPoints points of a level; hit is the first point of the level
+// that is not below the target (kGridPoints if none), cls its class.
+__device__ void grid_step(CovState& S, int hit, int cls) {
     const double Nbeta = 10.0;
     if (S.level == 0) {
         // skip straight to β = 1 (COV.cc:257-268)
-        S.cov_high = cov[0];
-        if (cov[0] < target || fabs(cov[0] - target) < tol) {
+        if (cls < 2) {
             S.done = 1;
             S.skip = 1;
             S.dbeta = S.high;
             return;
         }
     } else {
-        // scan of one level (COV.cc:287-311)
-        bool found = false;
-        int nb = 0;
-        for (; nb < S.npts; ++nb) {
-            if (fabs(cov[nb] - target) < tol) { found = true; break; }
-            if (cov[nb] >= target) { if (nb == 0) found = true; break; }
-        }
+        // scan of one level (COV.cc:287-311); the points are low, low + step, ... accumulated as the
+        // reference does.  A completed scan leaves the reference's accumulator one step past the
+        // last point and steps it back (COV.cc:301), which can differ from that point in the last bit
         const double step = S.step;
-        // a completed scan leaves the reference's accumulator one step past the last
-        // point and steps it back (COV.cc:301), which can differ from that point in the
-        // last bit
-        const double guess = (nb < S.npts) ? S.pts[nb] : (S.pts[S.npts - 1] + step) - step;
+        double guess = S.low;
+        for (int k = 0; k < hit; ++k) guess += step;
+        if (hit == kGridPoints) guess -= step;
         S.high = guess;
         S.low = guess - step;
-        if (found || S.level >= kGridLevels) {
+        if (cls == 1 || hit == 0 || S.level >= kGridLevels) {
             S.done = 1;
             S.dbeta = guess;
             return;
         }
     }
-    // next level: points low, low + step, ... accumulated as the reference does
     S.level += 1;
-    const double step = (S.high - S.low) / Nbeta;
-    S.step = step;
-    double g = S.low;
-    for (int k = 0; k < kGridPoints; ++k) {
-        S.pts[k] = g;
-        g += step;
-    }
-    S.npts = kGridPoints;
+    S.step = (S.high - S.low) / Nbeta;
 }
 
 // Brent's minimiser for δβ (COV.cc:58-219).  The reference minimises f(δβ) = (COV − target)²
@@ -545,14 +664,72 @@ __device__ bool grid_sync(GridBarrier* bar, uint32_t* flags) {
     return s_ok != 0;
 }
 
+// Sum of each of N <= 32 per-lane values over the warp: after the call, v[0] of lane l holds the
+// sum of value l (bit-reversed halving: 31 additions per lane where N butterflies take 5 N)
+template <int N>
+__device__ __forceinline__ void warp_sum_each(double (&v)[N], int lane) {
+    static_assert(N <= 32, "one value per lane");
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double a = i < N ? v[i < N ? i : 0] : 0.0, b = i + h < N ? v[i + h < N ? i + h : 0] : 0.0;
+            const double got = __shfl_xor_sync(0xffffffffu, up ? a : b, h);
+            if (i < N) v[i < N ? i : 0] = (up ? b : a) + got;
+        }
+    }
+}
+
+// Moments Σe and Σe², e = exp(g (llk − llk_max)), of this block's share of the chains at the
+// points of one grid level, pts[k] ≈ low + k step: e at successive points is a geometric
+// sequence, so a chain takes two exponentials and ten products instead of eleven exponentials
+// (FP64: 64 cycles per warp instruction and SM quarter is what bounds a round).  They only choose
+// among the grid points; the COV and the weights reported for the chosen δβ come from
+// exponentials of their own.
+template <int POINTS>
+__device__ void level_moments(const double* __restrict__ llk, int n, double low, double step, double llk_max,
+                              double* __restrict__ out, int stride) {
+    constexpr int N = 2 * POINTS;
+    __shared__ double s_part[8][N];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double m[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) m[k] = 0.0;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        const double y = llk[i] - llk_max;
+        double e = exp(low * y);
+        const double f = POINTS > 1 ? exp(step * y) : 1.0;
+#pragma unroll
+        for (int k = 0; k < POINTS; ++k) {
+            m[2 * k] += e;
+            m[2 * k + 1] = fma(e, e, m[2 * k + 1]);
+            if (k + 1 < POINTS) e *= f;
+        }
+    }
+    warp_sum_each(m, lane);
+    if (lane < N) s_part[warp][lane] = m[0];
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double a = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) a += s_part[w][threadIdx.x];
+        out[(size_t)threadIdx.x * stride] = a;
+    }
+}
+
 // The whole δβ search of one stage and its weights in one cooperative launch (COV.cc:58-368).
-// Each round, the blocks evaluate the (point, chunk) moments of the round's points, meet at a
-// grid barrier, and then every block adds the partials in chunk order and takes the same
-// decision on its own copy of the search state, so a round needs one barrier.  The partials
-// alternate between two buffers, so a block that starts the next round cannot overwrite
-// partials that a slower block is still adding.  Then the moments at the chosen δβ, one more
-// barrier, and the normalised weights.  Sums and decisions are those of one chunk per CTA and
-// a sequential total over the chunks, whatever the grid size.
+// Each round, the blocks evaluate the moments of the round's points, meet at a grid barrier, and
+// then every block adds the partials in a fixed order and takes the same decision on its own
+// copy of the search state, so a round needs one barrier.  A grid level has one partial per
+// block and moment, spread over the whole GPU; Brent's single points one per chunk of
+// kEvalChunk chains.  The partials alternate between two buffers, so a block that starts the next
+// round cannot overwrite partials that a slower block is still adding.  Then the exponentials at
+// the chosen δβ, their moments per chunk in chunk order, and the normalised weights.
+// With few chains a round is a chain of dependent FP64 instructions (67 cycles each) and the
+// barrier; with many the exponentials add to that.  Measured:
+// 32,768 chains 110 µs (352 µs with eleven exponentials per chain and level and the eleven COVs
+// formed in a row), 1,024 chains 70 µs (177 µs).
 template <bool BRENT>
 __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restrict__ llk, int n, double target,
                                                            double tol, int maxiter, int rounds,
@@ -561,63 +738,108 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
                                                            double* __restrict__ dbeta_cov, double* __restrict__ w,
                                                            uint32_t* __restrict__ flags) {
     __shared__ CovState sS;
-    __shared__ double s_tot[2 * kGridPoints];
-    if (threadIdx.x == 0) sS = *S;        // median, maximum and the first round's point
+    __shared__ double s_tot[2 * kGridPoints], s_limit[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) sS = *S;                // median, maximum and the first round's point
+    if (!BRENT && (tid == 32 || tid == 64)) {
+        const double t = tol > 0.0 ? tol : 0.0;
+        s_limit[tid >> 6] = cov_threshold(tid == 32 ? target - t : target + t, n);
+    }
     __syncthreads();
     const int nblk = (n + kEvalChunk - 1) / kEvalChunk;
-    const size_t pbuf = (size_t)kGridPoints * nblk * 2;
+    const size_t pbuf = cov_round_partials(n);
     const double med = sS.median, lmax = sS.llk_max;
     for (int round = 0; round < rounds && !sS.done; ++round) {
         double* pr = part + (size_t)(round & 1) * pbuf;
-        const int npts = sS.npts;
-        for (int it = blockIdx.x; it < npts * nblk; it += gridDim.x) {
-            const int pt = it / nblk, c = it - pt * nblk;
-            chunk_moments(llk, n, sS.pts[pt], med, lmax, c, pr + ((size_t)pt * nblk + c) * 2);
-        }
-        if (!grid_sync(bar, flags)) return;
-        if ((int)threadIdx.x < 2 * npts) {
-            const int pt = threadIdx.x >> 1, m = threadIdx.x & 1;
-            double a = 0.0;
-            for (int k = 0; k < nblk; ++k) a += __ldcg(pr + ((size_t)pt * nblk + k) * 2 + m);
-            s_tot[threadIdx.x] = a;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double cov[kGridPoints];
-            for (int pt = 0; pt < npts; ++pt)
-                cov[pt] = cov_from_moments(s_tot[2 * pt], s_tot[2 * pt + 1], sS.pts[pt] * (lmax - med), n);
-            if (BRENT)
-                brent_step(sS, cov, target, tol, maxiter);
+        if constexpr (!BRENT) {
+            const int points = round == 0 ? 1 : kGridPoints, parts = gridDim.x;
+            const double low = sS.low, step = sS.step;
+            if (round == 0)
+                level_moments<1>(llk, n, sS.high, 0.0, lmax, pr + blockIdx.x, parts);
             else
-                grid_step(sS, cov, target, tol);
+                level_moments<kGridPoints>(llk, n, low, step, lmax, pr + blockIdx.x, parts);
+            if (!grid_sync(bar, flags)) return;
+            // eight lanes per moment
+            const int q = tid >> 3;
+            double a = 0.0;
+            if (q < 2 * points) {
+#pragma unroll 4
+                for (int k = tid & 7; k < parts; k += 8) a += __ldcg(pr + (size_t)q * parts + k);
+            }
+            for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (q < 2 * points && (tid & 7) == 0) s_tot[q] = a;
+            __syncthreads();
+            if (warp == 0) {
+                int cls = 0;
+                if (lane < points) {
+                    const double g = round == 0 ? sS.high : low + lane * step;
+                    cls = cov_class(s_tot[2 * lane], s_tot[2 * lane + 1], g * (lmax - med), s_limit[0], s_limit[1]);
+                }
+                const unsigned up = __ballot_sync(0xffffffffu, cls > 0);
+                const int hit = up ? __ffs(up) - 1 : points;
+                cls = __shfl_sync(0xffffffffu, cls, hit & 31);
+                if (lane == 0) grid_step(sS, hit, hit < points ? cls : 0);
+            }
+        } else {
+            const int npts = sS.npts;
+            for (int it = blockIdx.x; it < npts * nblk; it += gridDim.x) {
+                const int pt = it / nblk, c = it - pt * nblk;
+                double m[2];
+                chunk_moments(llk, n, sS.pts[pt], med, lmax, c, m);
+                if (tid == 0) {
+                    pr[(size_t)(2 * pt) * nblk + c] = m[0];
+                    pr[(size_t)(2 * pt + 1) * nblk + c] = m[1];
+                }
+            }
+            if (!grid_sync(bar, flags)) return;
+            if (tid < 2 * npts) {
+                double a = 0.0;
+                for (int k = 0; k < nblk; ++k) a += __ldcg(pr + (size_t)tid * nblk + k);
+                s_tot[tid] = a;
+            }
+            __syncthreads();
+            if (tid == 0) {
+                double cov[2];
+                for (int pt = 0; pt < npts; ++pt)
+                    cov[pt] = cov_from_moments(s_tot[2 * pt], s_tot[2 * pt + 1], sS.pts[pt] * (lmax - med), n);
+                brent_step(sS, cov, target, tol, maxiter);
+            }
         }
         __syncthreads();
     }
-    // moments at the chosen δβ, then the state, β, and the normalised weights
+    // the exponentials at the chosen δβ, their moments, then the state, β, and the normalised weights
     double* fp = part + 2 * pbuf;
-    const double g = sS.dbeta;
-    for (int c = blockIdx.x; c < nblk; c += gridDim.x) chunk_moments(llk, n, g, med, lmax, c, fp + 2 * c);
+    const double g = sS.dbeta, mx = g * (lmax - med);
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        w[i] = exp(g * (llk[i] - med) - mx);
     if (!grid_sync(bar, flags)) return;
-    if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int k = 0; k < nblk; ++k) {
-            a += __ldcg(fp + 2 * k);
-            b += __ldcg(fp + 2 * k + 1);
+    for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
+        double m[2];
+        chunk_sums(n, c, [&](int i) { return __ldcg(w + i); }, m);
+        if (threadIdx.x == 0) {
+            fp[2 * c] = m[0];
+            fp[2 * c + 1] = m[1];
         }
-        sS.s1 = a;
-        sS.cov = cov_from_moments(a, b, g * (lmax - med), n);
-        if (blockIdx.x == 0) {
-            *S = sS;
-            // β bookkeeping (COV.cc:264, 323)
-            *beta = sS.skip ? 1.0 : sS.beta0 + sS.dbeta;
-            dbeta_cov[0] = sS.dbeta;
-            dbeta_cov[1] = sS.cov;
-        }
+    }
+    if (!grid_sync(bar, flags)) return;
+    if (threadIdx.x < 2) {
+        double a = 0.0;
+        for (int k = 0; k < nblk; ++k) a += __ldcg(fp + 2 * k + threadIdx.x);
+        s_tot[threadIdx.x] = a;
     }
     __syncthreads();
-    const double s1 = sS.s1, mx = g * (lmax - med);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        w[i] = exp(g * (llk[i] - med) - mx) / s1;
+    const double s1 = s_tot[0];
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        sS.s1 = s1;
+        sS.cov = cov_from_moments(s1, s_tot[1], mx, n);
+        *S = sS;
+        // β bookkeeping (COV.cc:264, 323)
+        *beta = sS.skip ? 1.0 : sS.beta0 + sS.dbeta;
+        dbeta_cov[0] = sS.dbeta;
+        dbeta_cov[1] = sS.cov;
+    }
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        w[i] = w[i] / s1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1295,10 +1517,9 @@ extern "C" int ag_posterior(const ag_stage_state* st, int32_t n, const double* p
     return launch_status("posterior_kernel");
 }
 
-// COV workspace: schedule state | grid barrier | partial moments (two round buffers of
-// kGridPoints x chunks x 2, then the final chunks x 2)
+// COV workspace: schedule state | grid barrier | partial moments (two round buffers, then the
+// final chunks x 2)
 static size_t cov_part_offset() { return (sizeof(CovState) + 255) / 256 * 256; }
-static size_t cov_part_doubles(int n) { return (size_t)(2 * kGridPoints + 1) * blocks(n, kEvalChunk) * 2; }
 
 extern "C" size_t ag_cov_workspace_bytes(int32_t n) {
     if (n <= 0) return 0;
@@ -1346,8 +1567,9 @@ static int cov_schedule_launch(const ag_stage_state* st, const double* data_llk,
     int grid = 0;
     int rc = cov_coresident_blocks<BRENT>(&grid);
     if (rc) return rc;
-    const int items = kGridPoints * blocks(n, kEvalChunk);
-    if (grid > items) grid = items;
+    // a grid level splits the chains over the GPU; Brent's one or two points have a chunk per block
+    const int want = BRENT ? 2 * blocks(n, kEvalChunk) : cov_blocks(n);
+    if (grid > want) grid = want;
     rc = cuda_status(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), s), "cudaMemsetAsync(COV barrier)");
     if (rc) return rc;
     cov_median_kernel<<<1, 1024, 0, s>>>(data_llk, n, st->beta, S);
@@ -1532,7 +1754,7 @@ constexpr int32_t kNoAllocMaxChains = 1 << 18;
 constexpr size_t kNoAllocState = (sizeof(CovState) + 255) / 256 * 256;
 constexpr size_t kNoAllocBytes =
     kNoAllocState + sizeof(GridBarrier) +
-    (size_t)(2 * kGridPoints + 1) * ((kNoAllocMaxChains + kEvalChunk - 1) / kEvalChunk) * 2 * sizeof(double);
+    cov_part_doubles(kNoAllocMaxChains) * sizeof(double);
 static_assert(kNoAllocState == (sizeof(CovState) + 255) / 256 * 256, "no-alloc layout follows the workspace layout");
 constexpr int kNoAllocMaxDevices = 64;
 

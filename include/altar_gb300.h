@@ -5,7 +5,7 @@
  * comment says otherwise; the library allocates nothing and keeps no global
  * mutable state apart from a per-thread error string, with one exception:
  * ag_cov_schedule_noalloc keeps its scratch in a fixed device array inside the
- * library (about 95 KB per device) and caches that array's address per
+ * library (about 58 KB per device) and caches that array's address per
  * device; the COV schedule entry points cache the co-resident block count of
  * their cooperative kernel per device.  Every call is
  * asynchronous on the given stream (a cudaStream_t passed as void*, NULL =
@@ -288,7 +288,7 @@ int ag_cov_schedule_brent(const ag_stage_state* st, const double* data_llk, int3
  * after start-up, or a loop that must not enter the allocator because cudaMalloc
  * and cudaFree may synchronise the device).  Same inputs and
  * results as ag_cov_schedule without the workspace: the scratch is a fixed
- * device array inside the library (about 95 KB, held by every device that
+ * device array inside the library (about 58 KB, held by every device that
  * loads the library until exit).  Supports at most
  * ag_cov_schedule_noalloc_max_chains() chains (262,144); more returns
  * AG_ERR_SIZE.  All calls share that array: calls that overlap on the GPU
