@@ -843,16 +843,36 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
 }
 
 // ---------------------------------------------------------------------------
-// weighted covariance (COV.py:106-156): per-chunk partial sums in fixed order.  A chunk
-// holds as many chains as fit the shared-memory budget (256 for up to 32 parameters).
-constexpr size_t kSigmaSmem = 96 * 1024;
-static int sigma_chunk(int p) {
-    int c = kSigmaChunk;
-    while (c > 1 && (size_t)c * (p + 1) * sizeof(double) > kSigmaSmem) c >>= 1;
-    return c;
+// weighted covariance (COV.py:106-156): per-block partial sums in fixed order.
+//
+// With x = (1, θ) the sums Σw, Σ w θ_a and Σ w θ_a θ_b are the lower triangle of Σ (w x)(x)ᵀ: one
+// FP64 FMA per entry and chain, the products w x formed once per chain in shared memory.  FP64
+// issue bounds it (64 cycles per warp instruction and SM quarter), so the chains are spread over
+// all SMs (as few as kSigmaMinRows per block, so that few chains still fill them) and, where the
+// entries leave threads over, groups of threads share a block's chains.  Measured, 10
+// parameters: 32,768 chains 24 µs (56 µs with one thread per entry and three instructions per
+// term); 4 parameters, 1,024 chains 8 µs (43 µs).
+constexpr size_t kSigmaSmem = 160 * 1024;
+constexpr int kSigmaBlocks = 152;  // one per SM
+constexpr int kSigmaMinRows = 16;
+static void sigma_grid(int n, int p, int* chunk, int* nblk, int* cpb) {
+    int most = (int)(kSigmaSmem / (2 * (p + 1) * sizeof(double)));
+    if (most > kSigmaChunk) most = kSigmaChunk;
+    const int rows = (n - 1) / kSigmaBlocks + 1;
+    *chunk = rows < kSigmaMinRows ? kSigmaMinRows : rows < most ? rows : most;
+    if (*chunk > most) *chunk = most;
+    const int nchunks = (n - 1) / *chunk + 1;
+    *cpb = (nchunks - 1) / kSigmaBlocks + 1;
+    *nblk = (nchunks - 1) / *cpb + 1;
 }
 
-constexpr int kSigmaBlocks = 256;  // at most this many partial sums per entry
+// entry e of a lower triangle stored by rows: row a starts at a (a + 1) / 2
+__device__ __forceinline__ void triangle_entry(int e, int& a, int& b) {
+    a = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+    while ((a + 1) * (a + 2) / 2 <= e) ++a;
+    while (a * (a + 1) / 2 > e) --a;
+    b = e - a * (a + 1) / 2;
+}
 
 // Block b sums the chunks [b·cpb, (b+1)·cpb) in order into part[b][e]; the last block to
 // finish adds the blocks' partials in block order and assembles Σ.
@@ -860,67 +880,100 @@ __global__ void __launch_bounds__(256) sigma_kernel(const double* __restrict__ t
                                                     const double* __restrict__ w, int n, int p, int chunk,
                                                     int cpb, double* __restrict__ part, double* __restrict__ tot,
                                                     unsigned* __restrict__ done, double* __restrict__ sigma) {
-    extern __shared__ double sm[];      // [chunk][p] θ, then [chunk] w
-    double* sth = sm;
-    double* sw = sm + (size_t)chunk * p;
-    // entries: 0 = Σw, 1..p = Σ w θ_a, then lower triangle (a >= b) Σ w θ_a θ_b
-    const int nent = 1 + p + p * (p + 1) / 2;
+    extern __shared__ double sm[];      // x [chunk][p + 1], w x [chunk][p + 1]
+    __shared__ double s_red[256];
+    const int tid = threadIdx.x, q = p + 1, nent = q * (q + 1) / 2;
+    double* sx = sm;
+    double* sy = sm + (size_t)chunk * q;
+    const int groups = nent < 256 ? 256 / nent : 1;
+    const int grp = groups > 1 ? tid / nent : 0;
     const int c0 = blockIdx.x * cpb;
+    // the sum over this group's share of count terms, two chains of dependent FMAs
+    auto group_sum = [&](double acc, int count, auto term) {
+        double odd = 0.0;
+        int i = grp;
+        for (; i + groups < count; i += 2 * groups) {
+            acc = term(i, acc);
+            odd = term(i + groups, odd);
+        }
+        if (i < count) acc = term(i, acc);
+        return acc + odd;
+    };
     for (int c = c0; c < c0 + cpb; ++c) {
-        const int begin = c * chunk;
+        const long begin = (long)c * chunk;
         if (begin >= n) break;
-        const int cnt = min(chunk, n - begin);
+        const int cnt = (int)(n - begin < chunk ? n - begin : chunk);
         __syncthreads();
-        for (int k = threadIdx.x; k < cnt * p; k += blockDim.x) sth[k] = theta[(size_t)begin * p + k];
-        for (int k = threadIdx.x; k < cnt; k += blockDim.x) sw[k] = w[begin + k];
+        for (int k = tid; k < cnt * p; k += blockDim.x) {
+            const int i = k / p, j = i * q + 1 + (k - i * p);
+            const double x = theta[(size_t)begin * p + k];
+            sx[j] = x;
+            sy[j] = w[begin + i] * x;
+        }
+        for (int i = tid; i < cnt; i += blockDim.x) {
+            sx[(size_t)i * q] = 1.0;
+            sy[(size_t)i * q] = w[begin + i];
+        }
         __syncthreads();
-        for (int e = threadIdx.x; e < nent; e += blockDim.x) {
-            int a = -1, b = -1;
-            if (e >= 1 && e <= p) {
-                a = e - 1;
-            } else if (e > p) {
-                // row a of the lower triangle starts at entry a (a + 1) / 2
-                int t = e - 1 - p;
-                a = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-                while ((a + 1) * (a + 2) / 2 <= t) ++a;
-                while (a * (a + 1) / 2 > t) --a;
-                b = t - a * (a + 1) / 2;
+        for (int e = groups > 1 ? tid - grp * nent : tid; e < nent; e += 256) {
+            double acc = (c == c0 || grp > 0) ? 0.0 : part[(size_t)blockIdx.x * nent + e];
+            if (grp < groups) {
+                int a, b;
+                triangle_entry(e, a, b);
+                acc = group_sum(acc, cnt, [&](int i, double t) { return fma(sy[i * q + a], sx[i * q + b], t); });
             }
-            double acc = (c == c0) ? 0.0 : part[(size_t)blockIdx.x * nent + e];
-            for (int i = 0; i < cnt; ++i) {
-                double v = sw[i];
-                if (a >= 0) v *= sth[i * p + a];
-                if (b >= 0) v *= sth[i * p + b];
-                acc += v;
+            if (groups == 1) {
+                part[(size_t)blockIdx.x * nent + e] = acc;
+            } else {
+                s_red[tid] = acc;
+                break;                  // one entry per thread
             }
-            part[(size_t)blockIdx.x * nent + e] = acc;
+        }
+        if (groups > 1) {
+            __syncthreads();
+            if (tid < nent) {
+                double acc = s_red[tid];
+                for (int g = 1; g < groups; ++g) acc += s_red[g * nent + tid];
+                part[(size_t)blockIdx.x * nent + tid] = acc;
+            }
         }
     }
     // the last block to finish (threadfence reduction: the count is cleared before the launch)
     __shared__ int s_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
+    if (tid == 0) s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // totals over the blocks, in block order
-    for (int e = threadIdx.x; e < nent; e += blockDim.x) {
+    // totals over the blocks, each group its share of them in block order
+    for (int e = groups > 1 ? tid - grp * nent : tid; e < nent; e += 256) {
         double acc = 0.0;
-        for (int k = 0; k < (int)gridDim.x; ++k) acc += __ldcg(part + (size_t)k * nent + e);
-        tot[e] = acc;
+        if (grp < groups)
+            acc = group_sum(acc, (int)gridDim.x, [&](int k, double t) { return t + __ldcg(part + (size_t)k * nent + e); });
+        if (groups == 1) {
+            tot[e] = acc;
+        } else {
+            s_red[tid] = acc;
+            break;
+        }
+    }
+    __syncthreads();
+    if (groups > 1 && tid < nent) {
+        double acc = s_red[tid];
+        for (int g = 1; g < groups; ++g) acc += s_red[g * nent + tid];
+        tot[tid] = acc;
     }
     __syncthreads();
     // Σ_ab = Σ w θ_a θ_b - θ̄_a θ̄_b with θ̄ = Σ w θ / Σ w (gsl_stats_wmean)
-    for (int e = threadIdx.x; e < p * (p + 1) / 2; e += blockDim.x) {
-        int a = (int)((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
-        while ((a + 1) * (a + 2) / 2 <= e) ++a;
-        while (a * (a + 1) / 2 > e) --a;
-        const int b = e - a * (a + 1) / 2;
-        const double ma = tot[1 + a] / tot[0], mb = tot[1 + b] / tot[0];
-        const double v = tot[1 + p + e] - ma * mb;
-        sigma[a * p + b] = v;
-        sigma[b * p + a] = v;
+    for (int e = tid; e < nent; e += 256) {
+        int a, b;
+        triangle_entry(e, a, b);
+        if (b == 0) continue;
+        const double ma = tot[a * (a + 1) / 2] / tot[0], mb = tot[b * (b + 1) / 2] / tot[0];
+        const double v = tot[e] - ma * mb;
+        sigma[(a - 1) * p + b - 1] = v;
+        sigma[(b - 1) * p + a - 1] = v;
     }
 }
 
@@ -1619,13 +1672,6 @@ extern "C" int ag_cov_schedule_brent(const ag_stage_state* st, const double* dat
                                      as_stream(stream));
 }
 
-static void sigma_grid(int n, int p, int* chunk, int* nblk, int* cpb) {
-    *chunk = sigma_chunk(p);
-    const int nchunks = blocks(n, *chunk);
-    *cpb = blocks(nchunks, kSigmaBlocks);
-    *nblk = blocks(nchunks, *cpb);
-}
-
 extern "C" size_t ag_sigma_workspace_bytes(int32_t n, int32_t p) {
     if (n <= 0 || p <= 0 || p > kMaxPLarge) return 0;
     int chunk, nblk, cpb;
@@ -1645,7 +1691,7 @@ extern "C" int ag_weighted_cov(const ag_stage_state* st, const double* theta, in
     int chunk, nblk, cpb;
     sigma_grid(n, p, &chunk, &nblk, &cpb);
     const int nent = 1 + p + p * (p + 1) / 2;
-    const size_t smem = (size_t)chunk * (p + 1) * sizeof(double);
+    const size_t smem = (size_t)chunk * 2 * (p + 1) * sizeof(double);
     if (smem > 48 * 1024) {
         rc = cuda_status(cudaFuncSetAttribute(sigma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                          "cudaFuncSetAttribute(sigma_kernel)");

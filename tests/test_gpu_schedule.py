@@ -48,3 +48,23 @@ def test_grid_schedule_partitions(cuda, kind, n):
     assert abs(db - db_ref) <= 1e-12 * abs(db_ref) and abs(b - b_ref) <= 1e-12
     assert abs(cov - cov_ref) <= 1e-9 * max(1.0, cov_ref)
     np.testing.assert_allclose(st.w.cpu().numpy(), w_ref, rtol=1e-10, atol=1e-300)
+
+
+@pytest.mark.parametrize("p", [1, 2, 10, 21, 22, 33])
+@pytest.mark.parametrize("n", [1, 16, 17, 2433, 39000])
+def test_weighted_cov_partitions(cuda, p, n):
+    """Σ where its partition changes: one to many groups of threads per block (22 parameters on, a
+    thread takes several entries), fewer chains than a block's, several chunks per block."""
+    rng = np.random.default_rng(100 * n + p)
+    theta = rng.normal(size=(n, p)) * np.logspace(0, 2, p) + 5.0
+    w = rng.random(n) + 1e-3
+    w /= w.sum()
+    st = StageState(n, p)
+    st.w.copy_(dev(w))
+    ws = workspace(_native.load().ag_sigma_workspace_bytes(n, p))
+    dth = dev(theta)
+    _native.call("ag_weighted_cov", st.struct, ptr(dth), n, p, ptr(ws), ws.numel(), stream_handle())
+    torch.cuda.synchronize()
+    # E[θθ] and the mean's square cancel: the bound is relative to the moments, not to their difference
+    np.testing.assert_allclose(st.sigma.cpu().numpy(), catmip.weighted_cov(theta, w), rtol=0,
+                               atol=1e-13 * np.max(theta ** 2))
