@@ -146,6 +146,7 @@ _SIGNATURES = {
     "ag_linear_llk_fp64": (c_int, [P, P, c_int32, c_double, P, P]),
     "ag_whiten_workspace_bytes": (c_size_t, [c_int32, c_int32]),
     "ag_whiten_llk": (c_int, [P, P, c_int32, c_int32, P, P, c_size_t, P, P]),
+    "ag_whiten_llk_lower": (c_int, [P, P, c_int32, c_int32, P, P, c_size_t, P, P]),
     "ag_reverso_llk": (c_int, [P, P, c_int32, ctypes.c_double, P, P, P, P]),
     "ag_mlp_param_count": (ctypes.c_int64, [P]),
     "ag_mlp_activation_floats": (ctypes.c_int64, [P, c_int32]),

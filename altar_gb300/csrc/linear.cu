@@ -11,7 +11,7 @@
 // the product A δ is one GEMM over the concatenated K axis
 //     [δ_hi | δ_lo | δ_hi] · [A_hi | A_hi | A_lo]ᵀ
 // (three BF16 products, FP32 accumulation; the dropped lo·lo term is
-// ~2^-18 relative).  The GEMM is a persistent tcgen05 kernel: TMA loads
+// ~2^-18 relative; δ is stored as [δ_hi | δ_lo], its first half read twice).  The GEMM is a persistent tcgen05 kernel: TMA loads
 // 128B-swizzled K-major tiles into a 4-stage shared-memory ring guarded by
 // mbarriers, one thread issues tcgen05.mma (M = 128 chains, N = 256
 // observations, K = 16) into one of two TMEM accumulators, and four epilogue
@@ -38,22 +38,30 @@ namespace ag {
 // TC_GROUP_M chain tiles so that CTAs running at the same time share both operands' k
 // slices in L2.  Every wait is bounded; a timeout stops all roles, drains the copies
 // and MMAs in flight and frees TMEM.
+//
+// LOWER: the second operand is lower triangular (W = L⁻¹), so a tile of observations n0 .. n0 + 255
+// needs k < n0 + 256 only; the products left out are zeros (half the multiplications of a dense
+// whitening were).  The tiles of a group are then taken longest first.  Measured, 3,000
+// observations and 16,384 chains: 296 µs (504 µs with the zeros).  (Tiles from a common counter instead of a fixed
+// stride, and the sum over observation tiles by the last CTA of a chain tile instead of a launch
+// of its own, were slower: the fence before the count alone took 12 of 85 µs of the linear model.)
 constexpr int TC_THREADS = 192;
 constexpr int TC_GROUP_M = 8;
 constexpr uint32_t TC_SMEM = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*bars*/;
 
-AG_DEVICE_INLINE void tile_coords(int t, int mtiles, int ntiles, int& mt, int& nt) {
+AG_DEVICE_INLINE void tile_coords(int t, int mtiles, int ntiles, bool lower, int& mt, int& nt) {
     const int span = TC_GROUP_M * ntiles;
     const int g = t / span, r = t % span;
     const int gm = (mtiles - g * TC_GROUP_M) < TC_GROUP_M ? (mtiles - g * TC_GROUP_M) : TC_GROUP_M;
     mt = g * TC_GROUP_M + r % gm;
-    nt = r / gm;
+    nt = lower ? ntiles - 1 - r / gm : r / gm;
 }
 
+template <bool LOWER>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  x K' (BF16)
-                        const __grid_constant__ CUtensorMap map_b,   // obs     x K' (BF16)
-                        int n, int m_obs, int kblocks, int mtiles, int ntiles,
+linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains x 2 kp (BF16)  [hi | lo]
+                        const __grid_constant__ CUtensorMap map_b,   // obs    x 3 kp (BF16)  [hi | hi | lo]
+                        int n, int m_obs, int kpb, int mtiles, int ntiles,
                         const float* __restrict__ rho0, double* __restrict__ partial,
                         uint32_t* __restrict__ flags) {
     extern __shared__ uint8_t smem_raw[];
@@ -68,6 +76,7 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  
     uint64_t* drain = bars + 2 * TC_STAGES + 4;  // [1]          all MMAs done (teardown)
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
+    __shared__ __align__(16) float s_rho[4][TC_BN];   // ρ₀ of the tile, a copy per epilogue warp
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total = mtiles * ntiles;
@@ -95,14 +104,27 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     auto aborted = [&]() { return *(volatile int*)&s_abort != 0; };
+    // k blocks of each of the three products for observation tile nt
+    auto blocks_of = [&](int nt) {
+        const int need = (nt + 1) * (TC_BN / TC_BK);
+        return LOWER && need < kpb ? need : kpb;
+    };
 
     int issued = 0;                              // TMA stages issued (producer thread)
     if (warp == 0 && lane == 0) {
         // TMA producer: the stage ring runs on across tiles
         for (int t = blockIdx.x; t < total && !aborted(); t += gridDim.x) {
             int mt, nt;
-            tile_coords(t, mtiles, ntiles, mt, nt);
-            for (int kb = 0; kb < kblocks; ++kb, ++issued) {
+            tile_coords(t, mtiles, ntiles, LOWER, mt, nt);
+            const int len = blocks_of(nt);
+            // δ_hi A_hi, δ_lo A_hi, δ_hi A_lo: the first half's blocks serve twice on each side
+            int g = 0, k = 0;
+            for (int kb = 0; kb < 3 * len; ++kb, ++issued) {
+                const int xa = (g == 1 ? kpb + k : k) * TC_BK, xb = (g == 2 ? 2 * kpb + k : k) * TC_BK;
+                if (++k == len) {
+                    k = 0;
+                    ++g;
+                }
                 const int s = issued % TC_STAGES;
                 if (issued >= TC_STAGES &&
                     !mbar_wait_bounded(&empty[s], (uint32_t)((issued / TC_STAGES) - 1) & 1u, TC_WAIT)) {
@@ -112,8 +134,8 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  
                 if (aborted()) break;
                 const uint32_t sa = base + s * TC_STAGE_BYTES;
                 mbar_arrive_expect_tx(&full[s], TC_STAGE_BYTES);
-                tma_load_2d(sa, &map_a, kb * TC_BK, mt * TC_BM, smem_addr(&full[s]));
-                tma_load_2d(sa + TC_A_BYTES, &map_b, kb * TC_BK, nt * TC_BN, smem_addr(&full[s]));
+                tma_load_2d(sa, &map_a, xa, mt * TC_BM, smem_addr(&full[s]));
+                tma_load_2d(sa + TC_A_BYTES, &map_b, xb, nt * TC_BN, smem_addr(&full[s]));
             }
         }
     } else if (warp == 1 && lane == 0) {
@@ -122,6 +144,9 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  
         int it = 0, local = 0;
         for (int t = blockIdx.x; t < total && !aborted(); t += gridDim.x, ++local) {
             const int b = local & 1;
+            int mt, nt;
+            tile_coords(t, mtiles, ntiles, LOWER, mt, nt);
+            const int kblocks = 3 * blocks_of(nt);
             if (local >= 2 && !mbar_wait_bounded(&tempty[b], (uint32_t)((local >> 1) - 1) & 1u, TC_WAIT)) {
                 atomicExch(&s_abort, 1);
                 break;
@@ -154,46 +179,51 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  
         // epilogue: thread = chain row (TMEM lane quarter of this warp), sums over observations
         const int quarter = warp & 3;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        float* rho = s_rho[quarter];
         int local = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++local) {
             const int b = local & 1;
+            int mt, nt;
+            tile_coords(t, mtiles, ntiles, LOWER, mt, nt);
+            const int n0 = nt * TC_BN;
+            // observations past the end have zero rows in the operand: with ρ₀ = 0 they add nothing
+#pragma unroll
+            for (int c = lane; c < TC_BN; c += 32) rho[c] = n0 + c < m_obs ? __ldg(rho0 + n0 + c) : 0.f;
             const bool ok = __all_sync(0xffffffffu,
                                        mbar_wait_bounded(&tfull[b], (uint32_t)(local >> 1) & 1u, TC_WAIT));
             if (!ok || aborted()) {
                 if (lane == 0) atomicExch(&s_abort, 1);
                 break;
             }
+            __syncwarp();
             tc_fence_after();
-            int mt, nt;
-            tile_coords(t, mtiles, ntiles, mt, nt);
-            const int n0 = nt * TC_BN;
             const int chain = mt * TC_BM + quarter * 32 + lane;
             double acc = 0.0;
 #pragma unroll 1
             for (int c0 = 0; c0 < TC_BN; c0 += 64) {
-                // two 32-column loads in flight per wait; lane l holds ρ₀ of observation
-                // n0 + c0 + l (and + 32), broadcast by shuffles
+                // two 32-column loads in flight per wait
                 uint32_t r0[32], r1[32];
                 tmem_ld32_nowait(tmem + lane_base + (uint32_t)(b * TC_BN + c0), r0);
                 tmem_ld32_nowait(tmem + lane_base + (uint32_t)(b * TC_BN + c0 + 32), r1);
-                const int obs_l = n0 + c0 + lane;
-                const float rho_a = (obs_l < m_obs) ? __ldg(rho0 + obs_l) : 0.f;
-                const float rho_b = (obs_l + 32 < m_obs) ? __ldg(rho0 + obs_l + 32) : 0.f;
                 tmem_wait_ld();
-                float sq = 0.f;
+                auto add = [&](const uint32_t (&r)[32], const float4* p) {
+                    float sq = 0.f;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float r = __uint_as_float(r0[i]) + __shfl_sync(0xffffffffu, rho_a, i);
-                    sq = (n0 + c0 + i < m_obs) ? fmaf(r, r, sq) : sq;
-                }
-                acc += (double)sq;
-                sq = 0.f;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float r = __uint_as_float(r1[i]) + __shfl_sync(0xffffffffu, rho_b, i);
-                    sq = (n0 + c0 + 32 + i < m_obs) ? fmaf(r, r, sq) : sq;
-                }
-                acc += (double)sq;
+                    for (int i = 0; i < 32; i += 4) {
+                        const float4 q = p[i >> 2];
+                        float d = __uint_as_float(r[i]) + q.x;
+                        sq = fmaf(d, d, sq);
+                        d = __uint_as_float(r[i + 1]) + q.y;
+                        sq = fmaf(d, d, sq);
+                        d = __uint_as_float(r[i + 2]) + q.z;
+                        sq = fmaf(d, d, sq);
+                        d = __uint_as_float(r[i + 3]) + q.w;
+                        sq = fmaf(d, d, sq);
+                    }
+                    acc += (double)sq;
+                };
+                add(r0, reinterpret_cast<const float4*>(rho + c0));
+                add(r1, reinterpret_cast<const float4*>(rho + c0 + 32));
             }
             if (chain < n) partial[(size_t)nt * n + chain] = acc;
             tc_fence_before();
@@ -220,84 +250,135 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains  
     }
 }
 
-// ρ₀ = W r̄ in FP64 (one warp per whitened observation)
-__global__ void whiten_rho0_kernel(const double* __restrict__ W, const double* __restrict__ mean, int m,
-                                   float* __restrict__ rho0) {
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= m) return;
-    double s = 0.0;
-    for (int j = lane; j < m; j += 32) s = fma(W[(size_t)row * m + j], mean[j], s);
-    s = warp_sum(s);
-    if (lane == 0) rho0[row] = (float)s;
-}
-
-// θ₀ = column means of θ (one thread per parameter, fixed order)
 // Centring point θ₀ (or r̄): the mean of up to kCentreRows rows taken at an even stride.
 // Any centre gives the same result, because ρ₀ = A θ₀ - b carries it exactly in FP64;
 // the centre only has to lie inside the population so that the BF16 split of θ - θ₀ keeps
-// its relative precision.  One thread per column, rows in a fixed order.
+// its relative precision.  32 columns per CTA (lanes), the sampled rows split over the 8 warps
+// (all of a warp's loads in flight at once), then the warp partial sums added in warp order.
+// Beside the FP64 centre, its two leading FP32 parts (centre32).
 constexpr int kCentreRows = 256;
 static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 template <class T>
 __global__ void __launch_bounds__(256) centre_kernel(const T* __restrict__ x, int ld, int col0, int n, int cols,
-                                                     double* __restrict__ centre) {
-    // 32 columns per CTA (lanes), the sampled rows split over the 8 warps, then the warp
-    // partial sums added in warp order
+                                                     double* __restrict__ centre, float2* __restrict__ centre32) {
     __shared__ double part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
     const int rows = n < kCentreRows ? n : kCentreRows;
     const long stride = n / rows;                      // >= 1
-    double s = 0.0;
-    if (j < cols) {
-#pragma unroll 4
-        for (int k = warp; k < rows; k += 8) s += (double)__ldg(x + (size_t)(k * stride) * ld + col0 + j);
+    T v[kCentreRows / 8];
+#pragma unroll
+    for (int q = 0; q < kCentreRows / 8; ++q) {
+        const int k = warp + 8 * q;
+        v[q] = (j < cols && k < rows) ? __ldg(x + (size_t)(k * stride) * ld + col0 + j) : (T)0;
     }
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < kCentreRows / 8; ++q)
+        if (warp + 8 * q < rows) s += (double)v[q];
     part[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && j < cols) {
         double t = 0.0;
         for (int w = 0; w < 8; ++w) t += part[w][lane];
-        centre[j] = t / rows;
+        t /= rows;
+        centre[j] = t;
+        const float hi = (float)t;
+        centre32[j] = make_float2(hi, (float)(t - (double)hi));
     }
 }
 
-// ρ₀ = A θ₀ - b in FP64 (one warp per observation)
-__global__ void rho0_kernel(const double* __restrict__ A, const double* __restrict__ b,
-                            const double* __restrict__ theta0, int m, int p, float* __restrict__ rho0) {
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= m) return;
-    double s = 0.0;
-    for (int j = lane; j < p; j += 32) s = fma(A[(size_t)row * p + j], theta0[j], s);
-    s = warp_sum(s);
-    if (lane == 0) rho0[row] = (float)(s - b[row]);
+// a double rounded to FP32 in integer arithmetic (the conversion instruction runs at the FP64
+// pipe's rate); values outside FP32's normal range take the instruction
+AG_DEVICE_INLINE float to_f32(double d) {
+    const uint64_t b = (uint64_t)__double_as_longlong(d);
+    const int e = (int)(b >> 52) & 0x7ff;
+    if (e < 1023 - 126 || e > 1023 + 126) return (float)d;
+    const uint64_t m = b & 0x7FFFFFFFFFFFFFFFull;
+    const uint64_t r = m + 0x0FFFFFFFull + ((m >> 29) & 1);          // to nearest, ties to even
+    return __uint_as_float((uint32_t)(r >> 29) - ((1023u - 127u) << 23) | ((uint32_t)(b >> 32) & 0x80000000u));
 }
 
-// δ = x - centre split as [hi | lo | hi] (BF16, row length 3 kp, kp = columns padded to
-// 64): one thread per 8 consecutive columns of a row, three 16-byte stores.  Rows of x have
-// stride ld and start at column col0 (θ: ld = p, col0 = 0; a residual block: the residual
-// rows and the block's first column).
-template <class T>
-__global__ void split_centred_kernel(const T* __restrict__ x, int ld, int col0, const double* __restrict__ centre,
-                                     int n, int cols, int kp, __nv_bfloat16* __restrict__ out) {
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// x - centre rounded to FP32.  θ in FP64: one subtraction.  Residuals in FP32 against the centre's
+// two FP32 parts (48 bits): the exact error of x - hi takes the rest, so that only FP32
+// instructions run (FP64 ones made the splits of 81 million residuals, 16,384 chains of
+// 4,950, 455 µs and ρ₀ 45 µs more; with ρ₀ in the same launch they take 126 µs).
+AG_DEVICE_INLINE float minus_centre(float x, float2 c) {
+    float s, e;
+    two_sum(x, -c.x, s, e);
+    return s + (e - c.y);
+}
+AG_DEVICE_INLINE float minus_centre(double x, double c) { return to_f32(x - c); }
+
+// Second launch of an evaluation, by CTAs of two kinds.  The first `rho_ctas`: ρ₀ = A θ₀ - b in
+// FP64 (b = NULL: W r̄), one warp per observation; a lower triangular A is read up to its diagonal.
+// The others: δ = x - centre split as [hi | lo] (BF16, row length 2 kp, kp = columns padded to
+// 64), a thread per 8 consecutive columns of kSplitRows rows whose loads are all in flight
+// together, two 16-byte stores a row.  Rows of x have stride ld and start at column col0 (θ:
+// ld = p, col0 = 0; a residual block: the residual rows and the block's first column).
+constexpr int kSplitRows = 2;
+template <class T> struct CentreOf { typedef double type; };
+template <> struct CentreOf<float> { typedef float2 type; };
+
+template <class T, bool LOWER>
+__global__ void __launch_bounds__(256) split_rho0_kernel(const T* __restrict__ x, int ld, int col0,
+                                                         const double* __restrict__ centre,
+                                                         const typename CentreOf<T>::type* __restrict__ shift, int n,
+                                                         int cols, int kp, __nv_bfloat16* __restrict__ out, int rho_ctas,
+                                                         const double* __restrict__ A, const double* __restrict__ b,
+                                                         int m, float* __restrict__ rho0) {
+    if ((int)blockIdx.x < rho_ctas) {
+        const int row = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        if (row >= m) return;
+        const int len = LOWER ? row + 1 : cols;
+        double s = 0.0;
+#pragma unroll 8
+        for (int j = lane; j < len; j += 32) s = fma(__ldg(A + (size_t)row * cols + j), __ldg(centre + j), s);
+        s = warp_sum(s);
+        if (lane == 0) rho0[row] = (float)(b ? s - b[row] : s);
+        return;
+    }
     const int groups = kp >> 3;
-    if (e >= (long)n * groups) return;
-    const int i = (int)(e / groups), j0 = (int)(e % groups) * 8;
-    __align__(16) __nv_bfloat16 hi[8], lo[8];
+    const long e = (long)((int)blockIdx.x - rho_ctas) * 256 + threadIdx.x;
+    const long band = e / groups;
+    const int j0 = (int)(e - band * groups) * 8;
+    const long i0 = band * kSplitRows;
+    if (i0 >= n) return;
+    // 16-byte loads where the row segments are aligned for them
+    const bool wide = j0 + 8 <= cols && ((size_t)(x + col0) % 16 == 0) && ((size_t)ld * sizeof(T)) % 16 == 0;
+    __align__(16) T v[kSplitRows][8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int j = j0 + q;
-        const float d = (j < cols) ? (float)((double)x[(size_t)i * ld + col0 + j] - centre[j]) : 0.f;
-        hi[q] = __float2bfloat16_rn(d);
-        lo[q] = __float2bfloat16_rn(d - __bfloat162float(hi[q]));
+    for (int r = 0; r < kSplitRows; ++r) {
+        const long i = i0 + r < n ? i0 + r : n - 1;
+        const T* src = x + (size_t)i * ld + col0 + j0;
+        if (wide) {
+#pragma unroll
+            for (int q = 0; q < (int)(8 * sizeof(T) / 16); ++q)
+                reinterpret_cast<uint4*>(v[r])[q] = __ldg(reinterpret_cast<const uint4*>(src) + q);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[r][q] = j0 + q < cols ? __ldg(src + q) : (T)0;
+        }
     }
-    __nv_bfloat16* row = out + (size_t)i * 3 * kp;
-    const uint4 h = *reinterpret_cast<const uint4*>(hi), l = *reinterpret_cast<const uint4*>(lo);
-    *reinterpret_cast<uint4*>(row + j0) = h;
-    *reinterpret_cast<uint4*>(row + kp + j0) = l;
-    *reinterpret_cast<uint4*>(row + 2 * kp + j0) = h;
+    // (the centre arrays are as long as a row's kp columns)
+    typename CentreOf<T>::type c[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = __ldg(shift + j0 + q);
+#pragma unroll
+    for (int r = 0; r < kSplitRows; ++r) {
+        if (i0 + r >= n) break;
+        __align__(16) __nv_bfloat16 hi[8], lo[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float d = j0 + q < cols ? minus_centre(v[r][q], c[q]) : 0.f;
+            hi[q] = __float2bfloat16_rn(d);
+            lo[q] = __float2bfloat16_rn(d - __bfloat162float(hi[q]));
+        }
+        __nv_bfloat16* row = out + (size_t)(i0 + r) * 2 * kp;
+        *reinterpret_cast<uint4*>(row + j0) = *reinterpret_cast<const uint4*>(hi);
+        *reinterpret_cast<uint4*>(row + kp + j0) = *reinterpret_cast<const uint4*>(lo);
+    }
 }
 
 // A split as [hi | hi | lo]
@@ -320,12 +401,10 @@ __global__ void linear_reduce_kernel(int n, int tiles, const double* __restrict_
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double s = 0.0;
+#pragma unroll 8
     for (int t = 0; t < tiles; ++t) s += partial[(size_t)t * n + i];
     llk[i] = (accumulate ? llk[i] : norm) - 0.5 * s;
 }
-
-
-
 
 // Exact FP64 reference path: ρ = A θ - b per chain (one warp per chain, observations strided)
 __global__ void linear_fp64_kernel(const double* __restrict__ A, const double* __restrict__ b,
@@ -361,11 +440,64 @@ extern "C" int ag_linear_prepare(const double* A, int32_t m, int32_t p, uint16_t
     return launch_status("split_a_kernel");
 }
 
+// workspace of an evaluation: centre [kp], FP64 and as two FP32 parts | ρ₀ [m] | split rows
+// [n][2 kp] | partials [tiles][n]
+static size_t eval_workspace(int m, int cols, int n) {
+    const size_t kp = ag_linear_kpad(cols);
+    return 2 * al256(kp * sizeof(double)) + al256((size_t)m * sizeof(float)) + al256((size_t)n * 2 * kp * 2) +
+           al256((size_t)cdiv(m, TC_BN) * n * sizeof(double));
+}
+
+// llk = (accumulate ? llk : norm) - 1/2 |A (x - x̄) + ρ₀|², ρ₀ = A x̄ - b: the centre; the split of
+// the centred rows with ρ₀; the tensor-core product with the fused misfit; the sum over tiles
+template <class T, bool LOWER>
+static int eval_llk(const T* x, int ld, int col0, int n, int cols, const double* a64, const double* b,
+                    const uint16_t* a_split, int m, double norm, int accumulate, double* llk, void* workspace,
+                    uint32_t* flags, cudaStream_t s) {
+    const int kp = ag_linear_kpad(cols), tiles = cdiv(m, TC_BN), mtiles = cdiv(n, TC_BM);
+    char* ws = static_cast<char*>(workspace);
+    double* centre = reinterpret_cast<double*>(ws); ws += al256(kp * sizeof(double));
+    float2* centre32 = reinterpret_cast<float2*>(ws); ws += al256(kp * sizeof(double));
+    float* rho0 = reinterpret_cast<float*>(ws); ws += al256((size_t)m * sizeof(float));
+    __nv_bfloat16* split = reinterpret_cast<__nv_bfloat16*>(ws); ws += al256((size_t)n * 2 * kp * 2);
+    double* partial = reinterpret_cast<double*>(ws);
+    centre_kernel<T><<<cdiv(cols, 32), 256, 0, s>>>(x, ld, col0, n, cols, centre, centre32);
+    int rc = launch_status("centre_kernel");
+    if (rc) return rc;
+    const typename CentreOf<T>::type* shift;
+    if constexpr (sizeof(T) == 4)
+        shift = centre32;
+    else
+        shift = centre;
+    const int split_ctas = cdiv((long)cdiv(n, kSplitRows) * (kp / 8), 256);
+    split_rho0_kernel<T, LOWER><<<cdiv(m, 8) + split_ctas, 256, 0, s>>>(x, ld, col0, centre, shift, n, cols, kp, split,
+                                                                        cdiv(m, 8), a64, b, m, rho0);
+    rc = launch_status("split_rho0_kernel");
+    if (rc) return rc;
+    CUtensorMap ma, mb;
+    rc = make_map(&ma, split, n, 2 * kp, TC_BM);
+    if (rc) return rc;
+    rc = make_map(&mb, a_split, m, 3 * kp, TC_BN);
+    if (rc) return rc;
+    // per call: the attribute belongs to the current device's context
+    rc = cuda_status(cudaFuncSetAttribute(linear_misfit_tc_kernel<LOWER>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM),
+                     "cudaFuncSetAttribute(linear_misfit_tc_kernel)");
+    if (rc) return rc;
+    int sms = 0;
+    rc = sm_count(&sms);
+    if (rc) return rc;
+    const int total = mtiles * tiles;
+    linear_misfit_tc_kernel<LOWER><<<total < sms ? total : sms, TC_THREADS, TC_SMEM, s>>>(
+        ma, mb, n, m, kp / TC_BK, mtiles, tiles, rho0, partial, flags);
+    rc = launch_status("linear_misfit_tc_kernel");
+    if (rc) return rc;
+    linear_reduce_kernel<<<cdiv(n, 128), 128, 0, s>>>(n, tiles, partial, norm, llk, accumulate);
+    return launch_status("linear_reduce_kernel");
+}
+
 extern "C" size_t ag_linear_workspace_bytes(int32_t m, int32_t p, int32_t n) {
-    if (m <= 0 || p <= 0 || n <= 0) return 0;
-    const size_t kp = ag_linear_kpad(p);
-    return al256(p * sizeof(double)) + al256((size_t)m * sizeof(float)) +
-           al256((size_t)n * 3 * kp * 2) + al256((size_t)cdiv(m, TC_BN) * n * sizeof(double));
+    return m <= 0 || p <= 0 || n <= 0 ? 0 : eval_workspace(m, p, n);
 }
 
 extern "C" int ag_linear_llk(const ag_linear_model* lm, const double* theta, int32_t n, double norm,
@@ -378,98 +510,41 @@ extern "C" int ag_linear_llk(const ag_linear_model* lm, const double* theta, int
     AG_REQUIRE(workspace && workspace_bytes >= need && aligned(workspace, 256),
                "ag_linear_llk needs %zu bytes of 256-byte aligned workspace", need);
     AG_REQUIRE(aligned(lm->a_split, 16), "a_split must be 16-byte aligned");
-    cudaStream_t s = as_stream(stream);
-    const int kp = ag_linear_kpad(p);
-    char* ws = static_cast<char*>(workspace);
-    double* theta0 = reinterpret_cast<double*>(ws); ws += al256(p * sizeof(double));
-    float* rho0 = reinterpret_cast<float*>(ws); ws += al256((size_t)m * sizeof(float));
-    __nv_bfloat16* tsplit = reinterpret_cast<__nv_bfloat16*>(ws); ws += al256((size_t)n * 3 * kp * 2);
-    double* partial = reinterpret_cast<double*>(ws);
-    const int tiles = cdiv(m, TC_BN);
-    centre_kernel<double><<<cdiv(p, 32), 256, 0, s>>>(theta, p, 0, n, p, theta0);
-    rho0_kernel<<<cdiv((long)m * 32, 256), 256, 0, s>>>(lm->a64, lm->b64, theta0, m, p, rho0);
-    split_centred_kernel<double><<<cdiv((long)n * (kp / 8), 256), 256, 0, s>>>(theta, p, 0, theta0, n, p, kp,
-                                                                                tsplit);
-    int rc = launch_status("linear prologue kernels");
-    if (rc) return rc;
-    CUtensorMap ma, mb;
-    rc = make_map(&ma, tsplit, n, 3 * kp, TC_BM);
-    if (rc) return rc;
-    rc = make_map(&mb, lm->a_split, m, 3 * kp, TC_BN);
-    if (rc) return rc;
-    // per call: the attribute belongs to the current device's context
-    rc = cuda_status(cudaFuncSetAttribute(linear_misfit_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)TC_SMEM),
-                     "cudaFuncSetAttribute(linear_misfit_tc_kernel)");
-    if (rc) return rc;
-    const int mtiles = cdiv(n, TC_BM), total = mtiles * tiles;
-    int sms = 0;
-    rc = sm_count(&sms);
-    if (rc) return rc;
-    linear_misfit_tc_kernel<<<total < sms ? total : sms, TC_THREADS, TC_SMEM, s>>>(
-        ma, mb, n, m, 3 * kp / TC_BK, mtiles, tiles, rho0, partial, flags);
-    rc = launch_status("linear_misfit_tc_kernel");
-    if (rc) return rc;
-    linear_reduce_kernel<<<cdiv(n, 256), 256, 0, s>>>(n, tiles, partial, norm, llk, 0);
-    return launch_status("linear_reduce_kernel");
+    return eval_llk<double, false>(theta, p, 0, n, p, lm->a64, lm->b64, lm->a_split, m, norm, 0, llk, workspace, flags,
+                                   as_stream(stream));
 }
 
 extern "C" size_t ag_whiten_workspace_bytes(int32_t m, int32_t n) {
-    if (m <= 0 || n <= 0) return 0;
-    const size_t kp = ag_linear_kpad(m);
-    return al256(m * sizeof(double)) + al256(sizeof(double)) + al256((size_t)m * sizeof(float)) +
-           al256((size_t)n * 3 * kp * 2) + al256((size_t)cdiv(m, TC_BN) * n * sizeof(double));
+    return m <= 0 || n <= 0 ? 0 : eval_workspace(m, m, n);
 }
 
-extern "C" int ag_whiten_llk(const ag_whiten_block* blk, const float* resid, int32_t ldr, int32_t n,
-                             double* llk, void* workspace, size_t workspace_bytes, uint32_t* flags,
-                             void* stream) {
+static int whiten_llk(bool lower, const ag_whiten_block* blk, const float* resid, int32_t ldr, int32_t n, double* llk,
+                      void* workspace, size_t workspace_bytes, uint32_t* flags, void* stream) {
     AG_REQUIRE(blk && blk->w64 && blk->w_split && resid && llk && n > 0, "invalid arguments");
     const int m = blk->m, col0 = blk->col0;
     AG_REQUIRE(m > 0 && col0 >= 0 && col0 + m <= ldr, "block columns [%d, %d) outside rows of %d", col0, col0 + m,
                ldr);
     const size_t need = ag_whiten_workspace_bytes(m, n);
     AG_REQUIRE(workspace && workspace_bytes >= need && aligned(workspace, 256),
-               "ag_whiten_llk needs %zu bytes of 256-byte aligned workspace", need);
+               "whitening needs %zu bytes of 256-byte aligned workspace", need);
     AG_REQUIRE(aligned(blk->w_split, 16), "w_split must be 16-byte aligned");
     cudaStream_t s = as_stream(stream);
-    const int kp = ag_linear_kpad(m);
-    char* ws = static_cast<char*>(workspace);
-    double* mean = reinterpret_cast<double*>(ws); ws += al256(m * sizeof(double));
-    ws += al256(sizeof(double));
-    float* rho0 = reinterpret_cast<float*>(ws); ws += al256((size_t)m * sizeof(float));
-    __nv_bfloat16* rsplit = reinterpret_cast<__nv_bfloat16*>(ws); ws += al256((size_t)n * 3 * kp * 2);
-    double* partial = reinterpret_cast<double*>(ws);
-    const int tiles = cdiv(m, TC_BN);
-    centre_kernel<float><<<cdiv(m, 32), 256, 0, s>>>(resid, ldr, col0, n, m, mean);
-    int rc = launch_status("whitening prologue");
-    if (rc) return rc;
-    split_centred_kernel<float><<<cdiv((long)n * (kp / 8), 256), 256, 0, s>>>(resid, ldr, col0, mean, n, m, kp,
-                                                                              rsplit);
-    rc = launch_status("split_centred_kernel");
-    if (rc) return rc;
-    CUtensorMap ma, mb;
-    rc = make_map(&ma, rsplit, n, 3 * kp, TC_BM);
-    if (rc) return rc;
-    rc = make_map(&mb, blk->w_split, m, 3 * kp, TC_BN);
-    if (rc) return rc;
-    rc = cuda_status(cudaFuncSetAttribute(linear_misfit_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)TC_SMEM),
-                     "cudaFuncSetAttribute(linear_misfit_tc_kernel)");
-    if (rc) return rc;
-    whiten_rho0_kernel<<<cdiv((long)m * 32, 256), 256, 0, s>>>(blk->w64, mean, m, rho0);
-    rc = launch_status("whiten_rho0_kernel");
-    if (rc) return rc;
-    const int mtiles = cdiv(n, TC_BM), total = mtiles * tiles;
-    int sms = 0;
-    rc = sm_count(&sms);
-    if (rc) return rc;
-    linear_misfit_tc_kernel<<<total < sms ? total : sms, TC_THREADS, TC_SMEM, s>>>(
-        ma, mb, n, m, 3 * kp / TC_BK, mtiles, tiles, rho0, partial, flags);
-    rc = launch_status("linear_misfit_tc_kernel (whitening)");
-    if (rc) return rc;
-    linear_reduce_kernel<<<cdiv(n, 256), 256, 0, s>>>(n, tiles, partial, 0.0, llk, 1);
-    return launch_status("linear_reduce_kernel (whitening)");
+    return lower ? eval_llk<float, true>(resid, ldr, col0, n, m, blk->w64, nullptr, blk->w_split, m, 0.0, 1, llk,
+                                         workspace, flags, s)
+                 : eval_llk<float, false>(resid, ldr, col0, n, m, blk->w64, nullptr, blk->w_split, m, 0.0, 1, llk,
+                                          workspace, flags, s);
+}
+
+extern "C" int ag_whiten_llk(const ag_whiten_block* blk, const float* resid, int32_t ldr, int32_t n,
+                             double* llk, void* workspace, size_t workspace_bytes, uint32_t* flags,
+                             void* stream) {
+    return whiten_llk(false, blk, resid, ldr, n, llk, workspace, workspace_bytes, flags, stream);
+}
+
+extern "C" int ag_whiten_llk_lower(const ag_whiten_block* blk, const float* resid, int32_t ldr, int32_t n,
+                                   double* llk, void* workspace, size_t workspace_bytes, uint32_t* flags,
+                                   void* stream) {
+    return whiten_llk(true, blk, resid, ldr, n, llk, workspace, workspace_bytes, flags, stream);
 }
 
 extern "C" int ag_linear_llk_fp64(const ag_linear_model* lm, const double* theta, int32_t n, double norm,

@@ -4,7 +4,7 @@ The batched two-source Mogi workload: LOS datasets of uneven sizes, each with
 its own dense Cd.  One fused launch of the Mogi kernel evaluates every chain
 against the concatenated stations and writes the residual rows; each
 dataset's block is then whitened by W = L⁻¹ (Cd = L Lᵀ) on the tensor cores
-(ag_whiten_llk).  The log-likelihood is the Gaussian
+(ag_whiten_llk_lower).  The log-likelihood is the Gaussian
     -1/2 Σ_k (M_k log 2π + log det Cd_k + r_kᵀ Cd_k⁻¹ r_k).
 Parameter sets per source s: ``location{s}`` (2), ``depth{s}`` (1),
 ``source{s}`` (1), laid out with a constant stride between sources.
@@ -98,7 +98,7 @@ class DenseMogi(Bayesian):
                      self.stations.struct, self.normalization, ptr(mask), ptr(out), ptr(status), ptr(resid),
                      None, 0, s)
         for b in self.blocks:
-            _native.call("ag_whiten_llk", ctypes.byref(b), ptr(resid), self.stations.m_padded, n, ptr(out),
+            _native.call("ag_whiten_llk_lower", ctypes.byref(b), ptr(resid), self.stations.m_padded, n, ptr(out),
                          ptr(self._ws), self._ws_bytes, ptr(self.flags), s)
         if residuals is not None:
             residuals.copy_(resid)

@@ -4,7 +4,7 @@ models/mogi/mogi/CUDA.py).
 Holds the device-resident stations and the parameter layout, and evaluates
 the fused forward model + misfit + log-likelihood for a batch of samples.
 With a dense data covariance the fused kernel writes the residual rows
-instead (station weights 0) and ag_whiten_llk adds -1/2 ‖L⁻¹ r‖² (Cd = L Lᵀ)
+instead (station weights 0) and ag_whiten_llk_lower adds -1/2 ‖L⁻¹ r‖² (Cd = L Lᵀ)
 on the tensor cores.
 Device tensors are used in place; host (numpy) samples are copied in and the
 log-likelihoods copied back, which is the reference's call pattern
@@ -100,7 +100,7 @@ class CUDA:
         if self._whiten is not None:
             # the fused misfit was 0 (weights 0): add -1/2 ‖W r‖² of the residual rows
             # (rows of masked or rejected chains hold stale values; their llk is not used)
-            _native.call("ag_whiten_llk", ctypes.byref(self._whiten[2]), ptr(resid), self.stations.m_padded, n,
+            _native.call("ag_whiten_llk_lower", ctypes.byref(self._whiten[2]), ptr(resid), self.stations.m_padded, n,
                          ptr(out), ptr(self._wws), self._wws_bytes, ptr(self._flags), s)
         return out
 

@@ -400,6 +400,10 @@ size_t ag_whiten_workspace_bytes(int32_t m, int32_t n);
 /* resid: n rows of ldr FP32 residuals (ag_forward_llk's residual output) */
 int ag_whiten_llk(const ag_whiten_block* block, const float* resid, int32_t ldr, int32_t n, double* llk,
                   void* workspace, size_t workspace_bytes, uint32_t* flags, void* stream);
+/* the same for a lower triangular W (zeros above the diagonal, as L⁻¹ has): the products with those
+ * zeros are left out; W's entries above the diagonal are taken as zeros */
+int ag_whiten_llk_lower(const ag_whiten_block* block, const float* resid, int32_t ldr, int32_t n, double* llk,
+                        void* workspace, size_t workspace_bytes, uint32_t* flags, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Reverso two-reservoir magma model (FP64).  Replaces the libreverso capsule
