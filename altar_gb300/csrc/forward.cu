@@ -17,9 +17,10 @@
 // cancellation never happens in floating point.
 //
 // Work decomposition: cdm_setup_kernel computes each chain's per-side
-// constants and per-rectangle quadrature parameters in FP64 and packs the
-// chains that have work (not masked, not above the free surface) into
-// consecutive slots; the likelihood kernel runs one warp per slot, lanes over
+// constants and per-rectangle quadrature parameters in FP64 and lists the
+// chains that have work (not masked, not above the free surface) in
+// consecutive slots; the likelihood kernel runs one warp per slot (several for
+// few chains, each over a share of the stations), lanes over
 // stations; a CTA holds WARPS chains whose constants live in shared memory and
 // are read with broadcast vector loads; station tiles stream through a ring of
 // shared-memory buffers filled by 1-D bulk copies (cp.async.bulk + mbarrier)
@@ -30,6 +31,8 @@
 // in FP64 in a fixed order.
 #include <math.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -46,7 +49,7 @@ constexpr uint32_t kWaitLimit = 1u << 24;
 struct __align__(16) ChainC {
     float4 hdr;                 // x0_hi, x0_lo, y0_hi, y0_lo
     uint32_t side_mask;         // active sides; 0 = chain inactive
-    uint32_t status;
+    int32_t chain;              // row of θ, llk and the residuals
     uint32_t pad0, pad1;
     float off[kMaxOffsets];     // per-dataset offsets θ[offset_idx + k]
     float pad2[8];
@@ -55,17 +58,26 @@ struct __align__(16) ChainC {
 };
 static_assert(sizeof(ChainC) % 16 == 0, "ChainC must be a whole number of float4");
 
-// Chain slots ordered by cost.  The chains of one CTA share its ring of station tiles, so a
+// Set-up.  A block takes kSetupChains chains and gives every step to as many threads as it has
+// parts: a thread per rotation (sine and cosine), per corner, per side and rectangle of the plan, per
+// side and rectangle of the constants.  Each part is 50 to 150 dependent FP64 instructions at ~67
+// cycles; one thread per chain took them one after another (159 µs for a set-up of 2,000
+// chains, whatever their number, and the plan twice), sixteen lanes per chain with every lane
+// repeating the corners issued twice the FP64 instructions.  Here lanes are full and nothing is
+// repeated: 31 µs for 2,000 chains (210 µs), 23 µs for 256 (248 µs).
+//
+// Chain slots ordered by cost (ORDERED).  The chains of one CTA share its ring of station tiles, so a
 // CTA advances at the pace of its most expensive chain; with rectangles integrated by
 // quadrature, with node counts that depend on each tile's distance, the work of a chain
-// ranges over several times its minimum.  The set-up therefore runs in two passes:
-// cdm_cost_kernel classifies every requested chain (masked, above the free surface, or the
-// cost bucket of its plan averaged over a sample of the tiles) and counts the chains per
-// bucket; cdm_setup_kernel gives each chain the next slot of its bucket, buckets in
-// decreasing cost, so the CTAs hold chains of similar cost and the expensive ones are
-// scheduled first (which also shortens the tail of the launch for one-chain CTAs).
+// ranges over several times its minimum.  The set-up counts the chains per cost bucket (the work
+// of their plan averaged over a sample of the tiles); cdm_slot_kernel gives each chain the next
+// slot of its bucket, buckets in decreasing cost, so the CTAs hold chains of similar cost and the
+// expensive ones are scheduled first (which also shortens the tail of the launch for one-chain
+// CTAs).  Few chains, whose stations are split over several CTAs, take slots as they come.
 constexpr int kCostBuckets = 64;
 constexpr int kCostBucketFlop = 96;      // FLOP per station per bucket
+constexpr int kSetupChains = 8;
+constexpr int kSetupThreads = 128;
 
 struct SetupHdr {                        // in the workspace, cleared before each set-up
     int32_t nslots;
@@ -74,73 +86,156 @@ struct SetupHdr {                        // in the workspace, cleared before eac
     int32_t fill[kCostBuckets];          // slots handed out per bucket
 };
 
-__device__ __forceinline__ int cost_bucket(uint32_t flop) {
-    const int b = (int)(flop / kCostBucketFlop);
-    return b < kCostBuckets - 1 ? b : kCostBuckets - 1;
-}
-
-// Per-station work of a chain averaged over every stride-th station tile (tile boxes
-// relative to the source centre as the likelihood kernel forms them)
-__device__ float sampled_tile_work(const RectQ* rect, uint32_t mask, const float4* __restrict__ tile_box,
-                                   int ntiles, int stride, float x0h, float x0l, float y0h, float y0l) {
-    float f = 0.f;
-    int cnt = 0;
-    for (int t = stride / 2; t < ntiles; t += stride) {
-        const float4 tb = __ldg(tile_box + t);
-        uint32_t fl, su;
-        tile_work(rect, mask, __fsub_rn(__fsub_rn(tb.x, x0h), x0l), __fsub_rn(__fsub_rn(tb.y, x0h), x0l),
-                  __fsub_rn(__fsub_rn(tb.z, y0h), y0l), __fsub_rn(__fsub_rn(tb.w, y0h), y0l), fl, su);
-        f += (float)fl;
-        ++cnt;
+// All requested chains (n, or the first *count_in of index_in): the constants of each chain with
+// work in row t of out, t its position among the requested; the status bit for one above the
+// free surface.
+template <bool ORDERED>
+__global__ void __launch_bounds__(kSetupThreads)
+cdm_setup_kernel(ag_layout L, const double* __restrict__ theta, int n, const uint32_t* __restrict__ mask_in,
+                 uint32_t* __restrict__ chain_status, const int32_t* __restrict__ index_in,
+                 const int32_t* __restrict__ count_in, int noffsets, const float4* __restrict__ tile_box, int ntiles,
+                 ChainC* __restrict__ out, int8_t* __restrict__ key, int32_t* __restrict__ slot_row,
+                 SetupHdr* __restrict__ hdr) {
+    __shared__ ChainC s_chain[kSetupChains];
+    __shared__ Vec3 s_V[kSetupChains][3][4], s_slip[kSetupChains][3];
+    __shared__ double s_sc[kSetupChains][6];
+    __shared__ int s_idx[kSetupChains], s_nq[kSetupChains][3];
+    __shared__ uint32_t s_above[kSetupChains], s_bits[kSetupChains], s_flop[kSetupChains];
+    const int tid = threadIdx.x, t0 = blockIdx.x * kSetupChains;
+    const int requested = index_in ? min(n, *count_in) : n;
+    if (t0 >= requested) return;
+    if (tid < kSetupChains) {
+        const int t = t0 + tid;
+        int i = -1;
+        if (t < requested) {
+            i = index_in ? index_in[t] : t;
+            if (mask_in && mask_in[i]) {
+                i = -1;
+                if (ORDERED) key[t] = -1;
+            }
+        }
+        s_idx[tid] = i;
+        s_above[tid] = 0u;
+        s_bits[tid] = 0u;
+        s_flop[tid] = 0u;
     }
-    return cnt ? f / (float)cnt : (float)kFlopStation;
-}
-
-// One thread per requested chain (all n, or the first *count_in of index_in): -1 for a masked
-// chain, -2 (and the status bit) for one above the free surface, else its cost bucket (the
-// work of its plan averaged over a sample of the station tiles)
-__global__ void cdm_cost_kernel(ag_layout L, const double* __restrict__ theta, int n,
-                                const uint32_t* __restrict__ mask_in, uint32_t* __restrict__ chain_status,
-                                const int32_t* __restrict__ index_in, const int32_t* __restrict__ count_in,
-                                const float4* __restrict__ tile_box, int ntiles, int8_t* __restrict__ key,
-                                SetupHdr* __restrict__ hdr) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    int i = t;
-    if (index_in) {
-        if (t >= *count_in) return;
-        i = index_in[t];
+    __syncthreads();
+    if (tid < 3 * kSetupChains) {
+        const int c = tid / 3, w = tid - 3 * c;
+        if (s_idx[c] >= 0) {
+            const double omega = theta[(size_t)s_idx[c] * L.nparams + L.omega_idx + w];
+            sincospi(omega / 180.0, &s_sc[c][2 * w], &s_sc[c][2 * w + 1]);
+        }
     }
-    if (mask_in && mask_in[i]) {
-        key[t] = -1;
-        return;
+    __syncthreads();
+    // threads 0-95: a corner, then a side, of one chain; threads 96-119: a rectangle
+    const bool on_side = tid < kSides * kSetupChains;
+    const int c = on_side ? tid / kSides : min((tid - kSides * kSetupChains) / 3, kSetupChains - 1);
+    const int e = on_side ? tid - kSides * c : 0;
+    const int r = on_side ? e >> 2 : tid - kSides * kSetupChains - 3 * c;        // >= 3: no rectangle
+    const double* th = theta + (size_t)(s_idx[c] < 0 ? 0 : s_idx[c]) * L.nparams;
+    if (on_side && s_idx[c] >= 0) {
+        const Vec3 p = cdm_corner(th, L, s_sc[c], r, e & 3);
+        s_V[c][r][e & 3] = p;
+        if (p.z > 0.0) atomicOr(&s_above[c], 1u);
     }
-    const double* th = theta + (size_t)i * L.nparams;
-    Vec3 V[3][4];
-    if (cdm_corners(th, L, V)) {
-        if (chain_status) chain_status[i] |= CHAIN_ABOVE_SURFACE;
-        key[t] = -2;
-        return;
+    __syncthreads();
+    const bool live = s_idx[c] >= 0 && !s_above[c];
+    const uint32_t use = live ? rects_used(th[L.axes_idx], th[L.axes_idx + 1], th[L.axes_idx + 2]) : 0u;
+    if (tid < kSetupChains && s_idx[tid] >= 0 && s_above[tid]) {
+        if (chain_status) chain_status[s_idx[tid]] |= CHAIN_ABOVE_SURFACE;
+        if (ORDERED) key[t0 + tid] = -2;
     }
+    // the plan (cdm_plan): far rectangles, sides that take part and near-vertical ones
+    if (r < 3 && (use >> r & 1u)) {
+        if (on_side) {
+            bool act, steep;
+            side_class(s_V[c][r][e & 3], s_V[c][r][(e + 1) & 3], act, steep);
+            if (act) atomicOr(&s_bits[c], (1u << e) | (steep ? 1u << (kSides + e) : 0u));
+        } else {
+            int n1 = 0, n2 = 0;
+            const bool far = far_rect(s_V[c][r], n1, n2);
+            if (far) atomicOr(&s_bits[c], 1u << (24 + r));
+            s_nq[c][r] = far ? n1 | (n2 << 8) : 0;
+            Vec3 nrm = v_cross(v_sub(s_V[c][r][1], s_V[c][r][0]), v_sub(s_V[c][r][3], s_V[c][r][0]));
+            nrm = v_scale(nrm, 1.0 / sqrt(v_dot(nrm, nrm)));
+            s_slip[c][r] = v_scale(nrm, th[L.strength_idx]);
+        }
+    }
+    __syncthreads();
+    uint32_t mask = s_bits[c];
+    for (int q = 0; q < 3; ++q) {
+        if (mask >> (24 + q) & 1u) mask &= ~((0xFu << (4 * q)) | (0xFu << (kSides + 4 * q)));
+        if ((mask >> (24 + q) & 1u) || (mask >> (4 * q) & 0xFu)) mask |= 1u << (27 + q);
+    }
+    ChainC& C = s_chain[c];
     const double x0 = th[L.x_idx], y0 = th[L.x_idx + 1];
-    float x0h, x0l, y0h, y0l;
-    split_hilo(x0, x0h, x0l);
-    split_hilo(y0, y0h, y0l);
-    RectQ rect[3];
-    const uint32_t mask = cdm_rects(th, L, V, x0, y0, rect);
-    const int stride = ntiles > 16 ? ntiles / 16 : 1;
-    const int b = cost_bucket((uint32_t)sampled_tile_work(rect, mask, tile_box, ntiles, stride, x0h, x0l, y0h, y0l));
-    key[t] = (int8_t)b;
-    atomicAdd(&hdr->hist[b], 1);
+    if (live && on_side && (mask >> e & 1u))
+        fill_side(C.side[e], s_V[c][r][e & 3], s_V[c][r][(e + 1) & 3], s_slip[c][r], L.nu, x0, y0,
+                  (mask >> (kSides + e)) & 1u);
+    if (live && !on_side && r < 3 && (mask >> (27 + r) & 1u)) {
+        int sf, su;
+        rect_side_work(mask, r, sf, su);
+        const int nq = s_nq[c][r];
+        fill_rect(C.rect[r], s_V[c][r], th[L.strength_idx], L.nu, x0, y0, sf, nq & 255, nq >> 8);
+    }
+    if (tid >= kSetupThreads - kSetupChains) {
+        const int k = tid - (kSetupThreads - kSetupChains), i = s_idx[k];
+        if (i >= 0 && !s_above[k]) {
+            const double* p = theta + (size_t)i * L.nparams;
+            uint32_t m = s_bits[k];
+            for (int q = 0; q < 3; ++q) {
+                if (m >> (24 + q) & 1u) m &= ~((0xFu << (4 * q)) | (0xFu << (kSides + 4 * q)));
+                if ((m >> (24 + q) & 1u) || (m >> (4 * q) & 0xFu)) m |= 1u << (27 + q);
+            }
+            ChainC& K = s_chain[k];
+            split_hilo(p[L.x_idx], K.hdr.x, K.hdr.y);
+            split_hilo(p[L.x_idx + 1], K.hdr.z, K.hdr.w);
+            for (int o = 0; o < kMaxOffsets; ++o) K.off[o] = (o < noffsets) ? (float)p[L.offset_idx + o] : 0.f;
+            K.side_mask = m | 0x80000000u;      // a chain with no active side still needs a llk
+            K.chain = i;
+        }
+    }
+    __syncthreads();
+    if (ORDERED) {
+        // work per station averaged over every stride-th station tile (tile boxes relative to the
+        // source centre as the likelihood kernel forms them)
+        const int stride = ntiles > 16 ? ntiles / 16 : 1;
+        const int first = stride / 2, samples = first < ntiles ? (ntiles - 1 - first) / stride + 1 : 0;
+        for (int k = tid; k < kSetupChains * samples; k += kSetupThreads) {
+            const int q = k / samples;
+            if (s_idx[q] < 0 || s_above[q]) continue;
+            const ChainC& K = s_chain[q];
+            const float4 tb = __ldg(tile_box + first + (k - q * samples) * stride);
+            uint32_t fl, su;
+            tile_work(K.rect, K.side_mask, __fsub_rn(__fsub_rn(tb.x, K.hdr.x), K.hdr.y),
+                      __fsub_rn(__fsub_rn(tb.y, K.hdr.x), K.hdr.y), __fsub_rn(__fsub_rn(tb.z, K.hdr.z), K.hdr.w),
+                      __fsub_rn(__fsub_rn(tb.w, K.hdr.z), K.hdr.w), fl, su);
+            atomicAdd(&s_flop[q], fl);
+        }
+        __syncthreads();
+        if (tid < kSetupChains && s_idx[tid] >= 0 && !s_above[tid]) {
+            const int b = (int)(s_flop[tid] / (uint32_t)(samples * kCostBucketFlop));
+            key[t0 + tid] = (int8_t)(b < kCostBuckets ? b : kCostBuckets - 1);
+            atomicAdd(&hdr->hist[b < kCostBuckets ? b : kCostBuckets - 1], 1);
+        }
+    } else if (tid < kSetupChains && s_idx[tid] >= 0 && !s_above[tid]) {
+        slot_row[atomicAdd(&hdr->nslots, 1)] = t0 + tid;
+    }
+    // the rows of chains with work, by 16-byte stores
+    constexpr int nvec = sizeof(ChainC) / 16;
+    for (int k = tid; k < kSetupChains * nvec; k += kSetupThreads) {
+        const int q = k / nvec;
+        if (s_idx[q] < 0 || s_above[q]) continue;
+        reinterpret_cast<float4*>(out + t0)[k] = reinterpret_cast<const float4*>(s_chain)[k];
+    }
 }
 
 // Every chain with work takes the next slot of its cost bucket (buckets in decreasing cost;
-// the order inside a bucket is that of the atomic, which does not affect any chain's result)
-// and writes its constants there, so the likelihood kernel's CTAs hold only chains with work.
-__global__ void cdm_setup_kernel(ag_layout L, const double* __restrict__ theta, int n,
-                                 const int8_t* __restrict__ key, ChainC* __restrict__ out, int noffsets,
-                                 const int32_t* __restrict__ index_in, const int32_t* __restrict__ count_in,
-                                 int32_t* __restrict__ index_out, SetupHdr* __restrict__ hdr) {
+// the order inside a bucket is that of the atomic, which does not affect any chain's result), so
+// the likelihood kernel's CTAs hold only chains with work.
+__global__ void cdm_slot_kernel(int n, const int8_t* __restrict__ key, const int32_t* __restrict__ count_in,
+                                int32_t* __restrict__ slot_row, SetupHdr* __restrict__ hdr) {
     __shared__ int s_start[kCostBuckets];
     if (threadIdx.x == 0) {
         int acc = 0;
@@ -152,30 +247,9 @@ __global__ void cdm_setup_kernel(ag_layout L, const double* __restrict__ theta, 
     }
     __syncthreads();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    int i = t;
-    if (index_in) {
-        if (t >= *count_in) return;
-        i = index_in[t];
-    }
+    if (t >= (count_in ? min(n, *count_in) : n)) return;
     const int b = key[t];
-    if (b < 0) return;
-    const double* th = theta + (size_t)i * L.nparams;
-    Vec3 V[3][4];
-    cdm_corners(th, L, V);
-    const int slot = s_start[b] + atomicAdd(&hdr->fill[b], 1);
-    index_out[slot] = i;
-    ChainC& C = out[slot];
-    C.side_mask = 0u;
-    C.status = 0u;
-    const double x0 = th[L.x_idx], y0 = th[L.x_idx + 1];
-    split_hilo(x0, C.hdr.x, C.hdr.y);
-    split_hilo(y0, C.hdr.z, C.hdr.w);
-    for (int k = 0; k < kMaxOffsets; ++k)
-        C.off[k] = (k < noffsets) ? (float)th[L.offset_idx + k] : 0.f;
-    const uint32_t mask = cdm_sides(th, L, V, x0, y0, C.side, C.rect);
-    // a chain with no active side still needs a llk: keep bit 31 as "evaluate"
-    C.side_mask = mask | 0x80000000u;
+    if (b >= 0) slot_row[s_start[b] + atomicAdd(&hdr->fill[b], 1)] = t;
 }
 
 __global__ void cdm_check_kernel(ag_layout L, const double* __restrict__ theta, int n,
@@ -248,15 +322,31 @@ __global__ void station_boxes_kernel(const float4* __restrict__ xy, int m, int n
 // refills that buffer with the tile STAGES ahead.  No CTA-wide barrier is
 // taken per tile, so warps drift apart by up to STAGES - 1 tiles instead of
 // waiting for the slowest one at every tile.
-template <int WARPS, int MINB, int SPL, int STAGES>
+//
+// The misfit is summed in kParts fixed parts of the tiles: each lane adds its stations of a part
+// in float-float, the warp adds the lanes in FP64, and the parts are added in order, so a chain's
+// log-likelihood has the same bits whoever computes its parts.  SPLIT (one warp per CTA): the
+// CTAs (slot, y) of one chain take consecutive parts each and the last to finish adds them up.
+// One warp per chain leaves most of the GPU idle below ~1,800 chains (12 resident CTAs on 152
+// SMs) and ends in a ragged last wave up to a few times that (figures at kSplitChains).
+constexpr int kParts = 32;
+
+__host__ __device__ constexpr int part_begin(int k, int ntiles) { return (int)((long)k * ntiles / kParts); }
+// first tile of share y of splits: whole parts, or whole tiles where a part has at most one
+__host__ __device__ constexpr int split_begin(int y, int splits, int ntiles) {
+    return ntiles <= kParts ? y * ntiles / splits : part_begin(y * kParts / splits, ntiles);
+}
+
+template <int WARPS, int MINB, int SPL, int STAGES, bool SPLIT = false>
 __global__ void __launch_bounds__(WARPS * 32, MINB)
-cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ slot_chain,
+cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ slot_row,
                const int32_t* __restrict__ nslots_ptr, int n, const float4* __restrict__ xy,
                const float4* __restrict__ losd, const float* __restrict__ wt,
                const int32_t* __restrict__ oid, const float4* __restrict__ tile_box,
                const int32_t* __restrict__ order, int m, int m_padded, double norm,
                const double* __restrict__ llk_floor, double* __restrict__ llk, float* __restrict__ resid,
-               uint32_t* __restrict__ flags) {
+               uint32_t* __restrict__ flags, double* __restrict__ parts, int* __restrict__ done) {
+    static_assert(!SPLIT || WARPS == 1, "the stations of a chain are split over CTAs of one warp");
     const int nslots = min(n, *nslots_ptr);
     if ((int)(blockIdx.x * WARPS) >= nslots) return;       // whole CTA past the active chains
     __shared__ ChainC s_chain[WARPS];
@@ -271,14 +361,17 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
     // each warp's quadrature nodes: one buffer per rectangle (one shared by the three where
     // shared memory is short), regenerated only when a tile needs other node counts
     constexpr int kNodeBufs = WARPS <= 4 ? 3 : 1;
-    __shared__ float4 s_node[WARPS][kNodeBufs][kQuadBudget];
+    // (several stations per lane: packed nodes)
+    typedef typename std::conditional<(SPL > 1), PackedNode, float4>::type Node;
+    __shared__ __align__(16) Node s_node[WARPS][kNodeBufs][kQuadBudget];
     __shared__ float s_gx[136], s_gw[136];             // Gauss-Legendre rules (FP32)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = blockIdx.x * WARPS + warp;
     const bool active = slot < nslots;
-    const int chain = active ? slot_chain[slot] : n;
     const int ntiles = m_padded / kTile;
+    const int tile0 = SPLIT ? split_begin(blockIdx.y, gridDim.y, ntiles) : 0;
+    const int tile1 = SPLIT ? split_begin(blockIdx.y + 1, gridDim.y, ntiles) : ntiles;
     const bool with_oid = (oid != nullptr);
     const uint32_t tile_bytes = kTile * (16u + 16u + 4u) + (with_oid ? kTile * 4u : 0u) + 16u;
 
@@ -288,7 +381,7 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
     }
     // this warp's chain constants
     if (active) {
-        const float4* src = reinterpret_cast<const float4*>(chains + slot);
+        const float4* src = reinterpret_cast<const float4*>(chains + slot_row[slot]);
         float4* dst = reinterpret_cast<float4*>(&s_chain[warp]);
         constexpr int nvec = sizeof(ChainC) / 16;
         for (int k = lane; k < nvec; k += 32) dst[k] = src[k];
@@ -308,12 +401,13 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
             s_done[b] = 0;
         }
         fence_mbar_init();
-        const int first = ntiles < STAGES ? ntiles : STAGES;
-        for (int t = 0; t < first; ++t) issue(t, t);
+        const int first = tile1 - tile0 < STAGES ? tile1 - tile0 : STAGES;
+        for (int t = 0; t < first; ++t) issue(tile0 + t, t);
         s_issued = first;
     }
     __syncthreads();
     const ChainC& C = s_chain[warp];
+    const int chain = active ? C.chain : n;
     const uint32_t smask = active ? C.side_mask : 0u;
     const float x0h = C.hdr.x, x0l = C.hdr.y, y0h = C.hdr.z, y0l = C.hdr.w;
     ff acc{0.f, 0.f};
@@ -324,10 +418,18 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
     // remaining stations are skipped (the llk is then reported as -inf)
     const double floor_llk = (llk_floor && active && !resid) ? llk_floor[chain] : -INFINITY;
     bool stopped = false;
-    int t_stop = ntiles;
-    for (int t = 0; t < ntiles; ++t) {
-        const int buf = t % STAGES;
-        const uint32_t phase = (uint32_t)(t / STAGES) & 1u;
+    int u_stop = tile1 - tile0;
+    // the finished parts' sum and the part at work, kept out of the registers of the tile loop
+    __shared__ double s_sum[WARPS];
+    __shared__ int s_part[WARPS];
+    if (lane == 0) {
+        s_sum[warp] = 0.0;
+        s_part[warp] = 0;
+    }
+    __syncwarp();
+    for (int t = tile0; t < tile1; ++t) {
+        const int u = t - tile0, buf = u % STAGES;
+        const uint32_t phase = (uint32_t)(u / STAGES) & 1u;
         const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[buf], phase, kWaitLimit));
         if (!ok) {
             failed = true;
@@ -352,13 +454,20 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
             }
             // one rectangle's nodes in this warp's buffer (every lane reads all of them); the
             // buffer is refilled only when it holds other nodes
-            auto load_nodes = [&](int r) -> const float4* {
+            auto load_nodes = [&](int r) -> const Node* {
                 const int n1 = (qpack >> (10 * r)) & 31, n2 = (qpack >> (10 * r + 5)) & 31;
                 const int b = kNodeBufs == 3 ? r : 0;
                 const uint64_t key = (uint64_t)(r | (n1 << 2) | (n2 << 7));
                 if (((node_keys >> (12 * b)) & 0xFFFull) != key) {
                     __syncwarp();
-                    if (lane < n1 * n2) s_node[warp][b][lane] = rect_node(C.rect[r], n1, n2, lane, s_gx, s_gw);
+                    if (lane < n1 * n2) {
+                        const float4 q = rect_node(C.rect[r], n1, n2, lane, s_gx, s_gw);
+                        if constexpr (SPL > 1)
+                            s_node[warp][b][lane] =
+                                PackedNode{make_float4(-q.x, -q.x, -q.y, -q.y), make_float4(q.z, q.z, q.w, q.w)};
+                        else
+                            s_node[warp][b][lane] = q;
+                    }
                     __syncwarp();
                     node_keys = (node_keys & ~(0xFFFull << (12 * b))) | (key << (12 * b));
                 }
@@ -400,9 +509,9 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
                     while (qm) {
                         const int r = __ffs(qm) - 1;
                         qm &= qm - 1;
-                        const float4* nodes = load_nodes(r);
-                        rect_quad<SV<SPL>>(C.rect[r], nodes, ((qpack >> (10 * r)) & 31) * ((qpack >> (10 * r + 5)) & 31),
-                                           Xr, Yr, ue, un, uv);
+                        const Node* nodes = load_nodes(r);
+                        const int nn = ((qpack >> (10 * r)) & 31) * ((qpack >> (10 * r + 5)) & 31);
+                        rect_quad_packed<SPL>(C.rect[r], nodes, nn, Xr, Yr, ue, un, uv);
                     }
 #pragma unroll
                     for (int q = 0; q < SPL; ++q) finish(ue.v[q], un.v[q], uv.v[q], j0 + 32 * q);
@@ -432,7 +541,20 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
                     finish(ue, un, uv, j);
                 }
             }
-            if (floor_llk > -INFINITY && norm - 0.5 * warp_sum(ff_to_double(acc)) < floor_llk) stopped = true;
+            if (floor_llk > -INFINITY && norm - 0.5 * (s_sum[warp] + warp_sum(ff_to_double(acc))) < floor_llk) stopped = true;
+            // the end of a part (parts without a tile are left out)
+            int part = s_part[warp];
+            while (part_begin(part + 1, ntiles) <= t) ++part;
+            if (t + 1 == part_begin(part + 1, ntiles)) {
+                const double p = warp_sum(ff_to_double(acc));
+                if (lane == 0) {
+                    if (SPLIT) __stcg(parts + (size_t)slot * kParts + part, p);
+                    s_sum[warp] += p;
+                    s_part[warp] = part + 1;
+                }
+                __syncwarp();
+                acc = ff{0.f, 0.f};
+            }
         }
         // done with this buffer: the last warp of the CTA to get here refills it
         __syncwarp();
@@ -441,7 +563,7 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
             if (atomicAdd(&s_done[buf], 1) == WARPS - 1) {
                 __threadfence_block();
                 s_done[buf] = 0;
-                if (t + STAGES < ntiles) {
+                if (t + STAGES < tile1) {
                     fence_proxy_async_smem();
                     issue(t + STAGES, buf);
                     atomicAdd(&s_issued, 1);
@@ -451,7 +573,7 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
         // a CTA of one stopped warp leaves the ring; CTAs of several warps keep counting tiles
         // (the stopped warp's share of each tile's completion) without computing
         if (WARPS == 1 && stopped) {
-            t_stop = t;
+            u_stop = u;
             break;
         }
     }
@@ -459,12 +581,10 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
         // wait (bounded) for the copies already issued into this CTA's ring before it exits
         if (lane == 0) {
             const int last = s_issued;
-            for (int t = t_stop + 1; t < last; ++t)
-                mbar_wait_bounded(&full[t % STAGES], (uint32_t)(t / STAGES) & 1u, kWaitLimit);
+            for (int u = u_stop + 1; u < last; ++u)
+                mbar_wait_bounded(&full[u % STAGES], (uint32_t)(u / STAGES) & 1u, kWaitLimit);
         }
         __syncwarp();
-        if (lane == 0) llk[chain] = -INFINITY;
-        return;
     }
     if (__syncthreads_or(failed)) {
         // a wait gave up: drain the copies still in flight (bounded) before the CTA exits
@@ -476,8 +596,28 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
         }
         return;
     }
-    const double sum = warp_sum(ff_to_double(acc));
-    if (lane == 0 && active) llk[chain] = stopped ? -INFINITY : norm - 0.5 * sum;
+    if (!SPLIT) {
+        if (lane == 0 && active) llk[chain] = stopped ? -INFINITY : norm - 0.5 * s_sum[warp];
+        return;
+    }
+    // the chain's last CTA adds its parts; a CTA that stopped below the floor says so in the count
+    int total = 0;
+    if (lane == 0) {
+        __threadfence();
+        total = atomicAdd(done + slot, stopped ? 0x10001 : 1) + (stopped ? 0x10001 : 1);
+        __threadfence();
+    }
+    total = __shfl_sync(0xffffffffu, total, 0);
+    if ((total & 0xFFFF) != (int)gridDim.y) return;
+    static_assert(kParts == 32, "one part per lane");
+    const bool full_part = part_begin(lane, ntiles) < part_begin(lane + 1, ntiles);
+    const double p = full_part && (total >> 16) == 0 ? __ldcg(parts + (size_t)slot * kParts + lane) : 0.0;
+    double sum = 0.0;
+    for (int k = 0; k < kParts; ++k) sum += __shfl_sync(0xffffffffu, p, k);
+    if (lane == 0) {
+        const double v = norm - 0.5 * sum;
+        llk[chain] = (total >> 16) != 0 || v < floor_llk ? -INFINITY : v;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -584,9 +724,10 @@ mogi_llk_kernel(ag_layout L, const double* __restrict__ theta, int n,
 using namespace ag;
 
 // CDM launch variants: warps (= chains) per CTA and resident CTAs per SM the
-// register allocation targets; chosen per problem by the autotuner
+// register allocation targets; 0, the default, splits the stations of few chains over CTAs and is
+// variant 11, the fastest of them at 32,768 x 40,000, for many; the others are chosen per problem by the autotuner
 struct CdmVariant { int warps; };
-static constexpr CdmVariant kCdmVariants[] = {{8}, {4}, {4}, {2}, {4}, {4}, {2}, {4}, {4}, {4}, {4}, {1}, {1}, {1}, {2}};
+static constexpr CdmVariant kCdmVariants[] = {{1}, {4}, {4}, {2}, {4}, {4}, {2}, {4}, {4}, {4}, {4}, {1}, {1}, {1}, {2}};
 static constexpr int kCdmVariantCount = 15;
 // Mogi launch variants: chains per CTA held in registers (16, 8, 32)
 static constexpr int kMogiChainsOf[] = {16, 8, 32};
@@ -596,15 +737,53 @@ extern "C" int32_t ag_forward_variants(int model) {
     return model == AG_MODEL_CDM ? kCdmVariantCount : model == AG_MODEL_MOGI ? kMogiVariantCount : 0;
 }
 
-// CDM workspace: compacted chain constants, the chain of each slot, the set-up header (slot
-// count and cost histogram), each requested chain's cost bucket
+// Chains up to which a launch of the default variant splits the stations of a chain over CTAs, and
+// the CTAs it aims at: 152 SMs x 12 resident CTAs, eight times over, so that the last wave is a small
+// share.  Split against one CTA per chain, slots ordered by cost (chains x stations): 64 x 577
+// 45 against 79 µs, 256 x 40,000 665 against 1,928, 1,024 x 5,000 422 against 492, 3,000 x 12,000
+// 2,189 against 2,211, but 4,096 x 2,500 756 against 689 and 8,100 x 10,000 4,151 against 3,986:
+// the order by cost then does more for the last wave.
+constexpr int kSplitChains = 3072;
+constexpr int kSplitCtas = 8 * 152 * 12;
+static int station_splits(int n, int ntiles) {
+    int s = (kSplitCtas - 1) / n + 1;
+    if (s > kParts) s = kParts;
+    return s < ntiles ? s : ntiles;
+}
+
+// CDM workspace: chain constants, the row of each slot, the set-up header (slot count and cost
+// histogram), each requested chain's cost bucket; for up to kSplitChains chains also the finished
+// CTAs and the partial misfits of each slot
+struct CdmWorkspace {
+    ChainC* chains;
+    int32_t* slot_row;
+    SetupHdr* hdr;
+    int32_t* done;
+    int8_t* key;
+    double* parts;
+};
 static size_t al256(size_t b) { return (b + 255) / 256 * 256; }
+static size_t cdm_workspace(char* base, int n, CdmWorkspace* w) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char* p = base + at;
+        at += al256(bytes);
+        return p;
+    };
+    const size_t split = n <= kSplitChains ? n : 0;
+    CdmWorkspace ws;
+    ws.chains = reinterpret_cast<ChainC*>(take((size_t)n * sizeof(ChainC)));
+    ws.slot_row = reinterpret_cast<int32_t*>(take((size_t)n * sizeof(int32_t)));
+    ws.hdr = reinterpret_cast<SetupHdr*>(take(sizeof(SetupHdr)));
+    ws.done = reinterpret_cast<int32_t*>(take(split * sizeof(int32_t)));     // cleared with the header
+    ws.key = reinterpret_cast<int8_t*>(take((size_t)n));
+    ws.parts = reinterpret_cast<double*>(take(split * kParts * sizeof(double)));
+    if (w) *w = ws;
+    return at;
+}
 
 extern "C" size_t ag_forward_workspace_bytes(int model, int32_t n) {
-    if (model == AG_MODEL_CDM && n > 0)
-        return al256((size_t)n * sizeof(ChainC)) + al256((size_t)n * sizeof(int32_t)) + al256(sizeof(SetupHdr)) +
-               al256((size_t)n);
-    return 0;
+    return model == AG_MODEL_CDM && n > 0 ? cdm_workspace(nullptr, n, nullptr) : 0;
 }
 
 static int check_stations(const ag_station_set* st) {
@@ -653,35 +832,47 @@ static int forward_llk(int model, const ag_layout* layout, const double* theta, 
                    "the CDM needs the stations' tile boxes (ag_station_boxes), 16-byte aligned");
         const float4* tile_box = reinterpret_cast<const float4*>(st->tile_box);
         const int ntiles = st->m_padded / AG_STATION_TILE;
-        ChainC* chains = reinterpret_cast<ChainC*>(workspace);
-        int32_t* slot_chain = reinterpret_cast<int32_t*>(static_cast<char*>(workspace) +
-                                                         al256((size_t)n * sizeof(ChainC)));
-        SetupHdr* hdr = reinterpret_cast<SetupHdr*>(reinterpret_cast<char*>(slot_chain) +
-                                                    al256((size_t)n * sizeof(int32_t)));
-        int8_t* key = reinterpret_cast<int8_t*>(reinterpret_cast<char*>(hdr) + al256(sizeof(SetupHdr)));
-        int32_t* nslots = &hdr->nslots;
-        rc = cuda_status(cudaMemsetAsync(hdr, 0, sizeof(SetupHdr), s), "cudaMemsetAsync(set-up header)");
-        if (rc) return rc;
-        cdm_cost_kernel<<<(n + 127) / 128, 128, 0, s>>>(L, theta, n, mask_in, chain_status, index, count, tile_box,
-                                                        ntiles, key, hdr);
-        rc = launch_status("cdm_cost_kernel");
-        if (rc) return rc;
-        cdm_setup_kernel<<<(n + 127) / 128, 128, 0, s>>>(L, theta, n, key, chains, noffsets, index, count,
-                                                         slot_chain, hdr);
-        rc = launch_status("cdm_setup_kernel");
-        if (rc) return rc;
+        CdmWorkspace ws;
+        cdm_workspace(static_cast<char*>(workspace), n, &ws);
+        int32_t* nslots = &ws.hdr->nslots;
         const int v = L.variant;
         AG_REQUIRE(v >= 0 && v < kCdmVariantCount, "CDM variant %d out of range [0, %d)", v, kCdmVariantCount);
+        const bool split = v == 0 && n <= kSplitChains;
+        rc = cuda_status(cudaMemsetAsync(ws.hdr, 0, al256(sizeof(SetupHdr)) + (split ? (size_t)n * sizeof(int32_t) : 0),
+                                         s),
+                         "cudaMemsetAsync(set-up header)");
+        if (rc) return rc;
+        const int setup_ctas = (n + kSetupChains - 1) / kSetupChains;
+        if (split) {
+            cdm_setup_kernel<false><<<setup_ctas, kSetupThreads, 0, s>>>(L, theta, n, mask_in, chain_status, index,
+                                                                        count, noffsets, tile_box, ntiles, ws.chains,
+                                                                        ws.key, ws.slot_row, ws.hdr);
+        } else {
+            cdm_setup_kernel<true><<<setup_ctas, kSetupThreads, 0, s>>>(L, theta, n, mask_in, chain_status, index,
+                                                                       count, noffsets, tile_box, ntiles, ws.chains,
+                                                                       ws.key, ws.slot_row, ws.hdr);
+            cdm_slot_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, ws.key, count, ws.slot_row, ws.hdr);
+        }
+        rc = launch_status("cdm set-up kernels");
+        if (rc) return rc;
+        if (split) {
+            const dim3 grid(n, station_splits(n, ntiles));
+            cdm_llk_kernel<1, 12, 4, 2, true><<<grid, 32, 0, s>>>(
+                ws.chains, ws.slot_row, nslots, n, xy, ld, st->weight, st->oid, tile_box, st->order, st->m,
+                st->m_padded, norm, llk_floor, llk, residuals, nullptr, ws.parts, ws.done);
+            return launch_status("cdm_llk_kernel (split)");
+        }
         const int warps = kCdmVariants[v].warps;
         const int grid = (n + warps - 1) / warps;
-#define AG_CDM_LAUNCH(W, B, SPL, ST)                                                                    \
-    cdm_llk_kernel<W, B, SPL, ST><<<grid, W * 32, 0, s>>>(chains, slot_chain, nslots, n, xy, ld, st->weight, \
+#define AG_CDM_LAUNCH(W, B, SPL, ST)                                                                             \
+    cdm_llk_kernel<W, B, SPL, ST><<<grid, W * 32, 0, s>>>(ws.chains, ws.slot_row, nslots, n, xy, ld, st->weight, \
                                                           st->oid, tile_box, st->order, st->m, st->m_padded,     \
-                                                          norm, llk_floor, llk, residuals, nullptr)
+                                                          norm, llk_floor, llk, residuals, nullptr, nullptr,     \
+                                                          nullptr)
         // warps per CTA, CTAs per SM, stations per lane, ring depth; a CTA of one warp has its
         // own ring, so its chain never waits for another chain's tiles
         switch (v) {
-            case 0: AG_CDM_LAUNCH(8, 2, 1, 4); break;
+            case 0: AG_CDM_LAUNCH(1, 12, 4, 2); break;
             case 1: AG_CDM_LAUNCH(4, 4, 1, 4); break;
             case 2: AG_CDM_LAUNCH(4, 5, 1, 4); break;
             case 3: AG_CDM_LAUNCH(2, 8, 1, 4); break;
