@@ -153,20 +153,23 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const fl
 // x_hi W + x_lo W in FP32 accumulators: the activations keep ~16 bits beyond BF16 and the
 // weights are the BF16 copy the SIMT layers read too.  The kernel is the linear model's
 // persistent tcgen05 structure (TMA ring of 128B-swizzled K-major tiles, one thread issuing
-// tcgen05.mma into one of two TMEM accumulators, four epilogue warps reading the other with
+// tcgen05.mma into one of two TMEM accumulators, epilogue warps reading the other with
 // tcgen05.ld); the epilogue adds the bias, applies GELU and writes the next layer's split
 // BF16 input directly, plus the FP32 pre-activation Z and output Y where asked.
-constexpr int kMlpThreads = 192;
+// The epilogue bounds a layer: ~35 instructions an element, most of them the error function's.
+// Sixteen warps share it (eight for 64 columns): 27 µs for 32,768 x 256 x 256, 33 µs with four.
 
 template <int BN>
 struct MlpTc {
+    static constexpr int EPI = BN >= 128 ? 16 : 8;           // epilogue warps
+    static constexpr int THREADS = 64 + 32 * EPI;
     static constexpr uint32_t B_BYTES = BN * TC_BK * 2;
     static constexpr uint32_t STAGE = TC_A_BYTES + B_BYTES;
     static constexpr uint32_t SMEM = TC_STAGES * STAGE + 1024 + 256;
 };
 
 template <int BN>
-__global__ void __launch_bounds__(kMlpThreads, 1)
+__global__ void __launch_bounds__(MlpTc<BN>::THREADS, 1)
 mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' split BF16 activations
                     const __grid_constant__ CUtensorMap map_w,   // fo x K' packed BF16 weights
                     int n, int fo, int kblocks, int mtiles, int ntiles, const float* __restrict__ bias,
@@ -183,8 +186,11 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
     uint64_t* tfull = bars + 2 * TC_STAGES;
     uint64_t* tempty = bars + 2 * TC_STAGES + 2;
     uint64_t* drain = bars + 2 * TC_STAGES + 4;
+    constexpr int EPI = MlpTc<BN>::EPI, COLS = BN * 4 / EPI;  // columns per epilogue warp
+    static_assert(COLS % 32 == 0, "whole tcgen05.ld of 32 columns");
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
+    __shared__ __align__(16) float s_bias[EPI][COLS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total = mtiles * ntiles;
     if (threadIdx.x == 0) {
@@ -194,7 +200,7 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], 4);
+            mbar_init(&tempty[b], EPI);
         }
         mbar_init(drain, 1);
         fence_mbar_init();
@@ -263,60 +269,67 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
         }
         mma_commit(smem_addr(drain));
     } else if (warp >= 2) {
-        // epilogue: thread = row of the tile (TMEM lane quarter of this warp)
-        const int quarter = warp & 3;
+        // epilogue: thread = row of the tile (TMEM lane quarter of this warp), the warps of a
+        // quarter share the columns
+        const int quarter = warp & 3, first = (warp - 2) / 4 * COLS;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        float* bs = s_bias[warp - 2];
         int local = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++local) {
             const int b = local & 1;
+            const int mt = t % mtiles, nt = t / mtiles;
+            const int n0 = nt * BN + first;                            // fo is a multiple of BN
+            for (int c = lane; c < COLS; c += 32) bs[c] = __ldg(bias + n0 + c);
             const bool ok = __all_sync(0xffffffffu,
                                        mbar_wait_bounded(&tfull[b], (uint32_t)(local >> 1) & 1u, TC_WAIT));
             if (!ok || aborted()) {
                 if (lane == 0) atomicExch(&s_abort, 1);
                 break;
             }
+            __syncwarp();
             tc_fence_after();
-            const int mt = t % mtiles, nt = t / mtiles;
-            const int n0 = nt * BN;
             const int row = mt * TC_BM + quarter * 32 + lane;
             const bool live = row < n;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
+            for (int c0 = 0; c0 < COLS; c0 += 32) {
                 uint32_t r[32];
-                tmem_ld32_nowait(tmem + lane_base + (uint32_t)(b * BN + c0), r);
-                const float bl = __ldg(bias + n0 + c0 + lane);        // fo is a multiple of BN
+                tmem_ld32_nowait(tmem + lane_base + (uint32_t)(b * BN + first + c0), r);
                 tmem_wait_ld();
-                float z[32], y[32];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    z[i] = __uint_as_float(r[i]) + __shfl_sync(0xffffffffu, bl, i);
-                    y[i] = gelu_on ? gelu(z[i]) : z[i];
-                }
-                if (!live) continue;
                 const size_t o = (size_t)row * fo + n0 + c0;
-                if (Z) {
+                __nv_bfloat16* hi = xnext + (size_t)row * (2 * kp_next) + n0 + c0;
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(Z + o + i) = make_float4(z[i], z[i + 1], z[i + 2], z[i + 3]);
-                }
-                if (Y) {
+                for (int i = 0; i < 32; i += 8) {
+                    float z[8], y[8];
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(Y + o + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
-                }
-                if (xnext) {
-                    __nv_bfloat16* hi = xnext + (size_t)row * (2 * kp_next) + n0 + c0;
-                    __nv_bfloat16* lo = hi + kp_next;
+                    for (int q = 0; q < 8; q += 4) {
+                        const float4 bb = *reinterpret_cast<const float4*>(bs + c0 + i + q);
+                        z[q] = __uint_as_float(r[i + q]) + bb.x;
+                        z[q + 1] = __uint_as_float(r[i + q + 1]) + bb.y;
+                        z[q + 2] = __uint_as_float(r[i + q + 2]) + bb.z;
+                        z[q + 3] = __uint_as_float(r[i + q + 3]) + bb.w;
+                    }
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        __align__(16) __nv_bfloat16 h8[8], l8[8];
+                    for (int q = 0; q < 8; ++q) y[q] = gelu_on ? gelu(z[q]) : z[q];
+                    if (live && Z) {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            h8[q] = __float2bfloat16_rn(y[i + q]);
-                            l8[q] = __float2bfloat16_rn(y[i + q] - __bfloat162float(h8[q]));
+                        for (int q = 0; q < 8; q += 4)
+                            *reinterpret_cast<float4*>(Z + o + i + q) = make_float4(z[q], z[q + 1], z[q + 2], z[q + 3]);
+                    }
+                    if (live && Y) {
+#pragma unroll
+                        for (int q = 0; q < 8; q += 4)
+                            *reinterpret_cast<float4*>(Y + o + i + q) = make_float4(y[q], y[q + 1], y[q + 2], y[q + 3]);
+                    }
+                    if (live && xnext) {
+                        __align__(16) __nv_bfloat162 h2[4], l2[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            h2[q] = __floats2bfloat162_rn(y[2 * q], y[2 * q + 1]);
+                            l2[q] = __floats2bfloat162_rn(y[2 * q] - __low2float(h2[q]),
+                                                          y[2 * q + 1] - __high2float(h2[q]));
                         }
-                        *reinterpret_cast<uint4*>(hi + i) = *reinterpret_cast<const uint4*>(h8);
-                        *reinterpret_cast<uint4*>(lo + i) = *reinterpret_cast<const uint4*>(l8);
+                        *reinterpret_cast<uint4*>(hi + i) = *reinterpret_cast<const uint4*>(h2);
+                        *reinterpret_cast<uint4*>(hi + kp_next + i) = *reinterpret_cast<const uint4*>(l2);
                     }
                 }
             }
@@ -340,16 +353,24 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
     }
 }
 
-// x (n x fi FP32) -> split BF16 rows [x_hi | 0 .. | x_lo | 0 ..] of width 2 kp
+// x (n x fi FP32) -> split BF16 rows [x_hi | 0 .. | x_lo | 0 ..] of width 2 kp; a thread per 8
+// columns of a row
 __global__ void split_rows_kernel(const float* __restrict__ x, int n, int fi, int kp,
                                   __nv_bfloat16* __restrict__ xs) {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long)n * kp) return;
-    const int r = (int)(e / kp), k = (int)(e % kp);
-    const float v = (k < fi) ? x[(size_t)r * fi + k] : 0.f;
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    xs[(size_t)r * 2 * kp + k] = h;
-    xs[(size_t)r * 2 * kp + kp + k] = __float2bfloat16_rn(v - __bfloat162float(h));
+    const int groups = kp >> 3;
+    const long r = e / groups;
+    const int k0 = (int)(e - r * groups) * 8;
+    if (r >= n) return;
+    __align__(16) __nv_bfloat16 hi[8], lo[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const float v = (k0 + q < fi) ? __ldg(x + r * fi + k0 + q) : 0.f;
+        hi[q] = __float2bfloat16_rn(v);
+        lo[q] = __float2bfloat16_rn(v - __bfloat162float(hi[q]));
+    }
+    *reinterpret_cast<uint4*>(xs + r * 2 * kp + k0) = *reinterpret_cast<const uint4*>(hi);
+    *reinterpret_cast<uint4*>(xs + r * 2 * kp + kp + k0) = *reinterpret_cast<const uint4*>(lo);
 }
 
 // W (fo x fi BF16) -> [W | W] of width 2 kp, zeros past fi
@@ -363,14 +384,25 @@ __global__ void pack_weights_kernel(const __nv_bfloat16* __restrict__ w, int fo,
     out[(size_t)o * 2 * kp + kp + k] = v;
 }
 
-// θ (FP64, N x p) -> x = 2 (θ - lo)/(hi - lo) - 1 (FP32); optional index list
+// θ (FP64, N x p) -> x = 2 (θ - lo)/(hi - lo) - 1 (FP32).  A thread keeps to one parameter j and
+// walks the rows, so that the division (~20 FP64 instructions) is made once for its rows; the FP32
+// result differs from the division's by its last bit at most, once in 2^28 elements.
+constexpr int kNormRows = 8;
 __global__ void normalize_kernel(const double* __restrict__ theta, int n, int p,
                                  const double* __restrict__ lo, const double* __restrict__ hi,
                                  float* __restrict__ x) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n * p) return;
-    const int j = e % p;
-    x[e] = (float)(2.0 * (theta[e] - lo[j]) / (hi[j] - lo[j]) - 1.0);
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long band = e / p;
+    const int j = (int)(e - band * p);
+    const long i0 = band * kNormRows;
+    if (i0 >= n) return;
+    const double l = lo[j], s = 2.0 / (hi[j] - l);
+    double v[kNormRows];
+#pragma unroll
+    for (int q = 0; q < kNormRows; ++q) v[q] = i0 + q < n ? __ldg(theta + (i0 + q) * p + j) : 0.0;
+#pragma unroll
+    for (int q = 0; q < kNormRows; ++q)
+        if (i0 + q < n) x[(i0 + q) * p + j] = (float)fma(v[q] - l, s, -1.0);
 }
 
 // dZ = dY ⊙ GELU'(Z)
@@ -429,40 +461,106 @@ __global__ void to_bf16_kernel(long count, const float* __restrict__ p, __nv_bfl
     if (e < count) q[e] = __float2bfloat16_rn(p[e]);
 }
 
-// llk_s = norm - ½ (q0 - 2 hᵀ c̃ + c̃ᵀ G c̃), c̃ = scale ⊙ c ; one warp per chain.  Each CTA
-// stages Gᵀ in shared memory once (lane a then reads column a of a row of Gᵀ: consecutive
-// words, no bank conflict) and walks chains with a grid stride; the warp's c̃ goes through
-// shared memory and is read as a broadcast.
+// llk_s = norm - ½ (q0 - 2 hᵀ c̃ + c̃ᵀ G c̃), c̃ = scale ⊙ c.  A CTA takes kSurChains chains; a thread forms
+// kSurRows rows of G c̃ for eight chains, so that four 16-byte shared-memory loads feed 64 FMAs
+// (shared-memory wavefronts bound it otherwise: with eight FMAs per three loads 34 µs for 32,768
+// chains and 64 coefficients).  Its FP32 terms are added exactly in float-float and the threads
+// of a chain in order (FP64 products and sums in a warp per chain took 61 µs at the FP64
+// pipe's rate).  Measured: 24 µs; staging the operands by 4-byte loads, 58 µs.
 constexpr int kSurMaxK = 96;
-constexpr int kSurWarps = 8;
-__global__ void __launch_bounds__(kSurWarps * 32)
+constexpr int kSurChains = 128;
+constexpr int kSurStride = kSurChains + 4;   // row of c̃: 16-byte aligned, spread over the banks
+constexpr int kSurRows = 8;
+static int sur_groups(int k) { return (k + kSurRows - 1) / kSurRows; }
+static size_t sur_smem(int k) {
+    return ((size_t)k * kSurRows * sur_groups(k) + (size_t)k * kSurStride + 2 * (size_t)sur_groups(k) * kSurChains) *
+           sizeof(float);
+}
+
+__global__ void __launch_bounds__(kSurChains / 8 * (kSurMaxK / kSurRows))
 surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float* __restrict__ scale,
                      const float* __restrict__ G, const float* __restrict__ h, double q0, double norm,
                      double* __restrict__ llk) {
-    extern __shared__ float s_mem[];
-    float* sGT = s_mem;                                  // k x k, sGT[b k + a] = G[a k + b]
-    float* sc = s_mem + k * k + (threadIdx.x >> 5) * k;  // this warp's c̃
-    for (int e = threadIdx.x; e < k * k; e += blockDim.x) {
-        const int a = e / k, b = e - a * k;
-        sGT[b * k + a] = G[e];
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int stride = gridDim.x * kSurWarps;
-    for (int i = blockIdx.x * kSurWarps + (threadIdx.x >> 5); i < n; i += stride) {
-        const float* c = coeff + (long)i * k;
-        for (int b = lane; b < k; b += 32) sc[b] = c[b] * scale[b];
-        __syncwarp();
-        double acc = 0.0;
-        for (int a = lane; a < k; a += 32) {
-            const float ca = sc[a];
-            float row = 0.f;
-            for (int b = 0; b < k; ++b) row = fmaf(sGT[b * k + a], sc[b], row);
-            acc += (double)ca * (double)row - 2.0 * (double)h[a] * (double)ca;
+    extern __shared__ __align__(16) float s_mem[];
+    const int groups = (k + kSurRows - 1) / kSurRows, rows = groups * kSurRows;
+    float* sGT = s_mem;                                  // [k][rows], sGT[b][a] = G[a][b]
+    float* sc = sGT + k * rows;                          // [k][kSurStride]
+    float2* s_part = reinterpret_cast<float2*>(sc + k * kSurStride);     // [groups][kSurChains]
+    const int tid = threadIdx.x, threads = kSurChains / 8 * groups;
+    const int c0 = tid % (kSurChains / 8) * 8, a0 = tid / (kSurChains / 8) * kSurRows;
+    const long i0 = (long)blockIdx.x * kSurChains;
+    const int chains = n - i0 < kSurChains ? (int)(n - i0) : kSurChains;
+    // staged by 16-byte loads, eight in flight per thread, where the rows allow
+    if (k % 4 == 0 && ((size_t)G | (size_t)coeff | (size_t)scale) % 16 == 0) {
+        const int kq = k / 4;
+#pragma unroll 8
+        for (int e = tid; e < k * kq; e += threads) {
+            const int a = e / kq, b = 4 * (e - a * kq);
+            const float4 v = __ldg(reinterpret_cast<const float4*>(G) + e);
+            float* to = sGT + b * rows + a;
+            to[0] = v.x; to[rows] = v.y; to[2 * rows] = v.z; to[3 * rows] = v.w;
         }
-        acc = warp_sum(acc);
-        if (lane == 0) llk[i] = norm - 0.5 * (q0 + acc);
-        __syncwarp();
+#pragma unroll 8
+        for (int e = tid; e < chains * kq; e += threads) {
+            const int q = e / kq, b = 4 * (e - q * kq);
+            const float4 v = __ldg(reinterpret_cast<const float4*>(coeff + i0 * k) + e);
+            const float4 f = __ldg(reinterpret_cast<const float4*>(scale + b));
+            float* to = sc + b * kSurStride + q;
+            to[0] = v.x * f.x; to[kSurStride] = v.y * f.y; to[2 * kSurStride] = v.z * f.z; to[3 * kSurStride] = v.w * f.w;
+        }
+    } else {
+        for (int e = tid; e < k * k; e += threads) {
+            const int a = e / k, b = e - a * k;
+            sGT[b * rows + a] = __ldg(G + e);
+        }
+        for (int e = tid; e < chains * k; e += threads) {
+            const int q = e / k, b = e - q * k;
+            sc[b * kSurStride + q] = __ldg(coeff + i0 * k + e) * __ldg(scale + b);
+        }
+    }
+    // rows past k and chains past n: zeros
+    for (int e = tid; e < (rows - k) * k; e += threads) sGT[e / (rows - k) * rows + k + e % (rows - k)] = 0.f;
+    for (int e = tid; e < (kSurChains - chains) * k; e += threads)
+        sc[e % k * kSurStride + chains + e / k] = 0.f;
+    __syncthreads();
+    float row[kSurRows][8] = {};
+#pragma unroll 2
+    for (int b = 0; b < k; ++b) {
+        float g[kSurRows], v[8];
+        *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(sGT + b * rows + a0);
+        *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(sGT + b * rows + a0 + 4);
+        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(sc + b * kSurStride + c0);
+        *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(sc + b * kSurStride + c0 + 4);
+#pragma unroll
+        for (int q = 0; q < kSurRows; ++q)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) row[q][c] = fmaf(g[q], v[c], row[q][c]);
+    }
+    ff acc[8] = {};
+#pragma unroll
+    for (int q = 0; q < kSurRows; ++q) {
+        if (a0 + q < k) {
+            const float h2 = -2.0f * __ldg(h + a0 + q);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float ca = sc[(a0 + q) * kSurStride + c0 + c];
+                float t = ca * row[q][c];
+                ff_add(acc[c], t, fmaf(ca, row[q][c], -t));
+                t = h2 * ca;
+                ff_add(acc[c], t, fmaf(h2, ca, -t));
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) s_part[a0 / kSurRows * kSurChains + c0 + c] = make_float2(acc[c].hi, acc[c].lo);
+    __syncthreads();
+    for (int c = tid; c < chains; c += threads) {
+        ff t{0.f, 0.f};
+        for (int g = 0; g < groups; ++g) {
+            const float2 p = s_part[g * kSurChains + c];
+            ff_add(t, p.x, p.y);
+        }
+        llk[i0 + c] = norm - 0.5 * (q0 + ff_to_double(t));
     }
 }
 
@@ -646,7 +744,7 @@ static int gemm(cudaStream_t s, int M, int N, int K, const float* A, long sam, l
 extern "C" int ag_normalize_inputs(const double* theta, int32_t n, int32_t p, const double* lo,
                                    const double* hi, float* x, void* stream) {
     AG_REQUIRE(theta && lo && hi && x && n > 0 && p > 0, "invalid arguments");
-    normalize_kernel<<<nblk((long)n * p, 256), 256, 0, as_stream(stream)>>>(theta, n, p, lo, hi, x);
+    normalize_kernel<<<nblk((long)nblk(n, kNormRows) * p, 128), 128, 0, as_stream(stream)>>>(theta, n, p, lo, hi, x);
     return launch_status("normalize_kernel");
 }
 
@@ -738,7 +836,7 @@ static int mlp_layer_launch(cudaStream_t s, const __nv_bfloat16* xs, int n, int 
     rc = sm_count(&sms);
     if (rc) return rc;
     const int mtiles = (n + TC_BM - 1) / TC_BM, ntiles = fo / BN, total = mtiles * ntiles;
-    mlp_layer_tc_kernel<BN><<<total < sms ? total : sms, kMlpThreads, MlpTc<BN>::SMEM, s>>>(
+    mlp_layer_tc_kernel<BN><<<total < sms ? total : sms, MlpTc<BN>::THREADS, MlpTc<BN>::SMEM, s>>>(
         mx, mw, n, fo, 2 * kp / TC_BK, mtiles, ntiles, bias, gelu_on, Z, Y, xnext, kp_next, flags);
     return launch_status("mlp_layer_tc_kernel");
 }
@@ -760,7 +858,7 @@ extern "C" int ag_mlp_forward_tc(const ag_mlp* net, const float* params, const u
     __nv_bfloat16* buf[2] = {reinterpret_cast<__nv_bfloat16*>(workspace),
                              reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(workspace) + need / 2)};
     const int fi0 = net->sizes[0], kp0 = mlp_kp(fi0);
-    split_rows_kernel<<<nblk((long)n * kp0, 256), 256, 0, s>>>(x, n, fi0, kp0, buf[0]);
+    split_rows_kernel<<<nblk((long)n * (kp0 / 8), 256), 256, 0, s>>>(x, n, fi0, kp0, buf[0]);
     rc = launch_status("split_rows_kernel");
     if (rc) return rc;
     const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(wpack);
@@ -859,15 +957,15 @@ extern "C" int ag_surrogate_llk(int32_t n, int32_t k, const float* coeff, const 
                                 void* stream) {
     AG_REQUIRE(n > 0 && k > 0 && coeff && scale && gram && h && llk, "invalid arguments");
     AG_REQUIRE(k <= kSurMaxK, "at most %d surrogate coefficients are supported (got %d)", kSurMaxK, k);
-    const size_t smem = (size_t)(k * k + kSurWarps * k) * sizeof(float);
-    int dev = 0, sms = 0;
-    int rc = cuda_status(cudaGetDevice(&dev), "cudaGetDevice");
-    if (rc) return rc;
-    rc = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "multiProcessorCount");
-    if (rc) return rc;
-    const int grid = min(nblk(n, kSurWarps), 4 * sms);
-    surrogate_llk_kernel<<<grid, kSurWarps * 32, smem, as_stream(stream)>>>(n, k, coeff, scale, gram, h, q0,
-                                                                           norm, llk);
+    const size_t smem = sur_smem(k);
+    if (smem > 48 * 1024) {
+        int rc = cuda_status(cudaFuncSetAttribute(surrogate_llk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)smem),
+                             "cudaFuncSetAttribute(surrogate_llk_kernel)");
+        if (rc) return rc;
+    }
+    surrogate_llk_kernel<<<nblk(n, kSurChains), kSurChains / 8 * sur_groups(k), smem, as_stream(stream)>>>(
+        n, k, coeff, scale, gram, h, q0, norm, llk);
     return launch_status("surrogate_llk_kernel");
 }
 
