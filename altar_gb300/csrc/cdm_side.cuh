@@ -944,29 +944,6 @@ struct PackedNode {
     float4 dw;    // d, d, w, w
 };
 
-typedef unsigned long long f32x2;
-AG_DEVICE_INLINE f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-AG_DEVICE_INLINE void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-AG_DEVICE_INLINE f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-AG_DEVICE_INLINE f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-AG_DEVICE_INLINE f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 template <int N>
 AG_DEVICE_INLINE void rect_quad_packed(const RectQ& Q, const PackedNode* node, int nn, SV<N> Xr, SV<N> Yr, SV<N>& ue,
                                        SV<N>& un, SV<N>& uv) {

@@ -138,6 +138,46 @@ AG_DEVICE_INLINE void ff_add_wsq(ff& acc, float r, float w) {
 
 AG_DEVICE_INLINE double ff_to_double(const ff& a) { return (double)a.hi + (double)a.lo; }
 
+// ---------------------------------------------------------------------------
+// packed FP32 pairs: one issue slot, each element rounded as by the scalar instruction (subnormals
+// flushed, as in the translation units compiled with -ftz=true that use them)
+typedef unsigned long long f32x2;
+AG_DEVICE_INLINE f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+AG_DEVICE_INLINE void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+AG_DEVICE_INLINE f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+AG_DEVICE_INLINE f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+AG_DEVICE_INLINE f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+AG_DEVICE_INLINE f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pack2(-1.0f, -1.0f), a); }
+
+// (hi, lo) += w r² for two sums at once, as ff_add_wsq without the final renormalisation: hi takes
+// the rounded sums, lo everything they leave (|lo| stays a few units of hi's last place per term)
+AG_DEVICE_INLINE void ff2_add_wsq(f32x2& hi, f32x2& lo, f32x2 r, f32x2 w, f32x2 nw) {
+    const f32x2 np = mul2(r, mul2(r, pack2(-1.0f, -1.0f)));      // -r²
+    const f32x2 pe = fma2(r, r, np);
+    const f32x2 q = mul2(np, nw), nq = mul2(np, w);
+    const f32x2 qe = fma2(pe, w, fma2(np, nw, nq));
+    const f32x2 s = add2(hi, q), bb = sub2(s, hi);
+    const f32x2 e = add2(sub2(hi, sub2(s, bb)), sub2(q, bb));
+    lo = add2(lo, add2(e, qe));
+    hi = s;
+}
+
 // warp sum of doubles (fixed butterfly order: deterministic)
 AG_DEVICE_INLINE double warp_sum(double v) {
 #pragma unroll

@@ -621,14 +621,50 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
 }
 
 // ---------------------------------------------------------------------------
-// Mogi: one thread per station, CH chains per CTA held in shared memory
-struct __align__(16) MogiSrc {
-    float4 pos;    // x0_hi, x0_lo, y0_hi, y0_lo
-    float4 prm;    // depth, C = (nu - 1) ΔV / π, 0, 0
+// Mogi: one thread per station, CH chains per CTA held in shared memory, two chains per packed
+// FP32 instruction (every element rounded as by the scalar one).  The FMA pipe bounds it: per pair
+// 15 operations per source, 16 for the residual and the float-float sum w r², and one reciprocal
+// square root.  Beside the scalar instructions' issue slots, FP64 took a sixth of the former
+// kernel: 128 conversions and additions per warp at 64 cycles each to add the lanes' sums, which
+// are now added in float-float (48 bits, as the sums themselves) with each step halving the
+// chains a lane holds.  16,384 chains x 10,007 stations with offsets 326 -> 197 µs (217 with two
+// CTAs per SM instead of four), 1,024 x 1,024 20.5 -> 8.3 µs; two sources with residual rows, 16,384 x
+// 4,950, 264 -> 145 µs.
+struct __align__(16) MogiPair {       // a source of two chains
+    float4 x;      // x0 hi, hi, lo, lo
+    float4 y;
+    float4 d;      // depth²,  depth², -depth, -depth
+    float2 c;      // C = (nu - 1) ΔV / π
+    float2 pad;
 };
 
+// sum over the warp of each of N (a power of two <= 32) float-float values per lane; on return v[0] of
+// lane l holds value l / (32 / N)
+template <int N>
+__device__ __forceinline__ void warp_sum_ff(ff (&v)[N], int lane) {
+    int held = N;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+        if (held > 1) {
+            held >>= 1;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i) {
+                if (i >= held) break;
+                const ff keep = up ? v[i + held] : v[i], send = up ? v[i] : v[i + held];
+                const float h = __shfl_xor_sync(0xffffffffu, send.hi, o), l = __shfl_xor_sync(0xffffffffu, send.lo, o);
+                v[i] = keep;
+                ff_add(v[i], h, l);
+            }
+        } else {
+            const float h = __shfl_xor_sync(0xffffffffu, v[0].hi, o), l = __shfl_xor_sync(0xffffffffu, v[0].lo, o);
+            ff_add(v[0], h, l);
+        }
+    }
+}
+
 template <int CH, int NSRC>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, CH <= 16 ? 4 : 2)
 mogi_llk_kernel(ag_layout L, const double* __restrict__ theta, int n,
                 const uint32_t* __restrict__ mask_in, const float4* __restrict__ xy,
                 const float4* __restrict__ losd, const float* __restrict__ wt,
@@ -636,84 +672,106 @@ mogi_llk_kernel(ag_layout L, const double* __restrict__ theta, int n,
                 int m_padded, double norm, double* __restrict__ llk, float* __restrict__ resid,
                 const int32_t* __restrict__ index, const int32_t* __restrict__ count) {
     if (index && (int)(blockIdx.x * CH) >= *count) return;
-    __shared__ MogiSrc s_src[CH][NSRC];
+    constexpr int CP = CH / 2;
+    __shared__ MogiPair s_src[CP][NSRC];
     __shared__ int s_chain[CH];
-    __shared__ float s_off[CH][kMaxOffsets];
+    __shared__ float2 s_off[CP][kMaxOffsets];
     __shared__ int s_act[CH];
-    __shared__ double s_part[CH][8];
+    __shared__ float2 s_part[CH][8];
     const int c0 = blockIdx.x * CH;
     const double PI = 3.14159265358979323846;
     const int nslots = index ? min(n, *count) : n;
     for (int c = threadIdx.x; c < CH; c += blockDim.x) {
         const int slot = c0 + c;
-        s_chain[c] = (slot < nslots) ? (index ? index[slot] : slot) : n;
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < CH * NSRC; k += blockDim.x) {
-        const int c = k / NSRC, src = k % NSRC, i = s_chain[c];
-        MogiSrc S{};
-        if (i < n) {
-            const double* th = theta + (size_t)i * L.nparams + src * L.source_stride;
-            split_hilo(th[L.x_idx], S.pos.x, S.pos.y);
-            split_hilo(th[L.x_idx + 1], S.pos.z, S.pos.w);
-            const double dv = L.log_strength ? pow(10.0, th[L.strength_idx]) : th[L.strength_idx];
-            S.prm = make_float4((float)th[L.depth_idx], (float)((L.nu - 1.0) * dv / PI), 0.f, 0.f);
-        }
-        s_src[c][src] = S;
-    }
-    for (int k = threadIdx.x; k < CH * kMaxOffsets; k += blockDim.x) {
-        const int c = k / kMaxOffsets, o = k % kMaxOffsets, i = s_chain[c];
-        s_off[c][o] = (i < n && o < noffsets)
-                          ? (float)theta[(size_t)i * L.nparams + L.offset_idx + o] : 0.f;
-    }
-    for (int c = threadIdx.x; c < CH; c += blockDim.x) {
-        const int i = s_chain[c];
+        const int i = (slot < nslots) ? (index ? index[slot] : slot) : n;
+        s_chain[c] = i;
         s_act[c] = (i < n) && !(mask_in && mask_in[i]);
     }
     __syncthreads();
-    ff acc[CH];
+    for (int k = threadIdx.x; k < CH * NSRC; k += blockDim.x) {
+        const int c = k / NSRC, src = k % NSRC, i = s_chain[c], h = c & 1;
+        float xh = 0.f, xl = 0.f, yh = 0.f, yl = 0.f, d = 0.f, C = 0.f;
+        if (i < n) {
+            const double* th = theta + (size_t)i * L.nparams + src * L.source_stride;
+            split_hilo(th[L.x_idx], xh, xl);
+            split_hilo(th[L.x_idx + 1], yh, yl);
+            const double dv = L.log_strength ? pow(10.0, th[L.strength_idx]) : th[L.strength_idx];
+            d = (float)th[L.depth_idx];
+            C = (float)((L.nu - 1.0) * dv / PI);
+        }
+        float* S = reinterpret_cast<float*>(&s_src[c >> 1][src]);
+        S[h] = xh; S[2 + h] = xl;
+        S[4 + h] = yh; S[6 + h] = yl;
+        S[8 + h] = __fmul_rn(d, d); S[10 + h] = -d;
+        S[12 + h] = C;
+    }
+    if (oid) {
+        for (int k = threadIdx.x; k < CH * kMaxOffsets; k += blockDim.x) {
+            const int c = k / kMaxOffsets, o = k % kMaxOffsets, i = s_chain[c];
+            reinterpret_cast<float*>(&s_off[c >> 1][o])[c & 1] =
+                (i < n && o < noffsets) ? (float)theta[(size_t)i * L.nparams + L.offset_idx + o] : 0.f;
+        }
+    }
+    __syncthreads();
+    f32x2 hi[CP], lo[CP];
 #pragma unroll
-    for (int c = 0; c < CH; ++c) acc[c] = ff{0.f, 0.f};
+    for (int c = 0; c < CP; ++c) hi[c] = lo[c] = 0ull;
     for (int j = threadIdx.x; j < m_padded; j += blockDim.x) {
         const float4 A = __ldg(xy + j);
         const float4 B = __ldg(losd + j);
         const float w = __ldg(wt + j);
         const int o = oid ? (__ldg(oid + j) & (kMaxOffsets - 1)) : 0;
+        const int col = order ? __ldg(order + j) : j;
+        const f32x2 nax = pack2(-A.x, -A.x), nay = pack2(-A.y, -A.y), naz = pack2(-A.z, -A.z), naw = pack2(-A.w, -A.w);
+        const f32x2 bx = pack2(B.x, B.x), by = pack2(B.y, B.y), bz = pack2(B.z, B.z), nd = pack2(-B.w, -B.w);
+        const f32x2 w2 = pack2(w, w), nw2 = pack2(-w, -w);
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
-            float u = 0.f;
+        for (int c = 0; c < CP; ++c) {
+            f32x2 u = 0ull;
 #pragma unroll
-            for (int sidx = 0; sidx < NSRC; ++sidx) {
-                const MogiSrc S = s_src[c][sidx];
+            for (int src = 0; src < NSRC; ++src) {
+                const MogiPair& S = s_src[c][src];
+                const ulonglong2 sx = *reinterpret_cast<const ulonglong2*>(&S.x);
+                const ulonglong2 sy = *reinterpret_cast<const ulonglong2*>(&S.y);
+                const ulonglong2 sd = *reinterpret_cast<const ulonglong2*>(&S.d);
+                const f32x2 sc = *reinterpret_cast<const f32x2*>(&S.c);
                 // source minus observation point (libmogi/Source.cc:86-88)
-                const float dx = (S.pos.x - A.x) + (S.pos.y - A.y);
-                const float dy = (S.pos.z - A.z) + (S.pos.w - A.w);
-                const float d = S.prm.x;
-                const float R2 = fmaf(dx, dx, fmaf(dy, dy, d * d));
-                const float iR = rsqrtf(R2);
-                const float iR3 = iR * iR * iR;
-                const float proj = fmaf(dx, B.x, fmaf(dy, B.y, -d * B.z));
-                u = fmaf(S.prm.y * proj, iR3, u);
+                const f32x2 dx = add2(add2(sx.x, nax), add2(sx.y, nay));
+                const f32x2 dy = add2(add2(sy.x, naz), add2(sy.y, naw));
+                const f32x2 R2 = fma2(dx, dx, fma2(dy, dy, sd.x));
+                float r0, r1;
+                unpack2(R2, r0, r1);
+                const f32x2 iR = pack2(rsqrtf(r0), rsqrtf(r1));
+                const f32x2 iR3 = mul2(mul2(iR, iR), iR);
+                const f32x2 proj = fma2(dx, bx, fma2(dy, by, mul2(sd.y, bz)));
+                u = fma2(mul2(sc, proj), iR3, u);
             }
-            float r = u - B.w;
-            if (oid) r -= s_off[c][o];
-            if (w != 0.f) ff_add_wsq(acc[c], r, w);
-            if (resid && s_chain[c] < n)
-                resid[(size_t)s_chain[c] * m_padded + (order ? __ldg(order + j) : j)] = (j < m) ? r : 0.f;
+            f32x2 r = add2(u, nd);
+            if (oid) r = sub2(r, *reinterpret_cast<const f32x2*>(&s_off[c][o]));
+            if (w != 0.f) ff2_add_wsq(hi[c], lo[c], r, w2, nw2);
+            if (resid) {
+                float r0, r1;
+                unpack2(r, r0, r1);
+                if (s_chain[2 * c] < n) resid[(size_t)s_chain[2 * c] * m_padded + col] = (j < m) ? r0 : 0.f;
+                if (s_chain[2 * c + 1] < n) resid[(size_t)s_chain[2 * c + 1] * m_padded + col] = (j < m) ? r1 : 0.f;
+            }
         }
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    ff v[CH];
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
-        const double v = warp_sum(ff_to_double(acc[c]));
-        if (lane == 0) s_part[c][warp] = v;
+    for (int c = 0; c < CP; ++c) {
+        unpack2(hi[c], v[2 * c].hi, v[2 * c + 1].hi);
+        unpack2(lo[c], v[2 * c].lo, v[2 * c + 1].lo);
     }
+    warp_sum_ff(v, lane);
+    if (lane % (32 / CH) == 0) s_part[lane / (32 / CH)][warp] = make_float2(v[0].hi, v[0].lo);
     __syncthreads();
     for (int c = threadIdx.x; c < CH; c += blockDim.x) {
         if (!s_act[c]) continue;
-        double s = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += s_part[c][k];
-        llk[s_chain[c]] = norm - 0.5 * s;
+        ff t{0.f, 0.f};
+        for (int k = 0; k < 8; ++k) ff_add(t, s_part[c][k].x, s_part[c][k].y);
+        llk[s_chain[c]] = norm - 0.5 * ff_to_double(t);
     }
 }
 
@@ -895,17 +953,22 @@ static int forward_llk(int model, const ag_layout* layout, const double* theta, 
         AG_REQUIRE(L.nsources == 1 || L.nsources == 2, "1 or 2 Mogi sources are supported");
         AG_REQUIRE(L.variant >= 0 && L.variant < kMogiVariantCount, "Mogi variant %d out of range [0, %d)",
                    L.variant, kMogiVariantCount);
-        const int ch = kMogiChainsOf[L.variant];
+        // the default takes fewer chains per CTA where sixteen would leave SMs
+        // with fewer than two: 4,096 x 3,000 27.0 µs with 8 and 32.9 with 32, 1,024 x 1,024 10.6 with 4
+        // and 16.6 with 32
+        const int ch = L.variant != 0 ? kMogiChainsOf[L.variant] : n >= 16 * 304 ? 16 : n >= 8 * 304 ? 8 : 4;
         const int grid = (n + ch - 1) / ch;
 #define AG_MOGI_LAUNCH(CH, NS)                                                                               \
     mogi_llk_kernel<CH, NS><<<grid, 256, 0, s>>>(L, theta, n, mask_in, xy, ld, st->weight, st->oid, st->order, \
                                                  noffsets, st->m, st->m_padded, norm, llk, residuals, index, count)
         if (L.nsources == 1) {
-            if (ch == 8) AG_MOGI_LAUNCH(8, 1);
+            if (ch == 4) AG_MOGI_LAUNCH(4, 1);
+            else if (ch == 8) AG_MOGI_LAUNCH(8, 1);
             else if (ch == 32) AG_MOGI_LAUNCH(32, 1);
             else AG_MOGI_LAUNCH(16, 1);
         } else {
-            if (ch == 8) AG_MOGI_LAUNCH(8, 2);
+            if (ch == 4) AG_MOGI_LAUNCH(4, 2);
+            else if (ch == 8) AG_MOGI_LAUNCH(8, 2);
             else if (ch == 32) AG_MOGI_LAUNCH(32, 2);
             else AG_MOGI_LAUNCH(16, 2);
         }
