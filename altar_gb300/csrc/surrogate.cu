@@ -56,6 +56,18 @@ AG_DEVICE_INLINE float load_b(const void* Bv, long idx) {
                   : reinterpret_cast<const float*>(Bv)[idx];
 }
 
+// shares of K of an M x N product and their length: K is split when the output tiles alone would leave
+// most of the GPU idle (the weight gradients: a few tiles, K = batch rows)
+__host__ __device__ __forceinline__ int product_split(int M, int N, int K) {
+    const int tiles = (N + BN - 1) / BN * ((M + BM - 1) / BM);
+    int split = 1;
+    while (split < 8 && tiles * split < 128 && K >= 2 * BK * (split * 2)) split *= 2;
+    return split;
+}
+__host__ __device__ __forceinline__ int product_share(int K, int split) {
+    return ((K + split - 1) / split + BK - 1) / BK * BK;
+}
+
 template <bool B_BF16>
 __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const float* __restrict__ A,
                                                    long sam, long sak, const void* __restrict__ Bv,
@@ -68,7 +80,7 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const fl
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int split = gridDim.z, part = blockIdx.z;
-    const int kchunk = ((K + split - 1) / split + BK - 1) / BK * BK;
+    const int kchunk = product_share(K, split);
     const int kb = min(K, part * kchunk), ke = min(K, kb + kchunk);
     // element e of a 16 x 64 operand tile: (k, m) with k fastest when that stride is 1
     const bool a_k1 = (sak == 1), b_k1 = (sbk == 1);
@@ -144,6 +156,448 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const fl
     cluster.sync();                                     // partial tiles stay alive until all have read them
 }
 
+
+// ---------------------------------------------------------------------------
+// Networks of widths up to kRowWidth (multiples of 8 behind the input): forward in one launch,
+// backward in one launch per layer.  A training batch of 1,024 rows is ~0.13 GFLOP per layer
+// product, a few microseconds of FP32 work that the tiled products spread over 15 µs of launch,
+// load latency and reduction, 33 launches per batch.  Every sum is taken in the tiled products'
+// order (shares of K by product_split, each one chain, the shares in order), so the results are
+// theirs bit for bit; packed FMAs take two rows or columns, never two terms of a sum.
+//
+// Forward: a CTA takes kNetRows rows through all layers; the activations stay in shared memory as
+// columns of eight rows, and the weights stream through a ring of chunks whose loads run ahead
+// across the layers.  A chunk holds 64 columns of a layer's weights, 64 / split of each share, so
+// that all shares advance together.  A thread owns four outputs of 2, 4 or 8 rows in one share: a
+// shared-memory load of 16 bytes per lane costs four cycles also where all lanes read one address,
+// so that one output per thread (8 cycles of loads per 4 packed FMAs) was bound by them.
+// Bound by issue at two warps per scheduler and the barrier of each chunk.  10-256-256-256-256-64,
+// 1,024 rows: 63.8 -> 35.1 µs.
+constexpr int kRowWidth = 256;
+constexpr int kNetRows = 8;
+// rows that go forward here: 2,048 rows take 74 µs against 91 of the tiled products (256 wide), 21 against
+// 27 (128), 15 against 25 (64); 4,096 rows 146 against 125, 38 against 33, 27 against 25, since every
+// CTA streams all the weights
+constexpr int kNetMost = 2048;
+constexpr int kNetThreads = 256;
+constexpr int kNetChunk = 64;                           // inputs per chunk of weights
+constexpr int kNetStride = kNetChunk + 8;               // BF16 row in shared memory: no bank conflicts
+constexpr int kNetStages = 4;
+constexpr size_t kNetStage = (size_t)kRowWidth * kNetStride * sizeof(__nv_bfloat16);
+constexpr int kNetSums = 4 * kNetRows * kRowWidth;      // floats: [share][row][output], 4 x 256 or 8 x 128
+constexpr size_t kNetSmem = kNetStages * kNetStage + (2 * (size_t)kRowWidth * kNetRows + kNetSums) * sizeof(float);
+
+// How the threads of a CTA divide a product of `rows` x `width` outputs with K terms: four outputs a
+// thread, `slots` threads per four outputs, over the shares first and then over the rows.
+struct NetSplit {
+    int split, share, groups, row_groups;
+};
+__host__ __device__ __forceinline__ NetSplit net_split(int rows, int width, int K) {
+    NetSplit v;
+    v.split = product_split(rows, width, K);
+    v.share = product_share(K, v.split);
+    v.groups = width > kRowWidth / 2 ? kRowWidth / 4 : kRowWidth / 8;
+    const int left = kNetThreads / v.groups / v.split;  // 0: more shares than slots
+    v.row_groups = left > 4 ? 4 : left;
+    return v;
+}
+
+struct NetLayers {
+    int nlayers;
+    int sizes[kMaxLayers + 1];
+    int64_t w[kMaxLayers], b[kMaxLayers];
+};
+
+AG_DEVICE_INLINE f32x2 fma2_full(f32x2 a, f32x2 b, f32x2 c) {      // subnormals kept
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+AG_DEVICE_INLINE void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+// 16 or 4 bytes, zeros where !take (src is not read then)
+template <int B> AG_DEVICE_INLINE void cp_async_or_zero(void* dst, const void* src, bool take) {
+    const int bytes = take ? B : 0;
+    if constexpr (B == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes) : "memory");
+}
+AG_DEVICE_INLINE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> AG_DEVICE_INLINE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// the eight BF16 values of a 16-byte word as FP32
+AG_DEVICE_INLINE void bf16x8(const uint4 v, float (&f)[8]) {
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        f[2 * q] = __uint_as_float(u[q] << 16);
+        f[2 * q + 1] = __uint_as_float(u[q] & 0xFFFF0000u);
+    }
+}
+
+// one chain of a thread: four outputs x RP pairs of rows, over the eight weights of `w` and inputs `v`
+template <int RP>
+AG_DEVICE_INLINE void net_fma(f32x2 (&acc)[4][RP], const float (&w)[4], const float* v) {
+    f32x2 x2[RP];
+    if constexpr (RP == 1) {
+        x2[0] = *reinterpret_cast<const f32x2*>(v);
+    } else {
+#pragma unroll
+        for (int q = 0; q < RP; q += 2) {
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(v + 2 * q);
+            x2[q] = u.x, x2[q + 1] = u.y;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const f32x2 ww = pack2(w[j], w[j]);
+#pragma unroll
+        for (int q = 0; q < RP; ++q) acc[j][q] = fma2_full(x2[q], ww, acc[j][q]);
+    }
+}
+
+// the chains of one layer, to s_red[share][row][output]; `next` waits for a chunk and returns its stage
+template <int RP, class Next>
+AG_DEVICE_INLINE void net_layer(const NetSplit d, int fi, int fo, const float* in, float* s_red, int stride, Next next) {
+    const int slot = threadIdx.x / d.groups, first = threadIdx.x % d.groups;
+    const int part = slot / d.row_groups, row = slot % d.row_groups * 2 * RP;
+    const int len = kNetChunk / d.split;
+    f32x2 acc[4][RP] = {};
+    for (int s = 0; s < d.share; s += len) {
+        const __nv_bfloat16* W = next() + part * len;
+        if (part >= d.split) continue;
+        const int k0 = part * d.share + s;
+#pragma unroll 1
+        for (int g = 0; g < len; g += 8) {
+            if (s + g >= d.share || k0 + g >= fi) break;
+            float w[4][8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int o = first + j * d.groups;     // rows past the last output: any values
+                bf16x8(*reinterpret_cast<const uint4*>(W + (o < fo ? o : 0) * kNetStride + g), w[j]);
+            }
+            const float* v = in + (k0 + g) * kNetRows + row;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float wq[4] = {w[0][q], w[1][q], w[2][q], w[3][q]};
+                net_fma<RP>(acc, wq, v + q * kNetRows);
+            }
+        }
+    }
+    if (part >= d.split) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int o = first + j * d.groups;
+        if (o >= fo) break;
+#pragma unroll
+        for (int q = 0; q < RP; ++q) {
+            float a, b;
+            unpack2(acc[j][q], a, b);
+            s_red[(part * kNetRows + row + 2 * q) * stride + o] = a;
+            s_red[(part * kNetRows + row + 2 * q + 1) * stride + o] = b;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kNetThreads, 1)
+net_forward_kernel(NetLayers net, const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf,
+                   const float* __restrict__ x, int n, float* __restrict__ out, float* __restrict__ acts) {
+    extern __shared__ __align__(16) uint8_t s_net[];
+    constexpr int kCols = kRowWidth * kNetRows;
+    float* xT = reinterpret_cast<float*>(s_net + kNetStages * kNetStage);   // [2][kRowWidth][kNetRows]
+    float* s_red = xT + 2 * kCols;
+    const int tid = threadIdx.x;
+    const long r0 = (long)blockIdx.x * kNetRows;
+    const int rows = n - r0 < kNetRows ? (int)(n - r0) : kNetRows;
+    int ql = 0, qs = 0, loaded = 0, used = 0;           // next chunk to load: layer, offset in the shares
+    auto load = [&]() {
+        if (ql < net.nlayers) {
+            const int fi = net.sizes[ql], fo = net.sizes[ql + 1];
+            const NetSplit d = net_split(n, fo, fi);
+            const int len = kNetChunk / d.split;
+            const __nv_bfloat16* W = wbf + net.w[ql];
+            __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(s_net + (loaded % kNetStages) * kNetStage);
+            constexpr int step = kNetThreads / (kNetChunk / 8);
+            const int o = tid / (kNetChunk / 8), i = tid % (kNetChunk / 8) * 8;
+            const int at = qs + i % len, k = i / len * d.share + at;       // eight inputs of one share
+            if (at < d.share && k < fi) {
+                if (fi % 8 == 0) {
+                    const __nv_bfloat16* from = W + (size_t)o * fi + k;
+#pragma unroll
+                    for (int q = 0; q < kRowWidth / step; ++q, from += (size_t)step * fi)
+                        if (o + q * step < fo) cp_async16(to + (o + q * step) * kNetStride + i, from);
+                } else {                                // zeros past the last input
+                    const unsigned short* w16 = reinterpret_cast<const unsigned short*>(W);
+                    unsigned short* to16 = reinterpret_cast<unsigned short*>(to);
+                    for (int q = o; q < fo; q += step)
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            to16[q * kNetStride + i + e] = k + e < fi ? __ldg(w16 + (size_t)q * fi + k + e) : 0;
+                }
+            }
+            qs += len;
+            if (qs >= d.share) {
+                qs = 0;
+                ++ql;
+            }
+        }
+        cp_async_commit();
+        ++loaded;
+    };
+    auto next = [&]() {
+        cp_async_wait<kNetStages - 2>();
+        __syncthreads();                                // the chunk and the layer's inputs are there
+        load();                                         // into the stage that the previous chunk left
+        return reinterpret_cast<const __nv_bfloat16*>(s_net + (used++ % kNetStages) * kNetStage);
+    };
+    for (int q = 0; q < kNetStages - 1; ++q) load();
+    const int fi0 = net.sizes[0], pad0 = (fi0 + 7) / 8 * 8;
+    for (int e = tid; e < pad0 * kNetRows; e += kNetThreads) {
+        const int r = e / pad0, i = e - r * pad0;
+        xT[i * kNetRows + r] = (r < rows && i < fi0) ? x[(r0 + r) * fi0 + i] : 0.f;
+    }
+    float* a = acts;
+    for (int l = 0; l < net.nlayers; ++l) {
+        const int fi = net.sizes[l], fo = net.sizes[l + 1];
+        const bool last = l == net.nlayers - 1;
+        const float* in = xT + (l & 1) * kCols;
+        float* to = xT + ((l + 1) & 1) * kCols;
+        const int stride = fo > kRowWidth / 2 ? kRowWidth : kRowWidth / 2;
+        const int o = tid % stride, step = kNetThreads / stride;       // an output's eight rows, or four
+        const float bias = o < fo ? params[net.b[l] + o] : 0.f;
+        const NetSplit d = net_split(n, fo, fi);
+        if (d.row_groups == 4)
+            net_layer<1>(d, fi, fo, in, s_red, stride, next);
+        else if (d.row_groups == 2)
+            net_layer<2>(d, fi, fo, in, s_red, stride, next);
+        else
+            net_layer<4>(d, fi, fo, in, s_red, stride, next);
+        __syncthreads();
+        if (o < fo) {
+            constexpr int R = kNetRows / 2;
+            for (int h = tid / stride; h < 2; h += step) {
+                float z[R] = {};
+#pragma unroll 4
+                for (int q = 0; q < d.split; ++q)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) z[r] += s_red[(q * kNetRows + h * R + r) * stride + o];
+                float y[R];
+                const long at = (r0 + h * R) * fo + o;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    z[r] += bias;
+                    y[r] = last ? z[r] : gelu(z[r]);
+                    if (h * R + r >= rows) continue;
+                    if (last) {
+                        out[at + r * fo] = y[r];
+                    } else {
+                        a[at + r * fo] = z[r];
+                        a[(long)n * fo + at + r * fo] = y[r];
+                    }
+                }
+                *reinterpret_cast<float4*>(to + o * kNetRows + h * R) = make_float4(y[0], y[1], y[2], y[3]);
+            }
+        }
+        a += 2 * (long)n * fo;
+    }
+    cp_async_wait<0>();
+}
+
+// the chains of one row block's dX = dZ W, to s_red[share][row][column]
+template <int RP>
+AG_DEVICE_INLINE void net_back_rows(const NetSplit d, int fi, int fo, const __nv_bfloat16* __restrict__ W,
+                                    const float* zT, float* s_red, int stride) {
+    const int slot = threadIdx.x / d.groups, i = threadIdx.x % d.groups * 4;
+    const int part = slot / d.row_groups, row = slot % d.row_groups * 2 * RP;
+    if (part >= d.split || i >= fi) return;
+    const uint2* w = reinterpret_cast<const uint2*>(W + i);
+    const int end = min(fo, (part + 1) * d.share);
+    f32x2 acc[4][RP] = {};
+#pragma unroll 16
+    for (int o = part * d.share; o < end; ++o) {
+        const uint2 u = __ldg(w + (size_t)o * (fi / 4));
+        const float f[4] = {__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xFFFF0000u),
+                            __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xFFFF0000u)};
+        net_fma<RP>(acc, f, zT + o * kNetRows + row);
+    }
+#pragma unroll
+    for (int q = 0; q < RP; ++q) {
+        float a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) unpack2(acc[j][q], a[j], b[j]);
+        float* to = s_red + (part * kNetRows + row + 2 * q) * stride + i;
+        *reinterpret_cast<float4*>(to) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4*>(to + stride) = make_float4(b[0], b[1], b[2], b[3]);
+    }
+}
+
+// Backward through one layer: CTAs of three kinds in clusters of kBackSplit.  The first `row_ctas` take
+// kNetRows rows each: dX = dZ W and, behind it, the previous layer's dZ = dX ⊙ GELU'(Z) (a thread per
+// four columns and 2, 4 or 8 rows of a share; W's rows stream from L2).  The next `sum_ctas` take eight
+// columns each for the bias's gradient, as colsum_kernel sums them.  Then a cluster per 64 x 64 tile
+// of dW = dZᵀ h: its CTAs take a share of the rows each, through double-buffered slabs of 64, with
+// 8 x 4 outputs in each of 128 threads (12 cycles of shared-memory loads per 16 packed FMAs; 4 x 4 in
+// 256 take 8 per 8), and add their tiles through distributed shared memory in rank order.
+// 10-256-256-256-256-64: 173 -> 65 µs at 1,024 rows, 2,472 -> 1,701 µs at 32,768.  At 1,024 rows a
+// layer's 15 µs are launch, load latency, ~4 µs of sums and the two cluster barriers in sequence.
+constexpr int kBackSplit = 8;
+constexpr int kBackSlab = 64;
+constexpr int kBackTile = 64;
+constexpr size_t kBackSmem = 4 * (size_t)kBackSlab * kBackTile * sizeof(float);
+static_assert(kBackSlab == kBackTile, "the tile's sums take a slab's place");
+static_assert((kRowWidth * kNetRows + kNetSums) * sizeof(float) <= kBackSmem, "row CTAs");
+
+__global__ void __launch_bounds__(kNetThreads, 2)
+net_backward_kernel(int n, int fi, int fo, const float* __restrict__ dZ, const __nv_bfloat16* __restrict__ W,
+                    const float* __restrict__ Zprev, float* __restrict__ dprev, int row_ctas, int sum_ctas,
+                    const float* __restrict__ h, int htiles, float* __restrict__ dW, float* __restrict__ db) {
+    extern __shared__ __align__(16) float s_back[];
+    const int tid = threadIdx.x;
+    int block = blockIdx.x;
+    if (block < row_ctas) {
+        const long r0 = (long)block * kNetRows;
+        if (r0 >= n) return;
+        const int rows = n - r0 < kNetRows ? (int)(n - r0) : kNetRows;
+        float* zT = s_back;                             // [fo][kNetRows]
+        float* s_red = zT + kRowWidth * kNetRows;
+        float z[kNetRows];
+        if (tid < fo) {
+#pragma unroll
+            for (int r = 0; r < kNetRows; ++r) z[r] = r < rows ? __ldg(dZ + (r0 + r) * fo + tid) : 0.f;
+            *reinterpret_cast<float4*>(zT + tid * kNetRows) = make_float4(z[0], z[1], z[2], z[3]);
+            *reinterpret_cast<float4*>(zT + tid * kNetRows + 4) = make_float4(z[4], z[5], z[6], z[7]);
+        }
+        if (tid < fi) {                                 // for the end; the loads run behind the sums
+#pragma unroll
+            for (int r = 0; r < kNetRows; ++r) z[r] = r < rows ? __ldg(Zprev + (r0 + r) * fi + tid) : 0.f;
+        }
+        __syncthreads();
+        const NetSplit d = net_split(n, fi, fo);
+        const int stride = fi > kRowWidth / 2 ? kRowWidth : kRowWidth / 2;
+        if (d.row_groups == 4)
+            net_back_rows<1>(d, fi, fo, W, zT, s_red, stride);
+        else if (d.row_groups == 2)
+            net_back_rows<2>(d, fi, fo, W, zT, s_red, stride);
+        else
+            net_back_rows<4>(d, fi, fo, W, zT, s_red, stride);
+        __syncthreads();
+        if (tid < fi) {
+            float v[kNetRows] = {};
+#pragma unroll 2
+            for (int q = 0; q < d.split; ++q)
+#pragma unroll
+                for (int r = 0; r < kNetRows; ++r) v[r] += s_red[(q * kNetRows + r) * stride + tid];
+#pragma unroll
+            for (int r = 0; r < kNetRows; ++r)
+                if (r < rows) dprev[(r0 + r) * fi + tid] = v[r] * gelu_grad(z[r]);
+        }
+        return;
+    }
+    block -= row_ctas;
+    if (block < sum_ctas) {
+        // thread t: rows t, t + 256, ... of eight columns; then the tree over t, a warp per column
+        const int c0 = block * 8;
+        if (c0 >= fo) return;
+        float v[8] = {};
+        for (int i = tid; i < n; i += kNetThreads) {
+            const float* z = dZ + (size_t)i * fo + c0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] += __ldg(z + c);
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) s_back[c * kNetThreads + tid] = v[c];
+        __syncthreads();
+        const int lane = tid & 31, c = tid >> 5;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = s_back[c * kNetThreads + 32 * q + lane];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < o; ++q) v[q] += v[q + o];
+        for (int o = 16; o > 0; o >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], o);
+        if (lane == 0) db[c0 + c] = v[0];
+        return;
+    }
+    block -= sum_ctas;
+    const int tile = block / kBackSplit, rank = block % kBackSplit;
+    const int m0 = tile / htiles * kBackTile, n0 = tile % htiles * kBackTile;
+    float* As = s_back;                                 // [2][kBackSlab][kBackTile] dZ
+    float* Bs = As + 2 * kBackSlab * kBackTile;         // [2][kBackSlab][kBackTile] h
+    float* Ps = s_back;                                 // afterwards: [kBackTile][kBackTile] sums of the share
+    const int share = product_share(n, product_split(fo, fi, n));
+    const int kb = min(n, rank * share), ke = min(n, kb + share);
+    auto slab = [&](const float* src, int ld, int c0, int k0, float* to) {
+        if (c0 + kBackTile <= ld && ld % 4 == 0 && (size_t)src % 16 == 0) {
+#pragma unroll
+            for (int q = 0; q < kBackSlab * kBackTile / 4 / kNetThreads; ++q) {
+                const int e = q * kNetThreads + tid, k = e / (kBackTile / 4), c = e % (kBackTile / 4) * 4;
+                const bool take = k0 + k < ke;
+                cp_async_or_zero<16>(to + k * kBackTile + c, take ? src + (size_t)(k0 + k) * ld + c0 + c : src, take);
+            }
+        } else {
+#pragma unroll 4
+            for (int q = 0; q < kBackSlab * kBackTile / kNetThreads; ++q) {
+                const int e = q * kNetThreads + tid, k = e / kBackTile, c = e % kBackTile;
+                const bool take = k0 + k < ke && c0 + c < ld;
+                cp_async_or_zero<4>(to + e, take ? src + (size_t)(k0 + k) * ld + c0 + c : src, take);
+            }
+        }
+    };
+    auto load = [&](int k0, int buf) {
+        if (k0 < ke) {
+            slab(dZ, fo, m0, k0, As + buf * kBackSlab * kBackTile);
+            slab(h, fi, n0, k0, Bs + buf * kBackSlab * kBackTile);
+        }
+        cp_async_commit();
+    };
+    const int tx = tid % 16, ty = tid / 16 % 8;
+    const bool sums = tid < kNetThreads / 2;
+    f32x2 acc[8][2] = {};                               // rows ty * 4 + {0-3, 32-35}, columns tx * 4 + {0-3}
+    load(kb, 0);
+    int buf = 0;
+    for (int k0 = kb; k0 < ke; k0 += kBackSlab, buf ^= 1) {
+        load(k0 + kBackSlab, buf ^ 1);
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* A = As + buf * kBackSlab * kBackTile + ty * 4;
+        const float* B = Bs + buf * kBackSlab * kBackTile + tx * 4;
+        if (sums) {
+#pragma unroll 8
+            for (int k = 0; k < kBackSlab; ++k) {
+                const float4 a0 = *reinterpret_cast<const float4*>(A + k * kBackTile);
+                const float4 a1 = *reinterpret_cast<const float4*>(A + k * kBackTile + 32);
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(B + k * kBackTile);
+                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const f32x2 aa = pack2(av[i], av[i]);
+                    acc[i][0] = fma2_full(b.x, aa, acc[i][0]);
+                    acc[i][1] = fma2_full(b.y, aa, acc[i][1]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    cp_async_wait<0>();
+    if (sums) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<ulonglong2*>(Ps + (i / 4 * 32 + ty * 4 + i % 4) * kBackTile + tx * 4) =
+                make_ulonglong2(acc[i][0], acc[i][1]);
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    constexpr int band = kBackTile / kBackSplit;
+    for (int e = tid; e < band * kBackTile; e += kNetThreads) {
+        const int i = rank * band + e / kBackTile, j = e % kBackTile;
+        float v = 0.f;
+#pragma unroll
+        for (int r = 0; r < kBackSplit; ++r) v += cluster.map_shared_rank(Ps, r)[i * kBackTile + j];
+        if (m0 + i < fo && n0 + j < fi) dW[(size_t)(m0 + i) * fi + n0 + j] = v;
+    }
+    cluster.sync();                                     // the tiles stay until all have read them
+}
 
 // ---------------------------------------------------------------------------
 // Network layers on the tcgen05 tensor cores (inference).  A layer is
@@ -426,18 +880,35 @@ __global__ void colsum_kernel(int rows, int cols, const float* __restrict__ dZ, 
     if (threadIdx.x == 0) db[j] = part[0];
 }
 
-// mean-squared error: dY = (out - y)/n, per-row squared error for the loss
-__global__ void mse_kernel(int n, int k, const float* __restrict__ out, const float* __restrict__ y,
-                           float* __restrict__ dY, float* __restrict__ row_loss) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// mean-squared error: dY = (out - y)/n, per-row squared error for the loss.  A CTA reads its rows in
+// lines and a thread per row forms that row's sum, one chain, from shared memory: 7.8 µs for
+// 1,024 x 64, where a thread per row of global memory (no two lanes on one line) took 42
+constexpr int kMseRows = 16;
+constexpr int kMseCols = 64;
+__global__ void __launch_bounds__(128) mse_kernel(int n, int k, const float* __restrict__ out,
+                                                  const float* __restrict__ y, float* __restrict__ dY,
+                                                  float* __restrict__ row_loss) {
+    __shared__ float s_d[kMseRows][kMseCols + 1];
+    const long r0 = (long)blockIdx.x * kMseRows;
+    const int rows = n - r0 < kMseRows ? (int)(n - r0) : kMseRows, tid = threadIdx.x;
     float s = 0.f;
-    for (int j = 0; j < k; ++j) {
-        const float d = out[(long)i * k + j] - y[(long)i * k + j];
-        dY[(long)i * k + j] = d / (float)n;
-        s = fmaf(d, d, s);
+    for (int c = 0; c < k; c += kMseCols) {
+        const int cols = min(kMseCols, k - c);
+#pragma unroll
+        for (int e = tid; e < kMseRows * kMseCols; e += 128) {
+            const int r = e / kMseCols, j = e % kMseCols;
+            if (r >= rows || j >= cols) continue;
+            const long at = (r0 + r) * k + c + j;
+            const float d = out[at] - y[at];
+            dY[at] = d / (float)n;
+            s_d[r][j] = d;
+        }
+        __syncthreads();
+        if (tid < rows)
+            for (int j = 0; j < cols; ++j) s = fmaf(s_d[tid][j], s_d[tid][j], s);
+        __syncthreads();
     }
-    if (row_loss) row_loss[i] = 0.5f * s;
+    if (tid < rows && row_loss) row_loss[r0 + tid] = 0.5f * s;
 }
 
 // Adam with bias correction (Kingma & Ba 2015); refreshes the BF16 weight copy
@@ -713,13 +1184,10 @@ extern "C" int64_t ag_mlp_activation_floats(const ag_mlp* net, int32_t n) {
     return c;
 }
 
-// Split K over a cluster of up to 8 CTAs when the output tiles alone would leave most of the
-// GPU idle (the weight gradients: a few tiles, K = batch rows).
+// the shares of K (product_split) on a cluster of up to 8 CTAs
 static int gemm(cudaStream_t s, int M, int N, int K, const float* A, long sam, long sak, const void* B,
                 bool bbf16, long sbk, long sbn, float* C, long ldc, const float* bias, int epi, float* Z) {
-    const int tiles = nblk(N, BN) * nblk(M, BM);
-    int split = 1;
-    while (split < 8 && tiles * split < 128 && K >= 2 * BK * (split * 2)) split *= 2;
+    const int split = product_split(M, N, K);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nblk(N, BN), nblk(M, BM), split);
     cfg.blockDim = dim3(256, 1, 1);
@@ -741,6 +1209,19 @@ static int gemm(cudaStream_t s, int M, int N, int K, const float* A, long sam, l
     return launch_status("gemm_kernel");
 }
 
+// whether the row-wise kernels take n rows of a network: a layer's outputs fit a CTA's threads with all
+// their shares of K, and the weights can be read in words of eight (four behind layer 0's odd size)
+static bool rows_net(const ag_mlp* net, int n, const void* wbf16) {
+    if (!aligned(wbf16, 16)) return false;
+    for (int l = 0; l <= net->nlayers; ++l)
+        if (net->sizes[l] > kRowWidth || (l > 0 && net->sizes[l] % 8)) return false;
+    for (int l = 0; l < net->nlayers; ++l) {
+        if (!net_split(n, net->sizes[l + 1], net->sizes[l]).row_groups) return false;
+        if (l > 0 && !net_split(n, net->sizes[l], net->sizes[l + 1]).row_groups) return false;
+    }
+    return true;
+}
+
 extern "C" int ag_normalize_inputs(const double* theta, int32_t n, int32_t p, const double* lo,
                                    const double* hi, float* x, void* stream) {
     AG_REQUIRE(theta && lo && hi && x && n > 0 && p > 0, "invalid arguments");
@@ -756,6 +1237,23 @@ extern "C" int ag_mlp_forward(const ag_mlp* net, const float* params, const uint
     cudaStream_t s = as_stream(stream);
     int64_t wo[kMaxLayers], bo[kMaxLayers];
     offsets(net, wo, bo);
+    if (n <= kNetMost && rows_net(net, n, wbf16)) {
+        NetLayers L;
+        L.nlayers = net->nlayers;
+        for (int l = 0; l < net->nlayers; ++l) {
+            L.sizes[l] = net->sizes[l];
+            L.w[l] = wo[l];
+            L.b[l] = bo[l];
+        }
+        L.sizes[net->nlayers] = net->sizes[net->nlayers];
+        rc = cuda_status(cudaFuncSetAttribute(net_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kNetSmem),
+                         "cudaFuncSetAttribute(net_forward_kernel)");
+        if (rc) return rc;
+        net_forward_kernel<<<nblk(n, kNetRows), kNetThreads, kNetSmem, s>>>(
+            L, params, reinterpret_cast<const __nv_bfloat16*>(wbf16), x, n, out, acts);
+        return launch_status("net_forward_kernel");
+    }
     const float* in = x;
     float* a = acts;
     for (int l = 0; l < net->nlayers; ++l) {
@@ -902,9 +1400,44 @@ extern "C" int ag_mlp_backward(const ag_mlp* net, const float* params, const uin
     // dY of the current layer lives in dout (last layer) or in scratch (n x maxw, ping-pong)
     float* cur = dout;
     float* bufs[2] = {scratch, scratch + (int64_t)n * maxw};
+    const bool by_rows = rows_net(net, n, wbf16);
+    if (by_rows) {
+        rc = cuda_status(cudaFuncSetAttribute(net_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kBackSmem),
+                         "cudaFuncSetAttribute(net_backward_kernel)");
+        if (rc) return rc;
+    }
     for (int l = net->nlayers - 1; l >= 0; --l) {
         const int fi = net->sizes[l], fo = net->sizes[l + 1];
         const bool last = (l == net->nlayers - 1);
+        if (by_rows) {
+            // cur holds this layer's dZ
+            const float* hin = (l == 0) ? x : acts + ao[l - 1] + (int64_t)n * fi;
+            const int row_ctas = l > 0 ? nblk(nblk(n, kNetRows), kBackSplit) * kBackSplit : 0;
+            const int sum_ctas = nblk(fo, 8 * kBackSplit) * kBackSplit;
+            const int htiles = nblk(fi, kBackTile), tiles = nblk(fo, kBackTile) * htiles;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(row_ctas + sum_ctas + tiles * kBackSplit);
+            cfg.blockDim = dim3(kNetThreads);
+            cfg.dynamicSmemBytes = kBackSmem;
+            cfg.stream = s;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = kBackSplit;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            float* nxt = bufs[l & 1];
+            rc = cuda_status(cudaLaunchKernelEx(&cfg, net_backward_kernel, n, fi, fo, (const float*)cur,
+                                                reinterpret_cast<const __nv_bfloat16*>(wbf16) + wo[l],
+                                                l > 0 ? acts + ao[l - 1] : nullptr, nxt, row_ctas, sum_ctas, hin, htiles,
+                                                grads + wo[l], grads + bo[l]),
+                             "cudaLaunchKernelEx(net_backward_kernel)");
+            if (rc) return rc;
+            cur = nxt;
+            continue;
+        }
         if (!last) {
             gelu_back_kernel<<<nblk((long)n * fo, 256), 256, 0, s>>>((long)n * fo, acts + ao[l], cur);
             rc = launch_status("gelu_back_kernel");
@@ -931,7 +1464,7 @@ extern "C" int ag_mlp_backward(const ag_mlp* net, const float* params, const uin
 extern "C" int ag_mse_grad(int32_t n, int32_t k, const float* out, const float* target, float* dout,
                            float* row_loss, void* stream) {
     AG_REQUIRE(n > 0 && k > 0 && out && target && dout, "invalid arguments");
-    mse_kernel<<<nblk(n, 256), 256, 0, as_stream(stream)>>>(n, k, out, target, dout, row_loss);
+    mse_kernel<<<nblk(n, kMseRows), 128, 0, as_stream(stream)>>>(n, k, out, target, dout, row_loss);
     return launch_status("mse_kernel");
 }
 
