@@ -179,28 +179,30 @@ class Surrogate:
         out = torch.empty(B, self.k, dtype=torch.float32, device=DEVICE)
         dout = torch.empty_like(out)
         scratch = torch.empty(2 * B * max(self.sizes), dtype=torch.float32, device=DEVICE)
-        rowloss = torch.empty(B, dtype=torch.float32, device=DEVICE)
+        batches = n_all // B if B else 0
+        rowloss = torch.empty(batches, B, dtype=torch.float32, device=DEVICE)
         gen = torch.Generator(device=DEVICE)
         gen.manual_seed(self.seed)
         s = stream_handle()
         net = ctypes.byref(self.net)
+        params, pbf, grads, m, v = (ptr(t) for t in (self.params, self.pbf, self.grads, self.m, self.v))
+        outp, actsp, doutp, scratchp, size = ptr(out), ptr(acts), ptr(dout), ptr(scratch), self.params.numel()
         for ep in range(epochs):
-            perm = torch.randperm(n_all, device=DEVICE, generator=gen)
-            tot = torch.zeros((), dtype=torch.float64, device=DEVICE)
-            for b0 in range(0, n_all - B + 1, B):
-                sel = perm[b0:b0 + B]
-                xb = self._x.index_select(0, sel)
-                yb = self._y.index_select(0, sel)
-                _native.call("ag_mlp_forward", net, ptr(self.params), ptr(self.pbf), ptr(xb), B, ptr(out),
-                             ptr(acts), s)
-                _native.call("ag_mse_grad", B, self.k, ptr(out), ptr(yb), ptr(dout), ptr(rowloss), s)
-                _native.call("ag_mlp_backward", net, ptr(self.params), ptr(self.pbf), ptr(xb), B, ptr(acts),
-                             ptr(dout), ptr(self.grads), ptr(scratch), s)
+            starts = range(0, batches * B, B)
+            # the samples of all batches in order by one gather, and one reduction of their losses
+            # afterwards: per batch the host issues the kernels alone
+            perm = torch.randperm(n_all, device=DEVICE, generator=gen)[:batches * B]
+            xs, ys = self._x.index_select(0, perm), self._y.index_select(0, perm)
+            x0, y0, loss0 = xs.data_ptr(), ys.data_ptr(), rowloss.data_ptr()
+            for b0 in starts:
+                xb, yb = ctypes.c_void_p(x0 + 4 * b0 * xs.shape[1]), ctypes.c_void_p(y0 + 4 * b0 * self.k)
+                _native.call("ag_mlp_forward", net, params, pbf, xb, B, outp, actsp, s)
+                _native.call("ag_mse_grad", B, self.k, outp, yb, doutp, ctypes.c_void_p(loss0 + 4 * b0), s)
+                _native.call("ag_mlp_backward", net, params, pbf, xb, B, actsp, doutp, grads, scratchp, s)
                 self.step_count += 1
-                _native.call("ag_adam_step", self.params.numel(), ptr(self.params), ptr(self.grads), ptr(self.m),
-                             ptr(self.v), self.step_count, lr, 0.9, 0.999, 1e-8, ptr(self.pbf), s)
-                tot += rowloss.double().mean()
-            self.losses.append(float(tot) / max(1, n_all // B))
+                _native.call("ag_adam_step", size, params, grads, m, v, self.step_count, lr, 0.9, 0.999, 1e-8,
+                             pbf, s)
+            self.losses.append(float(rowloss.double().mean(dim=1).sum()) / max(1, batches))
         self.trained = True
         self.pack()
         return self.losses
