@@ -190,6 +190,25 @@ AG_DEVICE_INLINE double warp_sum(double v) {
 AG_DEVICE_INLINE uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
+// asynchronous copies to shared memory, in the thread's groups
+AG_DEVICE_INLINE void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+AG_DEVICE_INLINE void cp_async8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+// 16 or 4 bytes, zeros where !take (src is not read then)
+template <int B> AG_DEVICE_INLINE void cp_async_or_zero(void* dst, const void* src, bool take) {
+    const int bytes = take ? B : 0;
+    if constexpr (B == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes)
+                     : "memory");
+}
+AG_DEVICE_INLINE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> AG_DEVICE_INLINE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 AG_DEVICE_INLINE void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count));

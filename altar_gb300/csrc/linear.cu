@@ -17,6 +17,7 @@
 // observations, K = 16) into one of two TMEM accumulators, and four epilogue
 // warps read the other accumulator with tcgen05.ld and reduce Σ (acc + ρ₀)²
 // per chain straight from registers while the next tile's MMAs run.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -26,6 +27,8 @@
 #include "common.cuh"
 #include "internal.h"
 #include "tcgen05.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace ag {
 
@@ -406,10 +409,14 @@ __global__ void linear_reduce_kernel(int n, int tiles, const double* __restrict_
     llk[i] = (accumulate ? llk[i] : norm) - 0.5 * s;
 }
 
-// Exact FP64 reference path: ρ = A θ - b per chain (one warp per chain, observations strided)
-__global__ void linear_fp64_kernel(const double* __restrict__ A, const double* __restrict__ b,
-                                   const double* __restrict__ theta, int n, int m, int p, double norm,
-                                   double* __restrict__ llk) {
+// Exact FP64 path, llk = norm - ½ |A θ - b|², one warp per chain and observations over the lanes: for
+// more parameters than the staged kernel below holds, and for the smallest products, whose two
+// or three rounds do not pay for the staging (64 chains, 50 x 4: 4.2 µs against 6.2; 50 x 30: 10.3
+// against 8.2)
+constexpr int kExactSmall = 400;                        // observations x parameters
+__global__ void linear_fp64_warp_kernel(const double* __restrict__ A, const double* __restrict__ b,
+                                        const double* __restrict__ theta, int n, int m, int p, double norm,
+                                        double* __restrict__ llk) {
     const int chain = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (chain >= n) return;
     const double* th = theta + (size_t)chain * p;
@@ -421,6 +428,101 @@ __global__ void linear_fp64_kernel(const double* __restrict__ A, const double* _
     }
     acc = warp_sum(acc);
     if (lane == 0) llk[chain] = norm - 0.5 * acc;
+}
+
+// The same, staged.  The floor is the FP64 pipe (64 cycles per warp
+// instruction and scheduler).  A lane owns one of kExactChains chains and every kExactRows-th
+// observation of its CTA's share.  Rows of A come through a double buffer of shared memory, filled
+// ahead by asynchronous copies: read where they are used, each row's first touch of a line was a
+// round trip to L2 that few warps per scheduler could not hide.  The observations are shared out
+// over a cluster of 1 to 8 CTAs; lanes, warps and CTAs are added in a fixed order.
+// 2,003 chains, 997 x 61: 264 -> 232 µs (216 are FP64 operations; 6% is the fullest SM's excess);
+// 1,000 chains 196 -> 121, 64 chains 196 -> 31; 4,096 chains, 500 x 30: 140 -> 127.
+constexpr int kExactWarps = 4;
+constexpr int kExactThreads = kExactWarps * 32;
+constexpr int kExactChains = 8;
+constexpr int kExactRows = kExactThreads / kExactChains;
+constexpr int kExactStage = 1024;                       // doubles of A per stage, at least kExactRows rows
+constexpr int kExactMostP = 600;                        // parameters whose stages fit shared memory
+
+// rounds of kExactRows rows per stage, and a CTA's dynamic shared memory: θ, two stages of A and b
+__host__ __device__ __forceinline__ int exact_rounds(int p) {
+    return p * kExactRows < kExactStage ? kExactStage / (p * kExactRows) : 1;
+}
+__host__ __device__ __forceinline__ size_t exact_smem(int p) {
+    return ((size_t)p * kExactChains + 2 * (size_t)exact_rounds(p) * kExactRows * (p + 1)) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(kExactThreads)
+linear_fp64_kernel(const double* __restrict__ A, const double* __restrict__ b, const double* __restrict__ theta,
+                   int n, int m, int p, double norm, int split, double* __restrict__ llk) {
+    extern __shared__ double s_theta[];                 // [p][kExactChains]
+    __shared__ double s_part[kExactWarps][kExactChains], s_sum[kExactChains];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = blockIdx.x % split, c0 = blockIdx.x / split * kExactChains;
+    const int chains = min(kExactChains, n - c0), tid = threadIdx.x;
+    const int c = tid % kExactChains, row = tid / kExactChains;
+    const int first = (int)((long)m * rank / split), end = (int)((long)m * (rank + 1) / split);
+    double acc = 0.0;
+    const int R = exact_rounds(p) * kExactRows;
+    double* stage = s_theta + p * kExactChains;         // [2][R][p] A, [2][R] b
+    double* stage_b = stage + 2 * R * p;
+    auto load = [&](int r0, int buf) {
+        const int rows = min(R, end - r0);
+        const double* from = A + (size_t)r0 * p;
+        for (int e = tid; e < rows * p; e += kExactThreads) cp_async8(stage + buf * R * p + e, from + e);
+        for (int e = tid; e < rows; e += kExactThreads) cp_async8(stage_b + buf * R + e, b + r0 + e);
+        cp_async_commit();
+    };
+    load(first, 0);
+    for (int e = tid; e < p * kExactChains; e += kExactThreads) {
+        const int q = e / p, j = e - q * p;
+        s_theta[j * kExactChains + q] = theta[(size_t)(c0 + min(q, chains - 1)) * p + j];
+    }
+    int buf = 0;
+    for (int r0 = first; r0 < end; r0 += R, buf ^= 1) {
+        load(r0 + R, buf ^ 1);
+        cp_async_wait<1>();
+        __syncthreads();
+        const int rows = min(R, end - r0);
+        for (int r = row; r < rows; r += kExactRows) {
+            const double* a = stage + (buf * R + r) * p;
+            const double* th = s_theta + c;
+            double s = -stage_b[buf * R + r];
+            int j = 0;
+            for (; j + 8 <= p; j += 8, th += 8 * kExactChains) {
+                double u[8], v[8];                      // all loads before the chain of FMAs
+#pragma unroll
+                for (int q = 0; q < 8; ++q) u[q] = a[j + q], v[q] = th[q * kExactChains];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) s = fma(u[q], v[q], s);
+            }
+            for (; j < p; ++j, th += kExactChains) s = fma(a[j], th[0], s);
+            acc = fma(s, s, acc);
+        }
+        __syncthreads();
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int o = kExactChains; o < 32; o *= 2) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((tid & 31) < kExactChains) s_part[tid >> 5][c] = acc;
+    __syncthreads();
+    if (tid < kExactChains) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kExactWarps; ++w) s += s_part[w][tid];
+        s_sum[tid] = s;
+    }
+    if (split > 1)
+        cluster.sync();
+    else
+        __syncthreads();
+    if (rank == 0 && tid < chains) {
+        double s = s_sum[tid];
+        for (int q = 1; q < split; ++q) s += cluster.map_shared_rank(s_sum, q)[tid];
+        llk[c0 + tid] = norm - 0.5 * s;
+    }
+    if (split > 1) cluster.sync();                      // the sums stay until they have been read
 }
 
 
@@ -550,7 +652,43 @@ extern "C" int ag_whiten_llk_lower(const ag_whiten_block* blk, const float* resi
 extern "C" int ag_linear_llk_fp64(const ag_linear_model* lm, const double* theta, int32_t n, double norm,
                                   double* llk, void* stream) {
     AG_REQUIRE(lm && lm->a64 && lm->b64 && theta && llk && n > 0, "invalid arguments");
-    linear_fp64_kernel<<<cdiv((long)n * 32, 256), 256, 0, as_stream(stream)>>>(lm->a64, lm->b64, theta, n,
-                                                                             lm->m_obs, lm->p, norm, llk);
-    return launch_status("linear_fp64_kernel");
+    if (lm->p <= 0 || lm->p > kExactMostP || (long)lm->m_obs * lm->p <= kExactSmall) {
+        linear_fp64_warp_kernel<<<cdiv((long)n * 32, 256), 256, 0, as_stream(stream)>>>(
+            lm->a64, lm->b64, theta, n, lm->m_obs, lm->p, norm, llk);
+        return launch_status("linear_fp64_warp_kernel");
+    }
+    // The CTAs per group of chains: those whose fullest SM has the least to do, in FMAs per lane
+    // with ~32 for a CTA's start, and a third more for a warp that has its scheduler to itself.
+    // 997 x 61, one CTA against the chosen number: 64 chains 191 and 31 µs (8), 1,000: 191 and 121 (8),
+    // 1,216: 191 and 144 (2), 2,003: 275 and 232 (4); 20,000 chains, 300 x 20: 232 (1) and 242 (4)
+    const int groups = cdiv(n, kExactChains);
+    long best = 0;
+    int split = 1;
+    for (int q = 1; q <= 8; q *= 2) {
+        const long ctas = cdiv((long)groups * q, 152);
+        const long cost = ctas * ((long)cdiv(lm->m_obs, (long)kExactRows * q) * lm->p + 32) * (ctas == 1 ? 4 : 3);
+        if (q == 1 || cost < best) best = cost, split = q;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(groups * split);
+    cfg.blockDim = dim3(kExactThreads);
+    cfg.dynamicSmemBytes = exact_smem(lm->p);
+    cfg.stream = as_stream(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = split;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = split > 1;
+    if (cfg.dynamicSmemBytes > 48 * 1024) {
+        const int rc = cuda_status(cudaFuncSetAttribute(linear_fp64_kernel,
+                                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)exact_smem(kExactMostP)),
+                                   "cudaFuncSetAttribute(linear_fp64_kernel)");
+        if (rc) return rc;
+    }
+    return cuda_status(cudaLaunchKernelEx(&cfg, linear_fp64_kernel, lm->a64, lm->b64, theta, (int)n,
+                                          (int)lm->m_obs, (int)lm->p, norm, split, llk),
+                       "cudaLaunchKernelEx(linear_fp64_kernel)");
 }

@@ -213,19 +213,6 @@ AG_DEVICE_INLINE f32x2 fma2_full(f32x2 a, f32x2 b, f32x2 c) {      // subnormals
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-AG_DEVICE_INLINE void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-// 16 or 4 bytes, zeros where !take (src is not read then)
-template <int B> AG_DEVICE_INLINE void cp_async_or_zero(void* dst, const void* src, bool take) {
-    const int bytes = take ? B : 0;
-    if constexpr (B == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes) : "memory");
-}
-AG_DEVICE_INLINE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> AG_DEVICE_INLINE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // the eight BF16 values of a 16-byte word as FP32
 AG_DEVICE_INLINE void bf16x8(const uint4 v, float (&f)[8]) {
     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
