@@ -187,6 +187,13 @@ AG_DEVICE_INLINE double warp_sum(double v) {
 
 // ---------------------------------------------------------------------------
 // bounded mbarrier helpers (shared::cta)
+// First statement of a kernel that launch_after() starts: waits for the kernel before it on the
+// stream to end, its writes visible, then lets the next one's CTAs come in as this one's leave.
+AG_DEVICE_INLINE void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 AG_DEVICE_INLINE uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }

@@ -67,6 +67,7 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains x
                         int n, int m_obs, int kpb, int mtiles, int ntiles,
                         const float* __restrict__ rho0, double* __restrict__ partial,
                         uint32_t* __restrict__ flags) {
+    after_previous();
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -265,6 +266,7 @@ static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 template <class T>
 __global__ void __launch_bounds__(256) centre_kernel(const T* __restrict__ x, int ld, int col0, int n, int cols,
                                                      double* __restrict__ centre, float2* __restrict__ centre32) {
+    after_previous();
     __shared__ double part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
@@ -331,6 +333,7 @@ __global__ void __launch_bounds__(256) split_rho0_kernel(const T* __restrict__ x
                                                          int cols, int kp, __nv_bfloat16* __restrict__ out, int rho_ctas,
                                                          const double* __restrict__ A, const double* __restrict__ b,
                                                          int m, float* __restrict__ rho0) {
+    after_previous();
     if ((int)blockIdx.x < rho_ctas) {
         const int row = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
         if (row >= m) return;
@@ -401,6 +404,7 @@ __global__ void split_a_kernel(const double* __restrict__ A, int m, int p, int k
 
 __global__ void linear_reduce_kernel(int n, int tiles, const double* __restrict__ partial, double norm,
                                      double* __restrict__ llk, int accumulate) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double s = 0.0;
@@ -417,6 +421,7 @@ constexpr int kExactSmall = 400;                        // observations x parame
 __global__ void linear_fp64_warp_kernel(const double* __restrict__ A, const double* __restrict__ b,
                                         const double* __restrict__ theta, int n, int m, int p, double norm,
                                         double* __restrict__ llk) {
+    after_previous();
     const int chain = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (chain >= n) return;
     const double* th = theta + (size_t)chain * p;
@@ -456,6 +461,7 @@ __host__ __device__ __forceinline__ size_t exact_smem(int p) {
 __global__ void __launch_bounds__(kExactThreads)
 linear_fp64_kernel(const double* __restrict__ A, const double* __restrict__ b, const double* __restrict__ theta,
                    int n, int m, int p, double norm, int split, double* __restrict__ llk) {
+    after_previous();
     extern __shared__ double s_theta[];                 // [p][kExactChains]
     __shared__ double s_part[kExactWarps][kExactChains], s_sum[kExactChains];
     cg::cluster_group cluster = cg::this_cluster();
@@ -563,7 +569,7 @@ static int eval_llk(const T* x, int ld, int col0, int n, int cols, const double*
     float* rho0 = reinterpret_cast<float*>(ws); ws += al256((size_t)m * sizeof(float));
     __nv_bfloat16* split = reinterpret_cast<__nv_bfloat16*>(ws); ws += al256((size_t)n * 2 * kp * 2);
     double* partial = reinterpret_cast<double*>(ws);
-    centre_kernel<T><<<cdiv(cols, 32), 256, 0, s>>>(x, ld, col0, n, cols, centre, centre32);
+    launch_after(centre_kernel<T>, cdiv(cols, 32), 256, 0, s, x, ld, col0, n, cols, centre, centre32);
     int rc = launch_status("centre_kernel");
     if (rc) return rc;
     const typename CentreOf<T>::type* shift;
@@ -572,8 +578,8 @@ static int eval_llk(const T* x, int ld, int col0, int n, int cols, const double*
     else
         shift = centre;
     const int split_ctas = cdiv((long)cdiv(n, kSplitRows) * (kp / 8), 256);
-    split_rho0_kernel<T, LOWER><<<cdiv(m, 8) + split_ctas, 256, 0, s>>>(x, ld, col0, centre, shift, n, cols, kp, split,
-                                                                        cdiv(m, 8), a64, b, m, rho0);
+    launch_after(split_rho0_kernel<T, LOWER>, cdiv(m, 8) + split_ctas, 256, 0, s, x, ld, col0, centre, shift, n,
+                 cols, kp, split, cdiv(m, 8), a64, b, m, rho0);
     rc = launch_status("split_rho0_kernel");
     if (rc) return rc;
     CUtensorMap ma, mb;
@@ -590,11 +596,11 @@ static int eval_llk(const T* x, int ld, int col0, int n, int cols, const double*
     rc = sm_count(&sms);
     if (rc) return rc;
     const int total = mtiles * tiles;
-    linear_misfit_tc_kernel<LOWER><<<total < sms ? total : sms, TC_THREADS, TC_SMEM, s>>>(
-        ma, mb, n, m, kp / TC_BK, mtiles, tiles, rho0, partial, flags);
+    launch_after(linear_misfit_tc_kernel<LOWER>, total < sms ? total : sms, TC_THREADS, TC_SMEM, s, ma, mb, n, m,
+                 kp / TC_BK, mtiles, tiles, rho0, partial, flags);
     rc = launch_status("linear_misfit_tc_kernel");
     if (rc) return rc;
-    linear_reduce_kernel<<<cdiv(n, 128), 128, 0, s>>>(n, tiles, partial, norm, llk, accumulate);
+    launch_after(linear_reduce_kernel, cdiv(n, 128), 128, 0, s, n, tiles, partial, norm, llk, accumulate);
     return launch_status("linear_reduce_kernel");
 }
 
@@ -653,8 +659,8 @@ extern "C" int ag_linear_llk_fp64(const ag_linear_model* lm, const double* theta
                                   double* llk, void* stream) {
     AG_REQUIRE(lm && lm->a64 && lm->b64 && theta && llk && n > 0, "invalid arguments");
     if (lm->p <= 0 || lm->p > kExactMostP || (long)lm->m_obs * lm->p <= kExactSmall) {
-        linear_fp64_warp_kernel<<<cdiv((long)n * 32, 256), 256, 0, as_stream(stream)>>>(
-            lm->a64, lm->b64, theta, n, lm->m_obs, lm->p, norm, llk);
+        launch_after(linear_fp64_warp_kernel, cdiv((long)n * 32, 256), 256, 0, as_stream(stream),
+                     lm->a64, lm->b64, theta, n, lm->m_obs, lm->p, norm, llk);
         return launch_status("linear_fp64_warp_kernel");
     }
     // The CTAs per group of chains: those whose fullest SM has the least to do, in FMAs per lane

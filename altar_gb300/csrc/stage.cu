@@ -331,6 +331,7 @@ __device__ inline uint64_t u64_max(uint64_t a, uint64_t b) { return a > b ? a : 
 __global__ void __launch_bounds__(kMedianThreads) cov_median_kernel(const double* __restrict__ llk, int n,
                                                                     const double* __restrict__ beta,
                                                                     CovState* __restrict__ S) {
+    after_previous();
     __shared__ int s_hist[1 << kMedianBits];
     __shared__ uint64_t s_list[kMedianList];
     __shared__ uint64_t s_a[32], s_b[32];
@@ -931,6 +932,7 @@ __global__ void __launch_bounds__(256) sigma_kernel(const double* __restrict__ t
                                                     const double* __restrict__ w, int n, int p, int chunk,
                                                     int cpb, double* __restrict__ part, double* __restrict__ tot,
                                                     unsigned* __restrict__ done, double* __restrict__ sigma) {
+    after_previous();
     extern __shared__ double sm[];      // x [chunk][p + 1], w x [chunk][p + 1]
     __shared__ double s_red[256];
     const int tid = threadIdx.x, q = p + 1, nent = q * (q + 1) / 2;
@@ -1227,6 +1229,7 @@ __device__ __forceinline__ bool cdf_apply(const double (&v)[PER], const CdfAdd (
 // one CTA; also clears the counts that the next kernel adds to
 __global__ void __launch_bounds__(kCdfThreads) cdf_kernel(const double* __restrict__ w, int n,
                                                           double* __restrict__ edges, int* __restrict__ counts) {
+    after_previous();
     __shared__ CdfAdd s_warp[kCdfThreads / 32];
     __shared__ double s_w[kCdfWarpEnd];
     __shared__ double s_acc;
@@ -1317,6 +1320,7 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_kernel(const double* __restri
 // One thread per uniform.
 __global__ void __launch_bounds__(256) counts_kernel(int n, uint64_t seed, const uint32_t* __restrict__ epoch,
                                                      const double* __restrict__ edges, int* __restrict__ counts) {
+    after_previous();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     u32x4 r = draw(seed, (uint32_t)j, 0u, STREAM_RESAMPLE, 0u, *epoch);
@@ -1349,6 +1353,7 @@ constexpr size_t kRankSmem = (size_t)kRankChunk * sizeof(int) + (size_t)kRankSma
 __global__ void __launch_bounds__(kRankThreads) rank_kernel(int n, const int* __restrict__ counts,
                                                             int* __restrict__ big_row, int* __restrict__ big_cnt,
                                                             int* __restrict__ start, ResampleHdr* __restrict__ hdr) {
+    after_previous();
     extern __shared__ int s_chunk[];               // [kRankThreads][kRankPer]
     uint16_t* s_col = reinterpret_cast<uint16_t*>(s_chunk + kRankChunk);     // [kRankSmall][kRankThreads]
     __shared__ int s_tot[kRankSmall], s_base[kRankSmall], s_seen[kRankSmall];
@@ -1492,6 +1497,7 @@ __global__ void gather_kernel(int n, int p, const double* __restrict__ beta,
                               const double* __restrict__ da_in, double* __restrict__ th_out,
                               double* __restrict__ pr_out, double* __restrict__ da_out,
                               double* __restrict__ po_out) {
+    after_previous();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(t / p), j = (int)(t - (long)i * p);
     if (i >= n) return;
@@ -1676,7 +1682,7 @@ static int cov_schedule_launch(const ag_stage_state* st, const double* data_llk,
     if (grid > want) grid = want;
     rc = cuda_status(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), s), "cudaMemsetAsync(COV barrier)");
     if (rc) return rc;
-    cov_median_kernel<<<1, 1024, 0, s>>>(data_llk, n, st->beta, S);
+    launch_after(cov_median_kernel, 1, 1024, 0, s, data_llk, n, st->beta, S);
     rc = launch_status("cov_median_kernel");
     if (rc) return rc;
     cudaLaunchAttribute attr[1];
@@ -1753,7 +1759,7 @@ extern "C" int ag_weighted_cov(const ag_stage_state* st, const double* theta, in
     unsigned* done = reinterpret_cast<unsigned*>(tot + nent);
     rc = cuda_status(cudaMemsetAsync(done, 0, sizeof(unsigned), s), "cudaMemsetAsync(Σ block count)");
     if (rc) return rc;
-    sigma_kernel<<<nblk, 256, smem, s>>>(theta, st->w, n, p, chunk, cpb, part, tot, done, st->sigma);
+    launch_after(sigma_kernel, nblk, 256, smem, s, theta, st->w, n, p, chunk, cpb, part, tot, done, st->sigma);
     return launch_status("sigma_kernel");
 }
 
@@ -1804,12 +1810,11 @@ extern "C" int ag_resample(const ag_stage_state* st, int32_t n, int32_t p, uint6
     rc = cuda_status(cudaFuncSetAttribute(rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRankSmem),
                      "cudaFuncSetAttribute(rank_kernel)");
     if (rc) return rc;
-    cdf_kernel<<<1, kCdfThreads, 0, s>>>(st->w, n, edges, cnt);
-    counts_kernel<<<blocks(n, 256), 256, 0, s>>>(n, seed, st->epoch, edges, cnt);
-    rank_kernel<<<1, kRankThreads, kRankSmem, s>>>(n, cnt, big_row, big_cnt, start, hdr);
-    gather_kernel<<<(unsigned)(((long)n * p + 255) / 256), 256, 0, s>>>(n, p, st->beta, cnt, start, hdr, theta_in,
-                                                                        prior_in, data_in, theta_out, prior_out,
-                                                                        data_out, post_out);
+    launch_after(cdf_kernel, 1, kCdfThreads, 0, s, st->w, n, edges, cnt);
+    launch_after(counts_kernel, blocks(n, 256), 256, 0, s, n, seed, st->epoch, edges, cnt);
+    launch_after(rank_kernel, 1, kRankThreads, kRankSmem, s, n, cnt, big_row, big_cnt, start, hdr);
+    launch_after(gather_kernel, (unsigned)(((long)n * p + 255) / 256), 256, 0, s, n, p,
+                 st->beta, cnt, start, hdr, theta_in, prior_in, data_in, theta_out, prior_out, data_out, post_out);
     return launch_status("resample kernels");
 }
 

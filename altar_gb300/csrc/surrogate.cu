@@ -290,6 +290,7 @@ AG_DEVICE_INLINE void net_layer(const NetSplit d, int fi, int fo, const float* i
 __global__ void __launch_bounds__(kNetThreads, 1)
 net_forward_kernel(NetLayers net, const float* __restrict__ params, const __nv_bfloat16* __restrict__ wbf,
                    const float* __restrict__ x, int n, float* __restrict__ out, float* __restrict__ acts) {
+    after_previous();
     extern __shared__ __align__(16) uint8_t s_net[];
     constexpr int kCols = kRowWidth * kNetRows;
     float* xT = reinterpret_cast<float*>(s_net + kNetStages * kNetStage);   // [2][kRowWidth][kNetRows]
@@ -439,6 +440,7 @@ __global__ void __launch_bounds__(kNetThreads, 2)
 net_backward_kernel(int n, int fi, int fo, const float* __restrict__ dZ, const __nv_bfloat16* __restrict__ W,
                     const float* __restrict__ Zprev, float* __restrict__ dprev, int row_ctas, int sum_ctas,
                     const float* __restrict__ h, int htiles, float* __restrict__ dW, float* __restrict__ db) {
+    after_previous();
     extern __shared__ __align__(16) float s_back[];
     const int tid = threadIdx.x;
     int block = blockIdx.x;
@@ -616,6 +618,7 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
                     int n, int fo, int kblocks, int mtiles, int ntiles, const float* __restrict__ bias,
                     int gelu_on, float* __restrict__ Z, float* __restrict__ Y,
                     __nv_bfloat16* __restrict__ xnext, int kp_next, uint32_t* __restrict__ flags) {
+    after_previous();
     constexpr uint32_t STAGE = MlpTc<BN>::STAGE;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
@@ -798,6 +801,7 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
 // columns of a row
 __global__ void split_rows_kernel(const float* __restrict__ x, int n, int fi, int kp,
                                   __nv_bfloat16* __restrict__ xs) {
+    after_previous();
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int groups = kp >> 3;
     const long r = e / groups;
@@ -832,6 +836,7 @@ constexpr int kNormRows = 8;
 __global__ void normalize_kernel(const double* __restrict__ theta, int n, int p,
                                  const double* __restrict__ lo, const double* __restrict__ hi,
                                  float* __restrict__ x) {
+    after_previous();
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long band = e / p;
     const int j = (int)(e - band * p);
@@ -875,6 +880,7 @@ constexpr int kMseCols = 64;
 __global__ void __launch_bounds__(128) mse_kernel(int n, int k, const float* __restrict__ out,
                                                   const float* __restrict__ y, float* __restrict__ dY,
                                                   float* __restrict__ row_loss) {
+    after_previous();
     __shared__ float s_d[kMseRows][kMseCols + 1];
     const long r0 = (long)blockIdx.x * kMseRows;
     const int rows = n - r0 < kMseRows ? (int)(n - r0) : kMseRows, tid = threadIdx.x;
@@ -902,6 +908,7 @@ __global__ void __launch_bounds__(128) mse_kernel(int n, int k, const float* __r
 __global__ void adam_kernel(long count, float* __restrict__ p, const float* __restrict__ g,
                             float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2,
                             float eps, float c1, float c2, __nv_bfloat16* __restrict__ pbf) {
+    after_previous();
     long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
     const float gi = g[e];
@@ -939,6 +946,7 @@ __global__ void __launch_bounds__(kSurChains / 8 * (kSurMaxK / kSurRows))
 surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float* __restrict__ scale,
                      const float* __restrict__ G, const float* __restrict__ h, double q0, double norm,
                      double* __restrict__ llk) {
+    after_previous();
     extern __shared__ __align__(16) float s_mem[];
     const int groups = (k + kSurRows - 1) / kSurRows, rows = groups * kSurRows;
     float* sGT = s_mem;                                  // [k][rows], sGT[b][a] = G[a][b]
@@ -1029,6 +1037,7 @@ __global__ void da_screen_kernel(int n, const double* __restrict__ beta, uint64_
                                  const double* __restrict__ prior, const double* __restrict__ sur,
                                  int32_t* __restrict__ pass, int32_t* __restrict__ index,
                                  int32_t* __restrict__ count) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int ok = 0;
@@ -1052,6 +1061,7 @@ __global__ void da_accept_kernel(int n, int p, const double* __restrict__ beta, 
                                  double* __restrict__ data, double* __restrict__ post,
                                  double* __restrict__ sur, unsigned long long* __restrict__ counters,
                                  unsigned long long* __restrict__ screened) {
+    after_previous();
     __shared__ unsigned int s_cnt[4];
     if (threadIdx.x < 4) s_cnt[threadIdx.x] = 0u;
     __syncthreads();
@@ -1095,6 +1105,7 @@ __global__ void da_floor_kernel(int n, const double* __restrict__ beta, uint64_t
                                 const double* __restrict__ csur, const double* __restrict__ prior,
                                 const double* __restrict__ sur, const double* __restrict__ post,
                                 double* __restrict__ floor) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double b = *beta;
@@ -1114,6 +1125,7 @@ __global__ void da_floor_kernel(int n, const double* __restrict__ beta, uint64_t
 __global__ void da_moved_kernel(int n, int p, const double* __restrict__ theta,
                                 const double* __restrict__ theta_s, int32_t* __restrict__ pass,
                                 int32_t* __restrict__ index, int32_t* __restrict__ count) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int moved = 0;
@@ -1136,7 +1148,7 @@ extern "C" int ag_da_moved(int32_t n, int32_t p, const double* theta, const doub
     cudaStream_t s = as_stream(stream);
     int rc = cuda_status(cudaMemsetAsync(count, 0, sizeof(int32_t), s), "memset count");
     if (rc) return rc;
-    da_moved_kernel<<<nblk(n, 256), 256, 0, s>>>(n, p, theta, theta_s, pass, index, count);
+    launch_after(da_moved_kernel, nblk(n, 256), 256, 0, s, n, p, theta, theta_s, pass, index, count);
     return launch_status("da_moved_kernel");
 }
 
@@ -1212,7 +1224,8 @@ static bool rows_net(const ag_mlp* net, int n, const void* wbf16) {
 extern "C" int ag_normalize_inputs(const double* theta, int32_t n, int32_t p, const double* lo,
                                    const double* hi, float* x, void* stream) {
     AG_REQUIRE(theta && lo && hi && x && n > 0 && p > 0, "invalid arguments");
-    normalize_kernel<<<nblk((long)nblk(n, kNormRows) * p, 128), 128, 0, as_stream(stream)>>>(theta, n, p, lo, hi, x);
+    launch_after(normalize_kernel, nblk((long)nblk(n, kNormRows) * p, 128), 128, 0, as_stream(stream), theta, n, p,
+                 lo, hi, x);
     return launch_status("normalize_kernel");
 }
 
@@ -1237,8 +1250,8 @@ extern "C" int ag_mlp_forward(const ag_mlp* net, const float* params, const uint
                                               (int)kNetSmem),
                          "cudaFuncSetAttribute(net_forward_kernel)");
         if (rc) return rc;
-        net_forward_kernel<<<nblk(n, kNetRows), kNetThreads, kNetSmem, s>>>(
-            L, params, reinterpret_cast<const __nv_bfloat16*>(wbf16), x, n, out, acts);
+        launch_after(net_forward_kernel, nblk(n, kNetRows), kNetThreads, kNetSmem, s, L, params,
+                     reinterpret_cast<const __nv_bfloat16*>(wbf16), x, n, out, acts);
         return launch_status("net_forward_kernel");
     }
     const float* in = x;
@@ -1321,8 +1334,8 @@ static int mlp_layer_launch(cudaStream_t s, const __nv_bfloat16* xs, int n, int 
     rc = sm_count(&sms);
     if (rc) return rc;
     const int mtiles = (n + TC_BM - 1) / TC_BM, ntiles = fo / BN, total = mtiles * ntiles;
-    mlp_layer_tc_kernel<BN><<<total < sms ? total : sms, MlpTc<BN>::THREADS, MlpTc<BN>::SMEM, s>>>(
-        mx, mw, n, fo, 2 * kp / TC_BK, mtiles, ntiles, bias, gelu_on, Z, Y, xnext, kp_next, flags);
+    launch_after(mlp_layer_tc_kernel<BN>, total < sms ? total : sms, MlpTc<BN>::THREADS, MlpTc<BN>::SMEM, s, mx, mw,
+                 n, fo, 2 * kp / TC_BK, mtiles, ntiles, bias, gelu_on, Z, Y, xnext, kp_next, flags);
     return launch_status("mlp_layer_tc_kernel");
 }
 
@@ -1343,7 +1356,7 @@ extern "C" int ag_mlp_forward_tc(const ag_mlp* net, const float* params, const u
     __nv_bfloat16* buf[2] = {reinterpret_cast<__nv_bfloat16*>(workspace),
                              reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(workspace) + need / 2)};
     const int fi0 = net->sizes[0], kp0 = mlp_kp(fi0);
-    split_rows_kernel<<<nblk((long)n * (kp0 / 8), 256), 256, 0, s>>>(x, n, fi0, kp0, buf[0]);
+    launch_after(split_rows_kernel, nblk((long)n * (kp0 / 8), 256), 256, 0, s, x, n, fi0, kp0, buf[0]);
     rc = launch_status("split_rows_kernel");
     if (rc) return rc;
     const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(wpack);
@@ -1408,13 +1421,15 @@ extern "C" int ag_mlp_backward(const ag_mlp* net, const float* params, const uin
             cfg.blockDim = dim3(kNetThreads);
             cfg.dynamicSmemBytes = kBackSmem;
             cfg.stream = s;
-            cudaLaunchAttribute attr[1];
+            cudaLaunchAttribute attr[2];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = kBackSplit;
             attr[0].val.clusterDim.y = 1;
             attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
-            cfg.numAttrs = 1;
+            cfg.numAttrs = 2;
             float* nxt = bufs[l & 1];
             rc = cuda_status(cudaLaunchKernelEx(&cfg, net_backward_kernel, n, fi, fo, (const float*)cur,
                                                 reinterpret_cast<const __nv_bfloat16*>(wbf16) + wo[l],
@@ -1451,7 +1466,7 @@ extern "C" int ag_mlp_backward(const ag_mlp* net, const float* params, const uin
 extern "C" int ag_mse_grad(int32_t n, int32_t k, const float* out, const float* target, float* dout,
                            float* row_loss, void* stream) {
     AG_REQUIRE(n > 0 && k > 0 && out && target && dout, "invalid arguments");
-    mse_kernel<<<nblk(n, kMseRows), 128, 0, as_stream(stream)>>>(n, k, out, target, dout, row_loss);
+    launch_after(mse_kernel, nblk(n, kMseRows), 128, 0, as_stream(stream), n, k, out, target, dout, row_loss);
     return launch_status("mse_kernel");
 }
 
@@ -1460,8 +1475,8 @@ extern "C" int ag_adam_step(int64_t count, float* params, const float* grads, fl
                             void* stream) {
     AG_REQUIRE(count > 0 && params && grads && m && v && t >= 1, "invalid arguments");
     const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
-    adam_kernel<<<nblk(count, 256), 256, 0, as_stream(stream)>>>(
-        count, params, grads, m, v, lr, b1, b2, eps, c1, c2, reinterpret_cast<__nv_bfloat16*>(wbf16));
+    launch_after(adam_kernel, nblk(count, 256), 256, 0, as_stream(stream), count, params, grads, m, v, lr, b1, b2,
+                 eps, c1, c2, reinterpret_cast<__nv_bfloat16*>(wbf16));
     return launch_status("adam_kernel");
 }
 
@@ -1484,8 +1499,8 @@ extern "C" int ag_surrogate_llk(int32_t n, int32_t k, const float* coeff, const 
                              "cudaFuncSetAttribute(surrogate_llk_kernel)");
         if (rc) return rc;
     }
-    surrogate_llk_kernel<<<nblk(n, kSurChains), kSurChains / 8 * sur_groups(k), smem, as_stream(stream)>>>(
-        n, k, coeff, scale, gram, h, q0, norm, llk);
+    launch_after(surrogate_llk_kernel, nblk(n, kSurChains), kSurChains / 8 * sur_groups(k), smem, as_stream(stream),
+                 n, k, coeff, scale, gram, h, q0, norm, llk);
     return launch_status("surrogate_llk_kernel");
 }
 
@@ -1498,8 +1513,8 @@ extern "C" int ag_da_screen(const ag_stage_state* st, int32_t n, uint64_t seed, 
     cudaStream_t s = as_stream(stream);
     int rc = cuda_status(cudaMemsetAsync(count, 0, sizeof(int32_t), s), "memset count");
     if (rc) return rc;
-    da_screen_kernel<<<nblk(n, 256), 256, 0, s>>>(n, st->beta, seed, step, st->epoch, mask, cprior, csur,
-                                                  prior, sur, pass, index, count);
+    launch_after(da_screen_kernel, nblk(n, 256), 256, 0, s, n,
+                 st->beta, seed, step, st->epoch, mask, cprior, csur, prior, sur, pass, index, count);
     return launch_status("da_screen_kernel");
 }
 
@@ -1508,8 +1523,8 @@ extern "C" int ag_da_floor(const ag_stage_state* st, int32_t n, uint64_t seed, u
                            const double* sur, const double* post, double* llk_floor, void* stream) {
     AG_REQUIRE(st && n > 0 && mask && pass && cprior && csur && prior && sur && post && llk_floor,
                "invalid arguments");
-    da_floor_kernel<<<nblk(n, 256), 256, 0, as_stream(stream)>>>(n, st->beta, seed, step, st->epoch, mask, pass,
-                                                                  cprior, csur, prior, sur, post, llk_floor);
+    launch_after(da_floor_kernel, nblk(n, 256), 256, 0, as_stream(stream), n,
+                 st->beta, seed, step, st->epoch, mask, pass, cprior, csur, prior, sur, post, llk_floor);
     return launch_status("da_floor_kernel");
 }
 
@@ -1521,8 +1536,7 @@ extern "C" int ag_da_accept(const ag_stage_state* st, int32_t n, int32_t p, uint
     AG_REQUIRE(st && n > 0 && p > 0 && mask && pass && cand && cprior && cdata && csur && theta && prior &&
                    data && post && sur,
                "invalid arguments");
-    da_accept_kernel<<<nblk(n, 256), 256, 0, as_stream(stream)>>>(
-        n, p, st->beta, seed, step, st->epoch, mask, pass, cand, cprior, cdata, csur, theta, prior, data,
-        post, sur, st->counters, screened);
+    launch_after(da_accept_kernel, nblk(n, 256), 256, 0, as_stream(stream), n, p,
+                 st->beta, seed, step, st->epoch, mask, pass, cand, cprior, cdata, csur, theta, prior, data, post, sur, st->counters, screened);
     return launch_status("da_accept_kernel");
 }
