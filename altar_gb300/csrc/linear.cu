@@ -38,25 +38,44 @@ namespace ag {
 // lane 0 issues tcgen05.mma into one of two TMEM accumulators (2 x 256 columns), warps
 // 2-5 read the other accumulator with tcgen05.ld and reduce the previous tile, so the
 // epilogue and the next tile's MMAs overlap.  Tiles are visited in groups of
-// TC_GROUP_M chain tiles so that CTAs running at the same time share both operands' k
+// chain tiles (tile_group) so that CTAs running at the same time share both operands' k
 // slices in L2.  Every wait is bounded; a timeout stops all roles, drains the copies
 // and MMAs in flight and frees TMEM.
 //
 // LOWER: the second operand is lower triangular (W = L⁻¹), so a tile of observations n0 .. n0 + 255
 // needs k < n0 + 256 only; the products left out are zeros (half the multiplications of a dense
-// whitening were).  The tiles of a group are then taken longest first.  Measured, 3,000
-// observations and 16,384 chains: 296 µs (504 µs with the zeros).  (Tiles from a common counter instead of a fixed
-// stride, and the sum over observation tiles by the last CTA of a chain tile instead of a launch
-// of its own, were slower: the fence before the count alone took 12 of 85 µs of the linear model.)
+// whitening were).  The kernel takes 296 µs for 3,000 observations and 16,384 chains (504 µs with the
+// zeros).  The tiles of a group are taken longest first and every other round runs through the CTAs
+// backwards, so that their loads even out; a group is as many chain tiles as keep their split rows in
+// L2, since the fewer the groups, the less their ends cost.  Whole evaluations, against groups of
+// eight chain tiles and one direction: 5,000 chains x 3,000 161 -> 130 µs, 5,000 x 1,300 66 -> 50,
+// 8,192 x 1,200 70 -> 60, 16,384 x 3,000 388 -> 384 (groups of 48 MB 153, 51, 60, 377).  (Tiles from a
+// common counter instead of a fixed stride, and the sum over observation tiles by the last CTA of a
+// chain tile instead of a launch of its own, were slower: the fence before the count alone took 12 of
+// 85 µs of the linear model.)
 constexpr int TC_THREADS = 192;
-constexpr int TC_GROUP_M = 8;
 constexpr uint32_t TC_SMEM = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*bars*/;
 
-AG_DEVICE_INLINE void tile_coords(int t, int mtiles, int ntiles, bool lower, int& mt, int& nt) {
-    const int span = TC_GROUP_M * ntiles;
+// chain tiles per group
+constexpr int TC_GROUP_M = 8;
+constexpr size_t TC_GROUP_BYTES = 96u << 20;              // LOWER: split rows of a group, of 129 MB of L2
+static inline int tile_group(bool lower, int mtiles, int kp) {
+    if (!lower) return TC_GROUP_M;
+    const size_t fit = TC_GROUP_BYTES / ((size_t)TC_BM * 2 * kp * sizeof(__nv_bfloat16));
+    return fit < 1 ? 1 : fit < (size_t)mtiles ? (int)fit : mtiles;
+}
+
+// the i-th tile of this CTA, or `total` and more when there are none left
+AG_DEVICE_INLINE int tile_of(int i, bool lower) {
+    const int c = blockIdx.x, ctas = gridDim.x;
+    return i * ctas + (lower && (i & 1) ? ctas - 1 - c : c);
+}
+
+AG_DEVICE_INLINE void tile_coords(int t, int mtiles, int ntiles, int group, bool lower, int& mt, int& nt) {
+    const int span = group * ntiles;
     const int g = t / span, r = t % span;
-    const int gm = (mtiles - g * TC_GROUP_M) < TC_GROUP_M ? (mtiles - g * TC_GROUP_M) : TC_GROUP_M;
-    mt = g * TC_GROUP_M + r % gm;
+    const int gm = (mtiles - g * group) < group ? (mtiles - g * group) : group;
+    mt = g * group + r % gm;
     nt = lower ? ntiles - 1 - r / gm : r / gm;
 }
 
@@ -64,7 +83,7 @@ template <bool LOWER>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains x 2 kp (BF16)  [hi | lo]
                         const __grid_constant__ CUtensorMap map_b,   // obs    x 3 kp (BF16)  [hi | hi | lo]
-                        int n, int m_obs, int kpb, int mtiles, int ntiles,
+                        int n, int m_obs, int kpb, int mtiles, int ntiles, int group,
                         const float* __restrict__ rho0, double* __restrict__ partial,
                         uint32_t* __restrict__ flags) {
     after_previous();
@@ -117,9 +136,9 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains x
     int issued = 0;                              // TMA stages issued (producer thread)
     if (warp == 0 && lane == 0) {
         // TMA producer: the stage ring runs on across tiles
-        for (int t = blockIdx.x; t < total && !aborted(); t += gridDim.x) {
+        for (int i = 0, t; (t = tile_of(i, LOWER)) < total && !aborted(); ++i) {
             int mt, nt;
-            tile_coords(t, mtiles, ntiles, LOWER, mt, nt);
+            tile_coords(t, mtiles, ntiles, group, LOWER, mt, nt);
             const int len = blocks_of(nt);
             // δ_hi A_hi, δ_lo A_hi, δ_hi A_lo: the first half's blocks serve twice on each side
             int g = 0, k = 0;
@@ -146,10 +165,10 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains x
         // MMA issuer: tile j of this CTA accumulates into TMEM columns (j & 1) * 256
         const uint32_t idesc = idesc_bf16(TC_BM, TC_BN);
         int it = 0, local = 0;
-        for (int t = blockIdx.x; t < total && !aborted(); t += gridDim.x, ++local) {
+        for (int t; (t = tile_of(local, LOWER)) < total && !aborted(); ++local) {
             const int b = local & 1;
             int mt, nt;
-            tile_coords(t, mtiles, ntiles, LOWER, mt, nt);
+            tile_coords(t, mtiles, ntiles, group, LOWER, mt, nt);
             const int kblocks = 3 * blocks_of(nt);
             if (local >= 2 && !mbar_wait_bounded(&tempty[b], (uint32_t)((local >> 1) - 1) & 1u, TC_WAIT)) {
                 atomicExch(&s_abort, 1);
@@ -185,10 +204,10 @@ linear_misfit_tc_kernel(const __grid_constant__ CUtensorMap map_a,   // chains x
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         float* rho = s_rho[quarter];
         int local = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++local) {
+        for (int t; (t = tile_of(local, LOWER)) < total; ++local) {
             const int b = local & 1;
             int mt, nt;
-            tile_coords(t, mtiles, ntiles, LOWER, mt, nt);
+            tile_coords(t, mtiles, ntiles, group, LOWER, mt, nt);
             const int n0 = nt * TC_BN;
             // observations past the end have zero rows in the operand: with ρ₀ = 0 they add nothing
 #pragma unroll
@@ -597,7 +616,7 @@ static int eval_llk(const T* x, int ld, int col0, int n, int cols, const double*
     if (rc) return rc;
     const int total = mtiles * tiles;
     launch_after(linear_misfit_tc_kernel<LOWER>, total < sms ? total : sms, TC_THREADS, TC_SMEM, s, ma, mb, n, m,
-                 kp / TC_BK, mtiles, tiles, rho0, partial, flags);
+                 kp / TC_BK, mtiles, tiles, tile_group(LOWER, mtiles, kp), rho0, partial, flags);
     rc = launch_status("linear_misfit_tc_kernel");
     if (rc) return rc;
     launch_after(linear_reduce_kernel, cdiv(n, 128), 128, 0, s, n, tiles, partial, norm, llk, accumulate);
