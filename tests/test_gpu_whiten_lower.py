@@ -49,3 +49,25 @@ def test_lower_whitening(cuda, m, n):
     dz = (3 * 2.0 ** -17 + 3 * m * 2.0 ** -24) * ((x - centre).abs() @ W.abs().T) + 2.0 ** -23 * (W @ centre).abs()
     miss = (torch.from_numpy(3.0 - got["ag_whiten_llk"]).cuda() - (z * z).sum(1)).abs()
     assert bool((miss <= (2 * z.abs() * dz + dz * dz).sum(1) + 1e-14).all())
+
+
+@pytest.mark.parametrize("m,n", [(3000, 9000), (700, 20001), (600, 9473)])
+def test_lower_whitening_tile_order(cuda, m, n):
+    """Several rounds of tiles, in two groups (3,000) and in one, forwards and backwards."""
+    lib = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(m)
+    W = torch.tril(torch.randn(m, m, generator=g, device="cuda", dtype=torch.float64)) / m ** 0.5
+    r = torch.randn(n, m, generator=g, device="cuda")
+    split = torch.empty(m * 3 * lib.ag_linear_kpad(m), dtype=torch.int16, device="cuda")
+    _native.call("ag_linear_prepare", ptr(W), m, m, ptr(split), stream_handle())
+    block = _native.WhitenBlock(W.data_ptr(), split.data_ptr(), 0, m)
+    ws = workspace(lib.ag_whiten_workspace_bytes(m, n))
+    flags = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = []
+    for name in ("ag_whiten_llk", "ag_whiten_llk_lower"):
+        llk = torch.zeros(n, dtype=torch.float64, device="cuda")
+        _native.call(name, ctypes.byref(block), ptr(r), m, n, ptr(llk), ptr(ws), ws.numel(), ptr(flags),
+                     stream_handle())
+        got.append(llk)
+    assert int(flags.item()) == 0 and bool((got[0] < 0).all())
+    assert torch.equal(got[0], got[1])
