@@ -599,27 +599,29 @@ net_backward_kernel(int n, int fi, int fo, const float* __restrict__ dZ, const _
 // tcgen05.mma into one of two TMEM accumulators, epilogue warps reading the other with
 // tcgen05.ld); the epilogue adds the bias, applies GELU and writes the next layer's split
 // BF16 input directly, plus the FP32 pre-activation Z and output Y where asked.
-// The epilogue bounds a layer: ~35 instructions an element, most of them the error function's.
-// Sixteen warps share it (eight for 64 columns): 27 µs for 32,768 x 256 x 256, 33 µs with four.
+// The epilogue is what a layer cannot hide: ~35 instructions an element, most of them the error
+// function's.  Tiles of 64 columns, two CTAs per SM with eight epilogue warps each, leave the last
+// wave nearly full (32,768 rows: 7 tiles per SM where the mean is 6.7; of 256 columns 2 where it is
+// 1.7).  They read X four times, so a CTA keeps to one block of columns and holds its weights (up to
+// kMlpHeld inputs; both halves of K' use the same ones), which leaves X alone to stream from L2.
+// Layers of 10-256-256-256-256-64, from tiles of 256 columns and one CTA per SM with 16 epilogue
+// warps: 256 rows 60 -> 33 µs, 8,192 64 -> 44, 32,768 110 -> 101, 65,536 233 -> 177 (tiles of 128 columns:
+// 37, 42, 105, 185); 10-64-128-64 loses 8% at 65,536 (43 -> 46).
+constexpr int kMlpCols = 64;                                 // columns of a tile
+constexpr int kMlpEpi = 8;                                   // epilogue warps, 32 columns each
+constexpr int kMlpThreads = 64 + 32 * kMlpEpi;
+constexpr int kMlpCtas = 2;                                  // per SM
+constexpr uint32_t kMlpW = kMlpCols * TC_BK * 2;             // bytes of a K-block of weights
+constexpr int kMlpHeld = TC_STAGES * TC_BK;                  // the held weights take the ring's place for them
+constexpr uint32_t kMlpSmem = TC_STAGES * (TC_A_BYTES + kMlpW) + 1024 + 256;
 
-template <int BN>
-struct MlpTc {
-    static constexpr int EPI = BN >= 128 ? 16 : 8;           // epilogue warps
-    static constexpr int THREADS = 64 + 32 * EPI;
-    static constexpr uint32_t B_BYTES = BN * TC_BK * 2;
-    static constexpr uint32_t STAGE = TC_A_BYTES + B_BYTES;
-    static constexpr uint32_t SMEM = TC_STAGES * STAGE + 1024 + 256;
-};
-
-template <int BN>
-__global__ void __launch_bounds__(MlpTc<BN>::THREADS, 1)
+__global__ void __launch_bounds__(kMlpThreads, kMlpCtas)
 mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' split BF16 activations
                     const __grid_constant__ CUtensorMap map_w,   // fo x K' packed BF16 weights
                     int n, int fo, int kblocks, int mtiles, int ntiles, const float* __restrict__ bias,
                     int gelu_on, float* __restrict__ Z, float* __restrict__ Y,
                     __nv_bfloat16* __restrict__ xnext, int kp_next, uint32_t* __restrict__ flags) {
-    after_previous();
-    constexpr uint32_t STAGE = MlpTc<BN>::STAGE;
+    constexpr uint32_t STAGE = TC_A_BYTES + kMlpW;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -630,13 +632,17 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
     uint64_t* tfull = bars + 2 * TC_STAGES;
     uint64_t* tempty = bars + 2 * TC_STAGES + 2;
     uint64_t* drain = bars + 2 * TC_STAGES + 4;
-    constexpr int EPI = MlpTc<BN>::EPI, COLS = BN * 4 / EPI;  // columns per epilogue warp
-    static_assert(COLS % 32 == 0, "whole tcgen05.ld of 32 columns");
+    uint64_t* wfull = bars + 2 * TC_STAGES + 5;
+    constexpr int EPI = kMlpEpi, COLS = 32, BN = kMlpCols;   // COLS: columns per epilogue warp
+    // held weights: K-blocks behind the ring's A tiles; else next to each A tile
+    const bool held = kblocks * TC_BK <= 2 * kMlpHeld;
+    const uint32_t astep = held ? TC_A_BYTES : STAGE;
+    const uint32_t wbase = base + TC_STAGES * TC_A_BYTES;
+    const int nt = blockIdx.x % ntiles, m0 = blockIdx.x / ntiles, mstep = gridDim.x / ntiles;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     __shared__ __align__(16) float s_bias[EPI][COLS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int total = mtiles * ntiles;
     if (threadIdx.x == 0) {
         for (int st = 0; st < TC_STAGES; ++st) {
             mbar_init(&full[st], 1);
@@ -647,6 +653,7 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
             mbar_init(&tempty[b], EPI);
         }
         mbar_init(drain, 1);
+        mbar_init(wfull, 1);
         fence_mbar_init();
         s_abort = 0;
     }
@@ -660,11 +667,17 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     auto aborted = [&]() { return *(volatile int*)&s_abort != 0; };
+    // the weights were packed at least two kernels ago (the rows are split in between)
+    if (held && threadIdx.x == 0) {
+        mbar_arrive_expect_tx(wfull, kblocks / 2 * kMlpW);
+        for (int kb = 0; kb < kblocks / 2; ++kb)
+            tma_load_2d(wbase + kb * kMlpW, &map_w, kb * TC_BK, nt * BN, smem_addr(wfull));
+    }
+    after_previous();
 
     int issued = 0;
     if (warp == 0 && lane == 0) {
-        for (int t = blockIdx.x; t < total && !aborted(); t += gridDim.x) {
-            const int mt = t % mtiles, nt = t / mtiles;
+        for (int mt = m0; mt < mtiles && !aborted(); mt += mstep) {
             for (int kb = 0; kb < kblocks; ++kb, ++issued) {
                 const int st = issued % TC_STAGES;
                 if (issued >= TC_STAGES &&
@@ -673,16 +686,17 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
                     break;
                 }
                 if (aborted()) break;
-                const uint32_t sa = base + st * STAGE;
-                mbar_arrive_expect_tx(&full[st], STAGE);
+                const uint32_t sa = base + st * astep;
+                mbar_arrive_expect_tx(&full[st], astep);
                 tma_load_2d(sa, &map_x, kb * TC_BK, mt * TC_BM, smem_addr(&full[st]));
-                tma_load_2d(sa + TC_A_BYTES, &map_w, kb * TC_BK, nt * BN, smem_addr(&full[st]));
+                if (!held) tma_load_2d(sa + TC_A_BYTES, &map_w, kb * TC_BK, nt * BN, smem_addr(&full[st]));
             }
         }
     } else if (warp == 1 && lane == 0) {
         const uint32_t idesc = idesc_bf16(TC_BM, BN);
         int it = 0, local = 0;
-        for (int t = blockIdx.x; t < total && !aborted(); t += gridDim.x, ++local) {
+        if (held && !mbar_wait_bounded(wfull, 0, TC_WAIT)) atomicExch(&s_abort, 1);
+        for (int mt = m0; mt < mtiles && !aborted(); mt += mstep, ++local) {
             const int b = local & 1;
             if (local >= 2 && !mbar_wait_bounded(&tempty[b], (uint32_t)((local >> 1) - 1) & 1u, TC_WAIT)) {
                 atomicExch(&s_abort, 1);
@@ -698,8 +712,9 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
                     break;
                 }
                 tc_fence_after();
-                const uint32_t sa = base + st * STAGE;
-                const uint64_t adesc = sw128_desc(sa), bdesc = sw128_desc(sa + TC_A_BYTES);
+                const uint32_t sa = base + st * astep;
+                const uint64_t adesc = sw128_desc(sa);
+                const uint64_t bdesc = sw128_desc(held ? wbase + kb % (kblocks / 2) * kMlpW : sa + TC_A_BYTES);
 #pragma unroll
                 for (int k = 0; k < TC_BK / 16; ++k)
                     mma_bf16(acc_addr, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
@@ -719,11 +734,11 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         float* bs = s_bias[warp - 2];
         int local = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++local) {
+        const int n0 = nt * BN + first;                                // fo is a multiple of BN
+        bs[lane] = __ldg(bias + n0 + lane);
+        __syncwarp();
+        for (int mt = m0; mt < mtiles; mt += mstep, ++local) {
             const int b = local & 1;
-            const int mt = t % mtiles, nt = t / mtiles;
-            const int n0 = nt * BN + first;                            // fo is a multiple of BN
-            for (int c = lane; c < COLS; c += 32) bs[c] = __ldg(bias + n0 + c);
             const bool ok = __all_sync(0xffffffffu,
                                        mbar_wait_bounded(&tfull[b], (uint32_t)(local >> 1) & 1u, TC_WAIT));
             if (!ok || aborted()) {
@@ -734,52 +749,50 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
             tc_fence_after();
             const int row = mt * TC_BM + quarter * 32 + lane;
             const bool live = row < n;
-#pragma unroll 1
-            for (int c0 = 0; c0 < COLS; c0 += 32) {
-                uint32_t r[32];
-                tmem_ld32_nowait(tmem + lane_base + (uint32_t)(b * BN + first + c0), r);
-                tmem_wait_ld();
-                const size_t o = (size_t)row * fo + n0 + c0;
-                __nv_bfloat16* hi = xnext + (size_t)row * (2 * kp_next) + n0 + c0;
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    float z[8], y[8];
-#pragma unroll
-                    for (int q = 0; q < 8; q += 4) {
-                        const float4 bb = *reinterpret_cast<const float4*>(bs + c0 + i + q);
-                        z[q] = __uint_as_float(r[i + q]) + bb.x;
-                        z[q + 1] = __uint_as_float(r[i + q + 1]) + bb.y;
-                        z[q + 2] = __uint_as_float(r[i + q + 2]) + bb.z;
-                        z[q + 3] = __uint_as_float(r[i + q + 3]) + bb.w;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) y[q] = gelu_on ? gelu(z[q]) : z[q];
-                    if (live && Z) {
-#pragma unroll
-                        for (int q = 0; q < 8; q += 4)
-                            *reinterpret_cast<float4*>(Z + o + i + q) = make_float4(z[q], z[q + 1], z[q + 2], z[q + 3]);
-                    }
-                    if (live && Y) {
-#pragma unroll
-                        for (int q = 0; q < 8; q += 4)
-                            *reinterpret_cast<float4*>(Y + o + i + q) = make_float4(y[q], y[q + 1], y[q + 2], y[q + 3]);
-                    }
-                    if (live && xnext) {
-                        __align__(16) __nv_bfloat162 h2[4], l2[4];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            h2[q] = __floats2bfloat162_rn(y[2 * q], y[2 * q + 1]);
-                            l2[q] = __floats2bfloat162_rn(y[2 * q] - __low2float(h2[q]),
-                                                          y[2 * q + 1] - __high2float(h2[q]));
-                        }
-                        *reinterpret_cast<uint4*>(hi + i) = *reinterpret_cast<const uint4*>(h2);
-                        *reinterpret_cast<uint4*>(hi + kp_next + i) = *reinterpret_cast<const uint4*>(l2);
-                    }
-                }
-            }
+            uint32_t r[32];
+            tmem_ld32_nowait(tmem + lane_base + (uint32_t)(b * BN + first), r);
+            tmem_wait_ld();
+            // the accumulator is free for the next tile but one
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[b]);
+            const size_t o = (size_t)row * fo + n0;
+            __nv_bfloat16* hi = xnext + (size_t)row * (2 * kp_next) + n0;
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+                float z[8], y[8];
+#pragma unroll
+                for (int q = 0; q < 8; q += 4) {
+                    const float4 bb = *reinterpret_cast<const float4*>(bs + i + q);
+                    z[q] = __uint_as_float(r[i + q]) + bb.x;
+                    z[q + 1] = __uint_as_float(r[i + q + 1]) + bb.y;
+                    z[q + 2] = __uint_as_float(r[i + q + 2]) + bb.z;
+                    z[q + 3] = __uint_as_float(r[i + q + 3]) + bb.w;
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) y[q] = gelu_on ? gelu(z[q]) : z[q];
+                if (live && Z) {
+#pragma unroll
+                    for (int q = 0; q < 8; q += 4)
+                        *reinterpret_cast<float4*>(Z + o + i + q) = make_float4(z[q], z[q + 1], z[q + 2], z[q + 3]);
+                }
+                if (live && Y) {
+#pragma unroll
+                    for (int q = 0; q < 8; q += 4)
+                        *reinterpret_cast<float4*>(Y + o + i + q) = make_float4(y[q], y[q + 1], y[q + 2], y[q + 3]);
+                }
+                if (live && xnext) {
+                    __align__(16) __nv_bfloat162 h2[4], l2[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        h2[q] = __floats2bfloat162_rn(y[2 * q], y[2 * q + 1]);
+                        l2[q] = __floats2bfloat162_rn(y[2 * q] - __low2float(h2[q]),
+                                                      y[2 * q + 1] - __high2float(h2[q]));
+                    }
+                    *reinterpret_cast<uint4*>(hi + i) = *reinterpret_cast<const uint4*>(h2);
+                    *reinterpret_cast<uint4*>(hi + kp_next + i) = *reinterpret_cast<const uint4*>(l2);
+                }
+            }
         }
     }
     __syncthreads();
@@ -788,6 +801,7 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
         for (int k = (issued > TC_STAGES ? issued - TC_STAGES : 0); k < issued; ++k)
             mbar_wait_bounded(&full[k % TC_STAGES], (uint32_t)(k / TC_STAGES) & 1u, TC_WAIT);
     }
+    if (warp == 0 && held) mbar_wait_bounded(wfull, 0, TC_WAIT);
     if (warp == 1) mbar_wait_bounded(drain, 0, TC_WAIT);
     tc_fence_before();
     __syncthreads();
@@ -1317,25 +1331,26 @@ extern "C" size_t ag_mlp_tc_workspace_bytes(const ag_mlp* net, int32_t n) {
     return 2 * one;
 }
 
-template <int BN>
 static int mlp_layer_launch(cudaStream_t s, const __nv_bfloat16* xs, int n, int kp, const __nv_bfloat16* w,
                             int fo, const float* bias, int gelu_on, float* Z, float* Y, __nv_bfloat16* xnext,
                             int kp_next, uint32_t* flags) {
     CUtensorMap mx, mw;
     int rc = make_map(&mx, xs, n, 2 * kp, TC_BM);
     if (rc) return rc;
-    rc = make_map(&mw, w, fo, 2 * kp, BN);
+    rc = make_map(&mw, w, fo, 2 * kp, kMlpCols);
     if (rc) return rc;
-    rc = cuda_status(cudaFuncSetAttribute(mlp_layer_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)MlpTc<BN>::SMEM),
+    rc = cuda_status(cudaFuncSetAttribute(mlp_layer_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kMlpSmem),
                      "cudaFuncSetAttribute(mlp_layer_tc_kernel)");
     if (rc) return rc;
     int sms = 0;
     rc = sm_count(&sms);
     if (rc) return rc;
-    const int mtiles = (n + TC_BM - 1) / TC_BM, ntiles = fo / BN, total = mtiles * ntiles;
-    launch_after(mlp_layer_tc_kernel<BN>, total < sms ? total : sms, MlpTc<BN>::THREADS, MlpTc<BN>::SMEM, s, mx, mw,
-                 n, fo, 2 * kp / TC_BK, mtiles, ntiles, bias, gelu_on, Z, Y, xnext, kp_next, flags);
+    // as many CTAs per block of columns as there are places for, or tiles
+    const int mtiles = (n + TC_BM - 1) / TC_BM, ntiles = fo / kMlpCols;
+    const int places = kMlpCtas * sms / ntiles, per_block = places < 1 ? 1 : places < mtiles ? places : mtiles;
+    launch_after(mlp_layer_tc_kernel, ntiles * per_block, kMlpThreads, kMlpSmem, s, mx, mw, n, fo,
+                 2 * kp / TC_BK, mtiles, ntiles, bias, gelu_on, Z, Y, xnext, kp_next, flags);
     return launch_status("mlp_layer_tc_kernel");
 }
 
@@ -1368,11 +1383,7 @@ extern "C" int ag_mlp_forward_tc(const ag_mlp* net, const float* params, const u
         float* Y = last ? out : (a ? a + (int64_t)n * fo : nullptr);
         __nv_bfloat16* xnext = last ? nullptr : buf[(l + 1) & 1];
         const int kp_next = last ? 0 : mlp_kp(fo);
-        rc = (fo % 256 == 0)
-                 ? mlp_layer_launch<256>(s, buf[l & 1], n, kp, w, fo, params + bo[l], last ? 0 : 1, Z, Y, xnext,
-                                         kp_next, flags)
-                 : mlp_layer_launch<64>(s, buf[l & 1], n, kp, w, fo, params + bo[l], last ? 0 : 1, Z, Y, xnext,
-                                        kp_next, flags);
+        rc = mlp_layer_launch(s, buf[l & 1], n, kp, w, fo, params + bo[l], last ? 0 : 1, Z, Y, xnext, kp_next, flags);
         if (rc) return rc;
         w += (size_t)fo * 2 * kp;
         if (a) a += 2 * (int64_t)n * fo;
