@@ -22,7 +22,7 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<size_t>(
 // Launch behind the kernel before it on the stream without waiting for that one's last CTA to leave
 // first (programmatic dependent launch).  The kernel's first statement is after_previous(), so it
 // touches memory only when its predecessor has ended; what it saves is the gap, ~2 µs per launch of
-// a chain of short kernels: linear model (4 kernels, 8,192 chains) 107 -> 98 µs, surrogate
+// a chain of short kernels: linear model (4 kernels, 16,384 chains) 107 -> 98 µs, surrogate
 // prediction (8) 158 -> 141, a stage's schedule, covariance and resampling (8) 275 -> 261, training
 // (8 per batch) 769 -> 753.  Not for the walk's propose, forward and accept kernels: a short run that
 // captures and replays 61 of them per stage took 5.4 ms instead of 4.6.
