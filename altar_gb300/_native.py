@@ -171,6 +171,7 @@ _SIGNATURES = {
     "ag_propose": (c_int, [P, P, c_int32, c_int32, P, P, c_uint64, c_uint32, P, P, P, P]),
     "ag_accept_floor": (c_int, [P, c_int32, c_uint64, c_uint32, P, P, P, P, P]),
     "ag_accept": (c_int, [P, c_int32, c_int32, c_uint64, c_uint32, P, P, P, P, P, P, P, P, P]),
+    "ag_accept_propose": (c_int, [P, c_int32, c_int32, P, P, c_uint64, c_uint32, P, P, P, P, P, P, P, P, P, P]),
     "ag_cov_workspace_bytes": (c_size_t, [c_int32]),
     "ag_cov_schedule": (c_int, [P, P, c_int32, c_double, c_double, P, c_size_t, P]),
     "ag_cov_schedule_brent": (c_int, [P, P, c_int32, c_double, c_double, c_int32, P, c_size_t, P]),

@@ -4,8 +4,8 @@ Same configuration (scaling .1, acceptanceWeight 8, rejectionWeight 1) and
 the same per-step semantics: propose θ' = θ + (L z)ᵀ with L = chol(scaling² Σ),
 reject samples outside the model's support (and, for the CDM, above the free
 surface), evaluate the likelihoods of every candidate, accept where
-log u <= post' - post.  Each step is three launches: propose (+verify +prior),
-the fused forward model, accept.
+log u <= post' - post.  Each step is the fused forward model and one launch that
+accepts and proposes (+verify +prior) for the next step.
 
 early_reject: before the forward model, the log-likelihood below which each proposal is
 certainly rejected (the accept test's own uniform, ag_accept_floor); a forward model that
@@ -94,24 +94,37 @@ class Metropolis:
         early = self.early_reject and getattr(model.strategy, "supports_floor", False)
         if early and (self._floor is None or self._floor.shape[0] != n):
             self._floor = torch.empty(n, dtype=torch.float64, device=DEVICE)
+        # the accept of a step and the proposal (and floor) of the next share a launch, unless a
+        # monitor looks in between
+        fused = not any(hasattr(m, ev) for m in getattr(d, "monitors", ()) for ev in
+                        (d.acceptFinish, d.chainAdvanceFinish, d.chainAdvanceStart, d.verifyStart, d.verifyFinish,
+                         d.dataStart))
         for k in range(self.steps):
             d.notify(event=d.chainAdvanceStart, controller=annealer)
             d.notify(event=d.verifyStart, controller=annealer)
-            _native.call("ag_propose", st, ptr(step.theta), n, p, ptr(model.lo), ptr(model.hi),
-                         self.seed, k, ptr(cand), ptr(mask), ptr(cprior), s)
+            ready = fused and k > 0                  # proposed with the previous step's accept
+            if not ready:
+                _native.call("ag_propose", st, ptr(step.theta), n, p, ptr(model.lo), ptr(model.hi),
+                             self.seed, k, ptr(cand), ptr(mask), ptr(cprior), s)
             d.notify(event=d.verifyFinish, controller=annealer)
             d.notify(event=d.dataStart, controller=annealer)
             if early:
-                _native.call("ag_accept_floor", st, n, self.seed, k, ptr(mask), ptr(cprior), ptr(step.posterior),
-                             ptr(self._floor), s)
+                if not ready:
+                    _native.call("ag_accept_floor", st, n, self.seed, k, ptr(mask), ptr(cprior),
+                                 ptr(step.posterior), ptr(self._floor), s)
                 model.strategy.forward(cand, cdata, mask=mask, status=mask, floor=self._floor)
             else:
                 model.strategy.forward(cand, cdata, mask=mask, status=mask)
             d.notify(event=d.dataFinish, controller=annealer)
             d.notify(event=d.acceptStart, controller=annealer)
-            _native.call("ag_accept", st, n, p, self.seed, k, ptr(mask), ptr(cand), ptr(cprior),
-                         ptr(cdata), ptr(step.theta), ptr(step.prior), ptr(step.data),
-                         ptr(step.posterior), s)
+            if fused and k + 1 < self.steps:
+                _native.call("ag_accept_propose", st, n, p, ptr(model.lo), ptr(model.hi), self.seed, k, ptr(mask),
+                             ptr(cand), ptr(cprior), ptr(cdata), ptr(step.theta), ptr(step.prior), ptr(step.data),
+                             ptr(step.posterior), ptr(self._floor) if early else None, s)
+            else:
+                _native.call("ag_accept", st, n, p, self.seed, k, ptr(mask), ptr(cand), ptr(cprior),
+                             ptr(cdata), ptr(step.theta), ptr(step.prior), ptr(step.data),
+                             ptr(step.posterior), s)
             d.notify(event=d.acceptFinish, controller=annealer)
             d.notify(event=d.chainAdvanceFinish, controller=annealer)
         # accepted, rejected, unlikely stay on the device until the stage report

@@ -76,6 +76,23 @@ __global__ void prior_llk_kernel(const double* __restrict__ theta, int n, int p,
     if (prior) prior[i] = s_prior;
 }
 
+// log u > d for u in (0, 1]: decided in FP32 unless the two are closer than that logarithm's error
+// (u rounds to FP32 within 2^-24 of itself and logf is good to 2 ulp: below 1e-6 (1 + |log u|)).
+// The FP64 logarithm was a quarter of accept_kernel: 4,096 chains 7.7 -> 5.7 µs.
+__device__ inline bool log_exceeds(double u, double d) {
+    const float l = logf((float)u);
+    const double gap = (double)l - d;
+    if (fabs(gap) > 1e-5 * (1.0 + fabs((double)l))) return gap > 0.0;
+    return log(u) > d;
+}
+
+// the acceptance floor of a chain inside the support from its post + log u (accept_floor_kernel)
+__device__ inline double floor_of(double post_logu, double cprior, double b) {
+    double f = (post_logu - cprior) / b;
+    f -= (fabs(f) + 1.0) * 1e-9;
+    return f == f ? f : -INFINITY;
+}
+
 // ---------------------------------------------------------------------------
 // Metropolis proposal, verify and prior (Metropolis.py:160-183, 236-259).  A block takes
 // kProposeChains chains: a thread per pair of normals (a logarithm, a square root and a sine and
@@ -84,27 +101,69 @@ __global__ void prior_llk_kernel(const double* __restrict__ theta, int n, int p,
 // then the rows, replaced by θ where an entry left the support.  Measured:
 // 4,096 chains, 6 parameters 7.3 µs (23.5 µs with a thread per chain); 1,024 chains, 4 parameters
 // 7.0 µs (16.4 µs).
+//
+// ACCEPT: first accepts or rejects the previous step's candidates, as accept_kernel does, in a warp
+// of its own beside the normals, and forms the new candidates' floors, as accept_floor_kernel does.
+// Each is a launch of 5 to 6 µs, nearly all latency; the kernel takes 7.5 µs with and 7.4 without them, and
+// a Reverso run of 4,096 chains and 20 steps per stage 4.3 ms instead of 4.6.
 constexpr int kProposeChains = 32;
-constexpr int kProposeThreads = 192;
-__global__ void __launch_bounds__(kProposeThreads)
-propose_kernel(const double* __restrict__ theta, int n, int p, const double* __restrict__ chol,
+struct AcceptArgs {
+    const double *beta, *cdata;
+    double *prior, *data, *post;
+    unsigned long long* counters;
+    double* floor;                             // null: none wanted
+};
+template <bool ACCEPT> constexpr int kProposeThreads = ACCEPT ? 224 : 192;
+
+template <bool ACCEPT>
+__global__ void __launch_bounds__(kProposeThreads<ACCEPT>)
+propose_kernel(double* theta, int n, int p, const double* __restrict__ chol,
                const double* __restrict__ lo, const double* __restrict__ hi, uint64_t seed, uint32_t step,
-               const uint32_t* __restrict__ epoch, double* __restrict__ cand, uint32_t* __restrict__ mask,
-               double* __restrict__ cprior, int chain0) {
+               const uint32_t* __restrict__ epoch, double* cand, uint32_t* mask, double* cprior, int chain0,
+               AcceptArgs acc) {
+    constexpr int kThreads = kProposeThreads<ACCEPT>;
     __shared__ double sz[kProposeChains * kMaxP], sv[kProposeChains * kMaxP], sL[kMaxP * kMaxP];
-    __shared__ double s_prior;
-    __shared__ int s_out[kProposeChains];
+    __shared__ double s_prior, s_floor[kProposeChains];
+    __shared__ int s_out[kProposeChains], s_take[kProposeChains];
     const int tid = threadIdx.x, i0 = blockIdx.x * kProposeChains;
     const int chains = n - i0 < kProposeChains ? n - i0 : kProposeChains;
     const uint32_t ep = *epoch;
     const int pairs = (p + 1) >> 1;
-    for (int k = tid; k < p * p; k += kProposeThreads) sL[k] = chol[k];
+    for (int k = tid; k < p * p; k += kThreads) sL[k] = chol[k];
     if (tid < kProposeChains) s_out[tid] = 0;
-    if (tid >= kProposeThreads - 32) {         // the last warp has the fewest pairs
+    if (tid >= kThreads - 32) {                // the last warp has the fewest pairs
         const double lp = uniform_log_prior(p, lo, hi);
-        if (tid == kProposeThreads - 1) s_prior = lp;
+        if (tid == kThreads - 1) s_prior = lp;
+    } else if (ACCEPT && tid >= kThreads - 64) {
+        const int c = tid & 31, i = i0 + c;
+        int kind = 3;                          // accepted, rejected, unlikely
+        if (c < chains) {
+            double now = acc.post[i];
+            kind = 1;
+            if (!mask[i]) {
+                const double b = *acc.beta;
+                const double cp = cprior[i] + b * acc.cdata[i];
+                const u32x4 r = draw(seed, (uint32_t)(chain0 + i), 0u, STREAM_ACCEPT, step - 1, ep);
+                kind = log_exceeds(u01_open_closed(r.x, r.y), cp - now) ? 2 : 0;
+                if (kind == 0) {
+                    acc.prior[i] = cprior[i];
+                    acc.data[i] = acc.cdata[i];
+                    acc.post[i] = now = cp;
+                }
+            }
+            s_take[c] = kind == 0;
+            if (acc.floor) {
+                const u32x4 r = draw(seed, (uint32_t)(chain0 + i), 0u, STREAM_ACCEPT, step, ep);
+                s_floor[c] = now + log(u01_open_closed(r.x, r.y));
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const unsigned m = __ballot_sync(0xffffffffu, kind == k);
+            if (c == k && m) atomicAdd(&acc.counters[k], (unsigned long long)__popc(m));
+        }
     }
-    for (int t = tid; t < chains * pairs; t += kProposeThreads) {
+    for (int t = tid; t < chains * pairs; t += kThreads) {
         const int c = t / pairs, j = 2 * (t - c * pairs);
         double z0, z1;
         normal_pair(draw(seed, (uint32_t)(chain0 + i0 + c), (uint32_t)(j >> 1), STREAM_PROPOSAL, step, ep), z0, z1);
@@ -112,20 +171,26 @@ propose_kernel(const double* __restrict__ theta, int n, int p, const double* __r
         if (j + 1 < p) sz[c * p + j + 1] = z1;
     }
     __syncthreads();
-    const double* th = theta + (size_t)i0 * p;
-    for (int t = tid; t < chains * p; t += kProposeThreads) {
+    double* th = theta + (size_t)i0 * p;
+    double* cd = cand + (size_t)i0 * p;
+    for (int t = tid; t < chains * p; t += kThreads) {
         const int c = t / p, j = t - c * p;
         double d = 0.0;
         for (int k = 0; k <= j; ++k) d = fma(sL[j * p + k], sz[c * p + k], d);
+        if (ACCEPT && s_take[c]) th[t] = cd[t];
         const double v = th[t] + d;
         sv[t] = v;
         if (!(lo[j] <= v && v <= hi[j])) s_out[c] = 1;
     }
     __syncthreads();
-    for (int t = tid; t < chains * p; t += kProposeThreads) cand[(size_t)i0 * p + t] = s_out[t / p] ? th[t] : sv[t];
+    for (int t = tid; t < chains * p; t += kThreads) cd[t] = s_out[t / p] ? th[t] : sv[t];
     if (tid < chains) {
         mask[i0 + tid] = s_out[tid] ? CHAIN_OUT_OF_SUPPORT : 0u;
         cprior[i0 + tid] = s_prior;
+        if (ACCEPT && acc.floor) {
+            const double b = *acc.beta;
+            acc.floor[i0 + tid] = !s_out[tid] && b > 0.0 ? floor_of(s_floor[tid], s_prior, b) : -INFINITY;
+        }
     }
 }
 
@@ -175,16 +240,6 @@ propose_warp_kernel(const double* __restrict__ theta, int n, int p, const double
         mask[i] = out ? CHAIN_OUT_OF_SUPPORT : 0u;
         cprior[i] = s_prior;
     }
-}
-
-// log u > d for u in (0, 1]: decided in FP32 unless the two are closer than that logarithm's error
-// (u rounds to FP32 within 2^-24 of itself and logf is good to 2 ulp: below 1e-6 (1 + |log u|)).
-// The FP64 logarithm was a quarter of accept_kernel: 4,096 chains 7.7 -> 5.7 µs.
-__device__ inline bool log_exceeds(double u, double d) {
-    const float l = logf((float)u);
-    const double gap = (double)l - d;
-    if (fabs(gap) > 1e-5 * (1.0 + fabs((double)l))) return gap > 0.0;
-    return log(u) > d;
 }
 
 // ---------------------------------------------------------------------------
@@ -239,10 +294,7 @@ __global__ void accept_floor_kernel(int n, const double* __restrict__ beta, uint
     double f = -INFINITY;
     if (!mask[i] && b > 0.0) {
         u32x4 r = draw(seed, (uint32_t)(chain0 + i), 0u, STREAM_ACCEPT, step, *epoch);
-        const double u = u01_open_closed(r.x, r.y);
-        f = (post[i] + log(u) - cprior[i]) / b;
-        f -= (fabs(f) + 1.0) * 1e-9;
-        if (!(f == f)) f = -INFINITY;
+        f = floor_of(post[i] + log(u01_open_closed(r.x, r.y)), cprior[i], b);
     }
     floor[i] = f;
 }
@@ -1577,8 +1629,9 @@ extern "C" int ag_propose(const ag_stage_state* st, const double* theta, int32_t
                "invalid arguments (p must be in 1..%d)", kMaxPLarge);
     cudaStream_t s = as_stream(stream);
     if (p <= kMaxP) {
-        propose_kernel<<<blocks(n, kProposeChains), kProposeThreads, 0, s>>>(theta, n, p, st->chol, lo, hi, seed, step, st->epoch, cand,
-                                                       mask, cprior, st->chain0);
+        propose_kernel<false><<<blocks(n, kProposeChains), kProposeThreads<false>, 0, s>>>(
+            const_cast<double*>(theta), n, p, st->chol, lo, hi, seed, step, st->epoch, cand, mask, cprior, st->chain0,
+            AcceptArgs{});
         return launch_status("propose_kernel");
     }
     const size_t smem = (size_t)kProposeWarps * p * sizeof(double);
@@ -1616,6 +1669,26 @@ extern "C" int ag_accept_floor(const ag_stage_state* st, int32_t n, uint64_t see
     accept_floor_kernel<<<blocks(n, 256), 256, 0, as_stream(stream)>>>(n, st->beta, seed, step, st->epoch, mask,
                                                                         cprior, post, llk_floor, st->chain0);
     return launch_status("accept_floor_kernel");
+}
+
+extern "C" int ag_accept_propose(const ag_stage_state* st, int32_t n, int32_t p, const double* lo, const double* hi,
+                                 uint64_t seed, uint32_t step, uint32_t* mask, double* cand, double* cprior,
+                                 const double* cdata, double* theta, double* prior, double* data, double* post,
+                                 double* llk_floor, void* stream) {
+    int rc = check_state(st);
+    if (rc) return rc;
+    AG_REQUIRE(n > 0 && p > 0 && p <= kMaxPLarge && lo && hi && mask && cand && cprior && cdata && theta && prior &&
+                   data && post,
+               "invalid arguments (p must be in 1..%d)", kMaxPLarge);
+    if (p > kMaxP) {
+        rc = ag_accept(st, n, p, seed, step, mask, cand, cprior, cdata, theta, prior, data, post, stream);
+        if (!rc) rc = ag_propose(st, theta, n, p, lo, hi, seed, step + 1, cand, mask, cprior, stream);
+        return rc || !llk_floor ? rc : ag_accept_floor(st, n, seed, step + 1, mask, cprior, post, llk_floor, stream);
+    }
+    propose_kernel<true><<<blocks(n, kProposeChains), kProposeThreads<true>, 0, as_stream(stream)>>>(
+        theta, n, p, st->chol, lo, hi, seed, step + 1, st->epoch, cand, mask, cprior, st->chain0,
+        AcceptArgs{st->beta, cdata, prior, data, post, st->counters, llk_floor});
+    return launch_status("propose_kernel (accept)");
 }
 
 extern "C" int ag_posterior(const ag_stage_state* st, int32_t n, const double* prior,

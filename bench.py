@@ -987,9 +987,10 @@ def run_ours(args):
                             "value_full_evaluations": (world * N * S / t_full) if t_full else None,
                             "ms_per_step_full_evaluations": t_full * 1e3 if t_full else None},
         # per stage (one CUDA graph): COV median + cooperative COV schedule, Σ, Cholesky, CDF,
-        # counts, ranks, gather, adapt; per Metropolis step propose, acceptance floor, CDM set-up,
-        # CDM slots (not with few chains and the default variant), CDM likelihood, accept
-        "gpu_launches": (9 + (5 if n <= 3072 and model.variant == 0 else 6) * S) * args.steps,
+        # counts, ranks, gather, adapt; the first proposal and its acceptance floor; per Metropolis step
+        # CDM set-up, CDM slots (not with few chains and the default variant), CDM likelihood, and
+        # the accept with the next step's proposal and floor
+        "gpu_launches": ((11 if early_on else 10) + (3 if n <= 3072 and model.variant == 0 else 4) * S) * args.steps,
         "cpu_baseline": {"value": cpu_rate, "unit": "chain-steps/s", "cores": cores, "kind": "port",
                          "sample": f"{args.cpu_chains} chains x {X.size} stations, likelihood only, "
                                    f"{cpu_dt:.1f} s (FP64 C restatement of models/cdm/cdm/libcdm.py)"},

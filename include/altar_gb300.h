@@ -255,6 +255,16 @@ int ag_accept_floor(const ag_stage_state* st, int32_t n, uint64_t seed, uint32_t
                     void* stream);
 
 /*
+ * One launch between two steps' likelihoods: ag_accept of step `step`, ag_propose of step + 1 and,
+ * with llk_floor, ag_accept_floor of step + 1, with the same results as the calls in that order
+ * (more than 32 parameters: those calls).
+ */
+int ag_accept_propose(const ag_stage_state* st, int32_t n, int32_t p, const double* lo, const double* hi,
+                      uint64_t seed, uint32_t step, uint32_t* mask, double* cand, double* cprior,
+                      const double* cdata, double* theta, double* prior, double* data, double* post,
+                      double* llk_floor, void* stream);
+
+/*
  * Bytes of workspace ag_cov_schedule needs for n chains.
  */
 size_t ag_cov_workspace_bytes(int32_t n);
