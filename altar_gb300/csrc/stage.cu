@@ -6,6 +6,7 @@
 // schedule state instead of host round trips), so one annealing stage can be
 // captured into one CUDA graph.  All reductions run in a fixed order, so
 // repeated runs are bitwise identical.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -13,6 +14,8 @@
 
 #include "common.cuh"
 #include "internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace ag {
 
@@ -330,9 +333,14 @@ struct CovState {
 
 // blocks of the schedule kernel for n chains, and the partial sums one round of it writes
 constexpr int kCovBlocks = 152;
+// up to this many blocks form one cluster, whose barrier is hardware's; few chains are spread over it
+constexpr int kCovCluster = 8;
 __host__ __device__ constexpr int cov_blocks(int n) {
-    return (n + 255) / 256 < kCovBlocks ? (n + 255) / 256 : kCovBlocks;
+    return n <= 256 * kCovCluster ? (n <= 128 * kCovCluster ? (n + 127) / 128 : kCovCluster)
+           : (n + 255) / 256 < kCovBlocks ? (n + 255) / 256 : kCovBlocks;
 }
+// a block's share of the chains, whole warps of them
+__device__ __forceinline__ long cov_share(int n) { return ((n + gridDim.x - 1) / gridDim.x + 31) / 32 * 32; }
 __host__ __device__ constexpr size_t cov_round_partials(int n) {
     // a grid level's moments per block, or Brent's two points per chunk
     const size_t level = (size_t)2 * kGridPoints * cov_blocks(n), brent = 4 * (size_t)((n + kEvalChunk - 1) / kEvalChunk);
@@ -800,7 +808,8 @@ __device__ void level_moments(const double* __restrict__ llk, int n, double low,
     double m[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) m[k] = 0.0;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const long share = cov_share(n), end = min((long)n, (blockIdx.x + 1) * share);
+    for (long i = blockIdx.x * share + threadIdx.x; i < end; i += blockDim.x) {
         const double y = llk[i] - llk_max;
         double e = exp(low * y);
         const double f = POINTS > 1 ? exp(step * y) : 1.0;
@@ -833,14 +842,26 @@ __device__ void level_moments(const double* __restrict__ llk, int n, double low,
 // With few chains a round is a chain of dependent FP64 instructions (67 cycles each) and the
 // barrier; with many the exponentials add to that.  Measured:
 // 32,768 chains 110 µs (352 µs with eleven exponentials per chain and level and the eleven COVs
-// formed in a row), 1,024 chains 70 µs (177 µs).
-template <bool BRENT>
+// formed in a row), 1,024 chains 70 µs without a cluster (177 µs).
+// CLUSTER: the blocks are one cluster (up to 2,048 chains; Brent 4,096) and meet at its barrier, which
+// needs no cooperative launch and no words to clear: 1,024 chains 51 µs.  4,096 chains, 53 µs in 16
+// blocks, would have two per thread in a cluster of eight.
+template <bool BRENT, bool CLUSTER>
 __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restrict__ llk, int n, double target,
                                                            double tol, int maxiter, int rounds,
                                                            CovState* __restrict__ S, double* __restrict__ part,
                                                            GridBarrier* __restrict__ bar, double* __restrict__ beta,
                                                            double* __restrict__ dbeta_cov, double* __restrict__ w,
                                                            uint32_t* __restrict__ flags) {
+    if (CLUSTER) after_previous();
+    auto meet = [&]() {
+        if constexpr (CLUSTER) {
+            cg::this_cluster().sync();        // orders the global writes before it, cluster-wide
+            return true;
+        } else {
+            return grid_sync(bar, flags);
+        }
+    };
     __shared__ CovState sS;
     __shared__ double s_tot[2 * kGridPoints], s_limit[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -862,7 +883,7 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
                 level_moments<1>(llk, n, sS.high, 0.0, lmax, pr + blockIdx.x, parts);
             else
                 level_moments<kGridPoints>(llk, n, low, step, lmax, pr + blockIdx.x, parts);
-            if (!grid_sync(bar, flags)) return;
+            if (!meet()) return;
             // eight lanes per moment
             const int q = tid >> 3;
             double a = 0.0;
@@ -895,7 +916,7 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
                     pr[(size_t)(2 * pt + 1) * nblk + c] = m[1];
                 }
             }
-            if (!grid_sync(bar, flags)) return;
+            if (!meet()) return;
             if (tid < 2 * npts) {
                 double a = 0.0;
                 for (int k = 0; k < nblk; ++k) a += __ldcg(pr + (size_t)tid * nblk + k);
@@ -914,9 +935,9 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
     // the exponentials at the chosen δβ, their moments, then the state, β, and the normalised weights
     double* fp = part + 2 * pbuf;
     const double g = sS.dbeta, mx = g * (lmax - med);
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        w[i] = exp(g * (llk[i] - med) - mx);
-    if (!grid_sync(bar, flags)) return;
+    const long share = cov_share(n), begin = blockIdx.x * share + threadIdx.x, end = min((long)n, (blockIdx.x + 1) * share);
+    for (long i = begin; i < end; i += blockDim.x) w[i] = exp(g * (llk[i] - med) - mx);
+    if (!meet()) return;
     for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
         double m[2];
         chunk_sums(n, c, [&](int i) { return __ldcg(w + i); }, m);
@@ -925,7 +946,7 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
             fp[2 * c + 1] = m[1];
         }
     }
-    if (!grid_sync(bar, flags)) return;
+    if (!meet()) return;
     if (threadIdx.x < 2) {
         double a = 0.0;
         for (int k = 0; k < nblk; ++k) a += __ldcg(fp + 2 * k + threadIdx.x);
@@ -942,8 +963,7 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
         dbeta_cov[0] = sS.dbeta;
         dbeta_cov[1] = sS.cov;
     }
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        w[i] = w[i] / s1;
+    for (long i = begin; i < end; i += blockDim.x) w[i] = w[i] / s1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1725,7 +1745,7 @@ static int cov_coresident_blocks(int* out) {
     std::lock_guard<std::mutex> lock(mu);
     if (!cache[dev]) {
         int occ = 0, sms = 0;
-        rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cov_schedule_kernel<BRENT>, 256, 0),
+        rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cov_schedule_kernel<BRENT, false>, 256, 0),
                          "cudaOccupancyMaxActiveBlocksPerMultiprocessor(cov_schedule_kernel)");
         if (rc) return rc;
         rc = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
@@ -1747,28 +1767,43 @@ static int cov_schedule_launch(const ag_stage_state* st, const double* data_llk,
     CovState* S = reinterpret_cast<CovState*>(base);
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(base + cov_part_offset());
     double* part = reinterpret_cast<double*>(base + cov_part_offset() + sizeof(GridBarrier));
-    int grid = 0;
-    int rc = cov_coresident_blocks<BRENT>(&grid);
-    if (rc) return rc;
     // a grid level splits the chains over the GPU; Brent's one or two points have a chunk per block
     const int want = BRENT ? 2 * blocks(n, kEvalChunk) : cov_blocks(n);
-    if (grid > want) grid = want;
-    rc = cuda_status(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), s), "cudaMemsetAsync(COV barrier)");
-    if (rc) return rc;
+    const bool cluster = want <= kCovCluster;
+    int grid = want, rc = AG_OK;
+    if (!cluster) {
+        rc = cov_coresident_blocks<BRENT>(&grid);
+        if (rc) return rc;
+        if (grid > want) grid = want;
+        rc = cuda_status(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), s), "cudaMemsetAsync(COV barrier)");
+        if (rc) return rc;
+    }
     launch_after(cov_median_kernel, 1, 1024, 0, s, data_llk, n, st->beta, S);
     rc = launch_status("cov_median_kernel");
     if (rc) return rc;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
+    cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cfg.attrs = attr;
+    if (cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = grid;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+        return cuda_status(cudaLaunchKernelEx(&cfg, cov_schedule_kernel<BRENT, true>, data_llk, n, target, tol, maxiter,
+                                              rounds, S, part, bar, st->beta, st->dbeta_cov, st->w, st->dev_flags),
+                           "cov_schedule_kernel (cluster launch)");
+    }
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, cov_schedule_kernel<BRENT>, data_llk, n, target, tol, maxiter,
+    return cuda_status(cudaLaunchKernelEx(&cfg, cov_schedule_kernel<BRENT, false>, data_llk, n, target, tol, maxiter,
                                           rounds, S, part, bar, st->beta, st->dbeta_cov, st->w, st->dev_flags),
                        "cov_schedule_kernel (cooperative launch)");
 }

@@ -50,6 +50,25 @@ def test_grid_schedule_partitions(cuda, kind, n):
     np.testing.assert_allclose(st.w.cpu().numpy(), w_ref, rtol=1e-10, atol=1e-300)
 
 
+@pytest.mark.parametrize("kind", ["normal", "ties"])
+@pytest.mark.parametrize("n", [2, 128, 129, 897, 1024, 1025, 2048, 2049])
+def test_grid_schedule_in_a_cluster(cuda, kind, n):
+    """One to eight blocks of one cluster (128 chains per block, then 256), and the first size beyond;
+    the bounds of the test above, twice in the same workspace."""
+    llk = _llk(kind, n, np.random.default_rng(7 * n))
+    b_ref, db_ref, _, w_ref = catmip.dbeta_grid(llk, 0.0, 1.0, 0.01)
+    ws = workspace(_native.load().ag_cov_workspace_bytes(n))
+    dllk = dev(llk)
+    for _ in range(2):
+        st = StageState(n, 1)
+        _native.call("ag_cov_schedule", st.struct, ptr(dllk), n, 1.0, 0.01, ptr(ws), ws.numel(), stream_handle())
+        torch.cuda.synchronize()
+        b, db, _ = st.scalars.cpu().numpy()[:3]
+        assert abs(db - db_ref) <= 1e-12 * abs(db_ref) and abs(b - b_ref) <= 1e-12
+        np.testing.assert_allclose(st.w.cpu().numpy(), w_ref, rtol=1e-10, atol=1e-300)
+        assert int(st.flags.item()) == 0
+
+
 @pytest.mark.parametrize("p", [1, 2, 10, 21, 22, 33])
 @pytest.mark.parametrize("n", [1, 16, 17, 2433, 39000])
 def test_weighted_cov_partitions(cuda, p, n):
