@@ -165,17 +165,19 @@ AG_DEVICE_INLINE f32x2 add2(f32x2 a, f32x2 b) {
 }
 AG_DEVICE_INLINE f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pack2(-1.0f, -1.0f), a); }
 
-// (hi, lo) += w r² for two sums at once, as ff_add_wsq without the final renormalisation: hi takes
-// the rounded sums, lo everything they leave (|lo| stays a few units of hi's last place per term)
+// (hi, lo) += w r² for two sums at once, every operation rounded as in ff_add_wsq (a subtraction takes
+// the negative's place).  Without the last three operations lo would be a plain FP32 sum of what the
+// additions leave: after 4,000 terms the sums were off by 2e-13 for noise (7e-15 with them) and by 5e-9
+// for equal small terms behind a large one.
 AG_DEVICE_INLINE void ff2_add_wsq(f32x2& hi, f32x2& lo, f32x2 r, f32x2 w, f32x2 nw) {
     const f32x2 np = mul2(r, mul2(r, pack2(-1.0f, -1.0f)));      // -r²
     const f32x2 pe = fma2(r, r, np);
-    const f32x2 q = mul2(np, nw), nq = mul2(np, w);
+    const f32x2 nq = mul2(np, w);                                // -w r²
     const f32x2 qe = fma2(pe, w, fma2(np, nw, nq));
-    const f32x2 s = add2(hi, q), bb = sub2(s, hi);
-    const f32x2 e = add2(sub2(hi, sub2(s, bb)), sub2(q, bb));
-    lo = add2(lo, add2(e, qe));
-    hi = s;
+    const f32x2 s = sub2(hi, nq), bb = sub2(s, hi);
+    const f32x2 e = add2(sub2(sub2(hi, sub2(s, bb)), add2(nq, bb)), add2(lo, qe));
+    hi = add2(s, e);
+    lo = sub2(e, sub2(hi, s));
 }
 
 // warp sum of doubles (fixed butterfly order: deterministic)

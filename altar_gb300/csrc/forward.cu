@@ -623,13 +623,15 @@ cdm_llk_kernel(const ChainC* __restrict__ chains, const int32_t* __restrict__ sl
 // ---------------------------------------------------------------------------
 // Mogi: one thread per station, CH chains per CTA held in shared memory, two chains per packed
 // FP32 instruction (every element rounded as by the scalar one).  The FMA pipe bounds it: per pair
-// 15 operations per source, 16 for the residual and the float-float sum w r², and one reciprocal
+// 15 operations per source, 18 for the residual and the float-float sum w r², and one reciprocal
 // square root.  Beside the scalar instructions' issue slots, FP64 took a sixth of the former
-// kernel: 128 conversions and additions per warp at 64 cycles each to add the lanes' sums, which
-// are now added in float-float (48 bits, as the sums themselves) with each step halving the
-// chains a lane holds.  16,384 chains x 10,007 stations with offsets 326 -> 197 µs (217 with two
-// CTAs per SM instead of four), 1,024 x 1,024 20.5 -> 8.3 µs; two sources with residual rows, 16,384 x
-// 4,950, 264 -> 145 µs.
+// kernel: 128 conversions and additions per warp at 64 cycles each to add the lanes' sums.  These
+// are now added in three FP32 parts, which leave out less than FP64 does, each step halving the
+// chains a lane holds, and only the warps' sums in FP64.  16,384 chains x 10,007 stations
+// 334 -> 201 µs, 40,000 x 300 219 -> 50 µs, two sources with residual rows, 16,384 x 4,950, 303 -> 187 µs
+// (L2 cold; two float-float parts between the lanes took 193, 46 and 183 but lost up to 5 bits against
+// FP64; FP64 additions shared out over the lanes took 207, 107 and 191; two CTAs per SM instead of four
+// 10% longer).
 struct __align__(16) MogiPair {       // a source of two chains
     float4 x;      // x0 hi, hi, lo, lo
     float4 y;
@@ -638,29 +640,46 @@ struct __align__(16) MogiPair {       // a source of two chains
     float2 pad;
 };
 
-// sum over the warp of each of N (a power of two <= 32) float-float values per lane; on return v[0] of
-// lane l holds value l / (32 / N)
+// a sum in three FP32 parts, each below the last places of the one before: what an addition leaves out
+// is below 2^-60 of it (FP64 leaves 2^-53, at 64 cycles per warp instruction)
+struct fff { float hi, mid, lo; };
+AG_DEVICE_INLINE fff fff_sum(fff a, fff b) {
+    float s, e, t, f, u, g;
+    two_sum(a.hi, b.hi, s, e);
+    two_sum(a.mid, b.mid, t, f);
+    two_sum(e, t, u, g);
+    return fff{s, u, (a.lo + b.lo) + (f + g)};
+}
+
+// sum over the warp of each of N (a power of two from 4 to 32) float-float values per lane, the additions of
+// a butterfly shared out over the lanes; on return lane l holds value l / (32 / N)
 template <int N>
-__device__ __forceinline__ void warp_sum_ff(ff (&v)[N], int lane) {
-    int held = N;
+__device__ __forceinline__ fff warp_sum_ff(const ff (&v)[N], int lane) {
+    fff w[N / 2];
+    const bool top = lane & 16;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const bool up = lane & o;
-        if (held > 1) {
-            held >>= 1;
+    for (int i = 0; i < N / 2; ++i) {
+        const ff keep = top ? v[i + N / 2] : v[i], send = top ? v[i] : v[i + N / 2];
+        const float h = __shfl_xor_sync(0xffffffffu, send.hi, 16), l = __shfl_xor_sync(0xffffffffu, send.lo, 16);
+        w[i] = fff_sum(fff{keep.hi, keep.lo, 0.f}, fff{h, l, 0.f});
+    }
+    int held = N / 2;
 #pragma unroll
-            for (int i = 0; i < N / 2; ++i) {
-                if (i >= held) break;
-                const ff keep = up ? v[i + held] : v[i], send = up ? v[i] : v[i + held];
-                const float h = __shfl_xor_sync(0xffffffffu, send.hi, o), l = __shfl_xor_sync(0xffffffffu, send.lo, o);
-                v[i] = keep;
-                ff_add(v[i], h, l);
-            }
-        } else {
-            const float h = __shfl_xor_sync(0xffffffffu, v[0].hi, o), l = __shfl_xor_sync(0xffffffffu, v[0].lo, o);
-            ff_add(v[0], h, l);
+    for (int o = 8; o > 0; o >>= 1) {
+        const bool split = held > 1, up = split && (lane & o);
+        if (split) held >>= 1;
+#pragma unroll
+        for (int i = 0; i < N / 4; ++i) {
+            if (i >= held) break;
+            const fff keep = up ? w[i + held] : w[i], send = up || !split ? w[i] : w[i + held];
+            fff got;
+            got.hi = __shfl_xor_sync(0xffffffffu, send.hi, o);
+            got.mid = __shfl_xor_sync(0xffffffffu, send.mid, o);
+            got.lo = __shfl_xor_sync(0xffffffffu, send.lo, o);
+            w[i] = fff_sum(keep, got);
         }
     }
+    return w[0];
 }
 
 template <int CH, int NSRC>
@@ -677,7 +696,7 @@ mogi_llk_kernel(ag_layout L, const double* __restrict__ theta, int n,
     __shared__ int s_chain[CH];
     __shared__ float2 s_off[CP][kMaxOffsets];
     __shared__ int s_act[CH];
-    __shared__ float2 s_part[CH][8];
+    __shared__ fff s_part[CH][8];
     const int c0 = blockIdx.x * CH;
     const double PI = 3.14159265358979323846;
     const int nslots = index ? min(n, *count) : n;
@@ -758,20 +777,24 @@ mogi_llk_kernel(ag_layout L, const double* __restrict__ theta, int n,
         }
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // 1/32 of the lanes' sums, so that the warp's stays below FP32's largest value where they do
     ff v[CH];
+    const f32x2 part = pack2(0.03125f, 0.03125f);
 #pragma unroll
     for (int c = 0; c < CP; ++c) {
-        unpack2(hi[c], v[2 * c].hi, v[2 * c + 1].hi);
-        unpack2(lo[c], v[2 * c].lo, v[2 * c + 1].lo);
+        unpack2(mul2(hi[c], part), v[2 * c].hi, v[2 * c + 1].hi);
+        unpack2(mul2(lo[c], part), v[2 * c].lo, v[2 * c + 1].lo);
     }
-    warp_sum_ff(v, lane);
-    if (lane % (32 / CH) == 0) s_part[lane / (32 / CH)][warp] = make_float2(v[0].hi, v[0].lo);
+    const fff sum = warp_sum_ff(v, lane);
+    if (lane % (32 / CH) == 0) s_part[lane / (32 / CH)][warp] = sum;
     __syncthreads();
-    for (int c = threadIdx.x; c < CH; c += blockDim.x) {
-        if (!s_act[c]) continue;
-        ff t{0.f, 0.f};
-        for (int k = 0; k < 8; ++k) ff_add(t, s_part[c][k].x, s_part[c][k].y);
-        llk[s_chain[c]] = norm - 0.5 * ff_to_double(t);
+    // eight lanes per chain, in FP64 over the warps
+    if (threadIdx.x < 8 * CH) {
+        const int c = threadIdx.x >> 3;
+        const fff q = s_part[c][threadIdx.x & 7];
+        double s = (double)q.hi + ((double)q.mid + (double)q.lo);
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 7) == 0 && s_act[c]) llk[s_chain[c]] = norm - 0.5 * (32.0 * s);
     }
 }
 
