@@ -1040,7 +1040,18 @@ surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float*
             const float2 p = s_part[g * kSurChains + c];
             ff_add(t, p.x, p.y);
         }
-        llk[i0 + c] = norm - 0.5 * (q0 + ff_to_double(t));
+        double acc = ff_to_double(t);
+        if (!isfinite(acc)) {
+            // a product or the sum left FP32's range (a NaN would be accepted as a sample): in FP64
+            acc = 0.0;
+            for (int a = 0; a < k; ++a) {
+                float z = 0.f;
+                for (int b = 0; b < k; ++b) z = fmaf(sGT[b * rows + a], sc[b * kSurStride + c], z);
+                const double ca = (double)sc[a * kSurStride + c];
+                acc += ca * (double)z - 2.0 * (double)h[a] * ca;
+            }
+        }
+        llk[i0 + c] = norm - 0.5 * (q0 + acc);
     }
 }
 
