@@ -940,36 +940,43 @@ __global__ void to_bf16_kernel(long count, const float* __restrict__ p, __nv_bfl
     if (e < count) q[e] = __float2bfloat16_rn(p[e]);
 }
 
-// llk_s = norm - ½ (q0 - 2 hᵀ c̃ + c̃ᵀ G c̃), c̃ = scale ⊙ c.  A CTA takes kSurChains chains; a thread forms
-// kSurRows rows of G c̃ for eight chains, so that four 16-byte shared-memory loads feed 64 FMAs
+// llk_s = norm - ½ (q0 - 2 hᵀ c̃ + c̃ᵀ G c̃), c̃ = scale ⊙ c.  A CTA takes 16 PER chains; a thread
+// forms kSurRows rows of G c̃ for PER chains, eight of them so that four 16-byte shared-memory loads feed 64 FMAs
 // (shared-memory wavefronts bound it otherwise: with eight FMAs per three loads 34 µs for 32,768
 // chains and 64 coefficients).  Its FP32 terms are added exactly in float-float and the threads
 // of a chain in order (FP64 products and sums in a warp per chain took 61 µs at the FP64
 // pipe's rate).  Measured: 24 µs; staging the operands by 4-byte loads, 58 µs.
 constexpr int kSurMaxK = 96;
-constexpr int kSurChains = 128;
-constexpr int kSurStride = kSurChains + 4;   // row of c̃: 16-byte aligned, spread over the banks
+constexpr int kSurLanes = 16;                // threads over the chains of a CTA
+__host__ __device__ constexpr int sur_stride(int chains) { return chains + 4; }   // row of c̃: 16-byte aligned, spread over the banks
 constexpr int kSurRows = 8;
+// chains per SM up to which a thread takes two of them (a fourth of the work in the chain of FMAs, four
+// times the CTAs): 1,000 x 64 7.4 µs against 13.4 with eight (10.4 with a warp per chain), 9,728 x 8
+// 7.0 against 10.4 (12.4), 9,728 x 64 8.8 against 13.9, 9,728 x 96 15.8 against 20.5; but 12,000 x 96
+// 28.2 against 21.2
+constexpr int kSurFew = 64;
 static int sur_groups(int k) { return (k + kSurRows - 1) / kSurRows; }
-static size_t sur_smem(int k) {
-    return ((size_t)k * kSurRows * sur_groups(k) + (size_t)k * kSurStride + 2 * (size_t)sur_groups(k) * kSurChains) *
+static size_t sur_smem(int k, int chains) {
+    return ((size_t)k * kSurRows * sur_groups(k) + (size_t)k * sur_stride(chains) + 2 * (size_t)sur_groups(k) * chains) *
            sizeof(float);
 }
 
-__global__ void __launch_bounds__(kSurChains / 8 * (kSurMaxK / kSurRows))
+template <int PER>
+__global__ void __launch_bounds__(kSurLanes * (kSurMaxK / kSurRows))
 surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float* __restrict__ scale,
                      const float* __restrict__ G, const float* __restrict__ h, double q0, double norm,
                      double* __restrict__ llk) {
     after_previous();
     extern __shared__ __align__(16) float s_mem[];
+    constexpr int kChains = kSurLanes * PER, kStride = sur_stride(kChains);
     const int groups = (k + kSurRows - 1) / kSurRows, rows = groups * kSurRows;
     float* sGT = s_mem;                                  // [k][rows], sGT[b][a] = G[a][b]
-    float* sc = sGT + k * rows;                          // [k][kSurStride]
-    float2* s_part = reinterpret_cast<float2*>(sc + k * kSurStride);     // [groups][kSurChains]
-    const int tid = threadIdx.x, threads = kSurChains / 8 * groups;
-    const int c0 = tid % (kSurChains / 8) * 8, a0 = tid / (kSurChains / 8) * kSurRows;
-    const long i0 = (long)blockIdx.x * kSurChains;
-    const int chains = n - i0 < kSurChains ? (int)(n - i0) : kSurChains;
+    float* sc = sGT + k * rows;                          // [k][kStride]
+    float2* s_part = reinterpret_cast<float2*>(sc + k * kStride);     // [groups][kChains]
+    const int tid = threadIdx.x, threads = kSurLanes * groups;
+    const int c0 = tid % kSurLanes * PER, a0 = tid / kSurLanes * kSurRows;
+    const long i0 = (long)blockIdx.x * kChains;
+    const int chains = n - i0 < kChains ? (int)(n - i0) : kChains;
     // staged by 16-byte loads, eight in flight per thread, where the rows allow
     if (k % 4 == 0 && ((size_t)G | (size_t)coeff | (size_t)scale) % 16 == 0) {
         const int kq = k / 4;
@@ -985,8 +992,8 @@ surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float*
             const int q = e / kq, b = 4 * (e - q * kq);
             const float4 v = __ldg(reinterpret_cast<const float4*>(coeff + i0 * k) + e);
             const float4 f = __ldg(reinterpret_cast<const float4*>(scale + b));
-            float* to = sc + b * kSurStride + q;
-            to[0] = v.x * f.x; to[kSurStride] = v.y * f.y; to[2 * kSurStride] = v.z * f.z; to[3 * kSurStride] = v.w * f.w;
+            float* to = sc + b * kStride + q;
+            to[0] = v.x * f.x; to[kStride] = v.y * f.y; to[2 * kStride] = v.z * f.z; to[3 * kStride] = v.w * f.w;
         }
     } else {
         for (int e = tid; e < k * k; e += threads) {
@@ -995,35 +1002,39 @@ surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float*
         }
         for (int e = tid; e < chains * k; e += threads) {
             const int q = e / k, b = e - q * k;
-            sc[b * kSurStride + q] = __ldg(coeff + i0 * k + e) * __ldg(scale + b);
+            sc[b * kStride + q] = __ldg(coeff + i0 * k + e) * __ldg(scale + b);
         }
     }
     // rows past k and chains past n: zeros
     for (int e = tid; e < (rows - k) * k; e += threads) sGT[e / (rows - k) * rows + k + e % (rows - k)] = 0.f;
-    for (int e = tid; e < (kSurChains - chains) * k; e += threads)
-        sc[e % k * kSurStride + chains + e / k] = 0.f;
+    for (int e = tid; e < (kChains - chains) * k; e += threads)
+        sc[e % k * kStride + chains + e / k] = 0.f;
     __syncthreads();
-    float row[kSurRows][8] = {};
+    float row[kSurRows][PER] = {};
 #pragma unroll 2
     for (int b = 0; b < k; ++b) {
-        float g[kSurRows], v[8];
+        float g[kSurRows], v[PER];
         *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(sGT + b * rows + a0);
         *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(sGT + b * rows + a0 + 4);
-        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(sc + b * kSurStride + c0);
-        *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(sc + b * kSurStride + c0 + 4);
+        if constexpr (PER == 8) {
+            *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(sc + b * kStride + c0);
+            *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(sc + b * kStride + c0 + 4);
+        } else {
+            *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(sc + b * kStride + c0);
+        }
 #pragma unroll
         for (int q = 0; q < kSurRows; ++q)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) row[q][c] = fmaf(g[q], v[c], row[q][c]);
+            for (int c = 0; c < PER; ++c) row[q][c] = fmaf(g[q], v[c], row[q][c]);
     }
-    ff acc[8] = {};
+    ff acc[PER] = {};
 #pragma unroll
     for (int q = 0; q < kSurRows; ++q) {
         if (a0 + q < k) {
             const float h2 = -2.0f * __ldg(h + a0 + q);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float ca = sc[(a0 + q) * kSurStride + c0 + c];
+            for (int c = 0; c < PER; ++c) {
+                const float ca = sc[(a0 + q) * kStride + c0 + c];
                 float t = ca * row[q][c];
                 ff_add(acc[c], t, fmaf(ca, row[q][c], -t));
                 t = h2 * ca;
@@ -1032,12 +1043,12 @@ surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float*
         }
     }
 #pragma unroll
-    for (int c = 0; c < 8; ++c) s_part[a0 / kSurRows * kSurChains + c0 + c] = make_float2(acc[c].hi, acc[c].lo);
+    for (int c = 0; c < PER; ++c) s_part[a0 / kSurRows * kChains + c0 + c] = make_float2(acc[c].hi, acc[c].lo);
     __syncthreads();
     for (int c = tid; c < chains; c += threads) {
         ff t{0.f, 0.f};
         for (int g = 0; g < groups; ++g) {
-            const float2 p = s_part[g * kSurChains + c];
+            const float2 p = s_part[g * kChains + c];
             ff_add(t, p.x, p.y);
         }
         double acc = ff_to_double(t);
@@ -1046,8 +1057,8 @@ surrogate_llk_kernel(int n, int k, const float* __restrict__ coeff, const float*
             acc = 0.0;
             for (int a = 0; a < k; ++a) {
                 float z = 0.f;
-                for (int b = 0; b < k; ++b) z = fmaf(sGT[b * rows + a], sc[b * kSurStride + c], z);
-                const double ca = (double)sc[a * kSurStride + c];
+                for (int b = 0; b < k; ++b) z = fmaf(sGT[b * rows + a], sc[b * kStride + c], z);
+                const double ca = (double)sc[a * kStride + c];
                 acc += ca * (double)z - 2.0 * (double)h[a] * ca;
             }
         }
@@ -1514,15 +1525,20 @@ extern "C" int ag_surrogate_llk(int32_t n, int32_t k, const float* coeff, const 
                                 void* stream) {
     AG_REQUIRE(n > 0 && k > 0 && coeff && scale && gram && h && llk, "invalid arguments");
     AG_REQUIRE(k <= kSurMaxK, "at most %d surrogate coefficients are supported (got %d)", kSurMaxK, k);
-    const size_t smem = sur_smem(k);
+    int sms = 0;
+    int rc = sm_count(&sms);
+    if (rc) return rc;
+    const bool few = n <= kSurFew * sms;
+    const int chains = kSurLanes * (few ? 2 : 8);
+    const auto kernel = few ? surrogate_llk_kernel<2> : surrogate_llk_kernel<8>;
+    const size_t smem = sur_smem(k, chains);
     if (smem > 48 * 1024) {
-        int rc = cuda_status(cudaFuncSetAttribute(surrogate_llk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)smem),
-                             "cudaFuncSetAttribute(surrogate_llk_kernel)");
+        rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                         "cudaFuncSetAttribute(surrogate_llk_kernel)");
         if (rc) return rc;
     }
-    launch_after(surrogate_llk_kernel, nblk(n, kSurChains), kSurChains / 8 * sur_groups(k), smem, as_stream(stream),
-                 n, k, coeff, scale, gram, h, q0, norm, llk);
+    launch_after(kernel, nblk(n, chains), kSurLanes * sur_groups(k), smem, as_stream(stream), n, k, coeff, scale, gram,
+                 h, q0, norm, llk);
     return launch_status("surrogate_llk_kernel");
 }
 
