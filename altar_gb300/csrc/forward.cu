@@ -833,8 +833,9 @@ static int station_splits(int n, int ntiles) {
 }
 
 // CDM workspace: chain constants, the row of each slot, the set-up header (slot count and cost
-// histogram), each requested chain's cost bucket; for up to kSplitChains chains also the finished
-// CTAs and the partial misfits of each slot
+// histogram), each requested chain's cost bucket; the finished CTAs and the partial misfits of each
+// slot of a split launch, which has up to kSplitChains: a population of more takes as much, so that
+// its workspace serves every smaller call
 struct CdmWorkspace {
     ChainC* chains;
     int32_t* slot_row;
@@ -851,7 +852,7 @@ static size_t cdm_workspace(char* base, int n, CdmWorkspace* w) {
         at += al256(bytes);
         return p;
     };
-    const size_t split = n <= kSplitChains ? n : 0;
+    const size_t split = n <= kSplitChains ? n : kSplitChains;
     CdmWorkspace ws;
     ws.chains = reinterpret_cast<ChainC*>(take((size_t)n * sizeof(ChainC)));
     ws.slot_row = reinterpret_cast<int32_t*>(take((size_t)n * sizeof(int32_t)));

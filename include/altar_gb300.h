@@ -115,7 +115,8 @@ int ag_last_error(char* buf, size_t len);
 const char* ag_version(void);
 
 /*
- * Bytes of caller-provided device workspace the forward model needs for n chains.
+ * Bytes of caller-provided device workspace the forward model needs for n chains, never fewer for
+ * more: a workspace made for the largest call serves the smaller ones.
  */
 size_t ag_forward_workspace_bytes(int model, int32_t n);
 
