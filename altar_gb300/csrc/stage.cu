@@ -978,7 +978,8 @@ __global__ void __launch_bounds__(256) cov_schedule_kernel(const double* __restr
 // term); 4 parameters, 1,024 chains 8 µs (43 µs).
 constexpr size_t kSigmaSmem = 160 * 1024;
 constexpr int kSigmaBlocks = 152;  // one per SM
-constexpr int kSigmaMinRows = 16;
+constexpr int kSigmaMinRows = 16;      // of a chunk (kSigmaSmem holds as many at kMaxPLarge)
+static_assert(kSigmaMinRows * 2 * (kMaxPLarge + 1) * sizeof(double) <= kSigmaSmem, "the workspace counts on it");
 static void sigma_grid(int n, int p, int* chunk, int* nblk, int* cpb) {
     int most = (int)(kSigmaSmem / (2 * (p + 1) * sizeof(double)));
     if (most > kSigmaChunk) most = kSigmaChunk;
@@ -1894,10 +1895,10 @@ extern "C" int ag_cov_schedule_brent(const ag_stage_state* st, const double* dat
 
 extern "C" size_t ag_sigma_workspace_bytes(int32_t n, int32_t p) {
     if (n <= 0 || p <= 0 || p > kMaxPLarge) return 0;
-    int chunk, nblk, cpb;
-    sigma_grid(n, p, &chunk, &nblk, &cpb);
+    // the most blocks that any smaller number of chains takes, so that more chains never need less
+    const size_t rows = ((size_t)n - 1) / kSigmaMinRows + 1, nblk = rows < kSigmaBlocks ? rows : kSigmaBlocks;
     const size_t nent = 1 + p + (size_t)p * (p + 1) / 2;
-    return ((size_t)nblk + 1) * nent * sizeof(double) + 256;    // partials, totals, the block count
+    return (nblk + 1) * nent * sizeof(double) + 256;    // partials, totals, the block count
 }
 
 extern "C" int ag_weighted_cov(const ag_stage_state* st, const double* theta, int32_t n, int32_t p,

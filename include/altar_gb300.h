@@ -316,7 +316,7 @@ int ag_cov_schedule_noalloc(const ag_stage_state* st, const double* data_llk, in
                             double target, double tol, void* stream);
 int32_t ag_cov_schedule_noalloc_max_chains(void);
 
-/* Bytes of workspace ag_weighted_cov needs. */
+/* Bytes of workspace ag_weighted_cov needs, never fewer for more chains. */
 size_t ag_sigma_workspace_bytes(int32_t n, int32_t p);
 
 /*

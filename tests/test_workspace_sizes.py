@@ -22,6 +22,11 @@ def test_forward(native_lib, model):
     _never_falls(lambda n: native_lib.ag_forward_workspace_bytes(model, n))
 
 
+@pytest.mark.parametrize("p", [1, 4, 10, 21, 22, 100, 512])
+def test_covariance(native_lib, p):
+    _never_falls(lambda n: native_lib.ag_sigma_workspace_bytes(n, p))
+
+
 def test_stage(native_lib):
     _never_falls(native_lib.ag_cov_workspace_bytes)
     _never_falls(native_lib.ag_resample_workspace_bytes)
