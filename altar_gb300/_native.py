@@ -144,6 +144,7 @@ _SIGNATURES = {
     "ag_linear_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32]),
     "ag_linear_llk": (c_int, [P, P, c_int32, c_double, P, P, c_size_t, P, P]),
     "ag_linear_llk_fp64": (c_int, [P, P, c_int32, c_double, P, P]),
+    "ag_whiten_prepare_lower": (c_int, [P, c_int32, P, P]),
     "ag_whiten_workspace_bytes": (c_size_t, [c_int32, c_int32]),
     "ag_whiten_llk": (c_int, [P, P, c_int32, c_int32, P, P, c_size_t, P, P]),
     "ag_whiten_llk_lower": (c_int, [P, P, c_int32, c_int32, P, P, c_size_t, P, P]),

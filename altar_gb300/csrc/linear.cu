@@ -406,13 +406,13 @@ __global__ void __launch_bounds__(256) split_rho0_kernel(const T* __restrict__ x
     }
 }
 
-// A split as [hi | hi | lo]
-__global__ void split_a_kernel(const double* __restrict__ A, int m, int p, int kp,
+// A split as [hi | hi | lo]; lower: its entries above the diagonal as zeros, whatever they hold
+__global__ void split_a_kernel(const double* __restrict__ A, int m, int p, int kp, bool lower,
                                __nv_bfloat16* __restrict__ out) {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long)m * kp) return;
     const int i = (int)(e / kp), j = (int)(e % kp);
-    const float a = (j < p) ? (float)A[(size_t)i * p + j] : 0.f;
+    const float a = (j < p && !(lower && j > i)) ? (float)A[(size_t)i * p + j] : 0.f;
     const __nv_bfloat16 hi = __float2bfloat16_rn(a);
     const __nv_bfloat16 lo = __float2bfloat16_rn(a - __bfloat162float(hi));
     __nv_bfloat16* row = out + (size_t)i * 3 * kp;
@@ -559,12 +559,20 @@ static inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
 extern "C" int32_t ag_linear_kpad(int32_t p) { return p > 0 ? cdiv(p, TC_BK) * TC_BK : 0; }
 
-extern "C" int ag_linear_prepare(const double* A, int32_t m, int32_t p, uint16_t* a_split, void* stream) {
+static int split_a(const double* A, int m, int p, bool lower, uint16_t* a_split, void* stream) {
     AG_REQUIRE(A && a_split && m > 0 && p > 0, "invalid arguments");
     const int kp = ag_linear_kpad(p);
-    split_a_kernel<<<cdiv((long)m * kp, 256), 256, 0, as_stream(stream)>>>(A, m, p, kp,
+    split_a_kernel<<<cdiv((long)m * kp, 256), 256, 0, as_stream(stream)>>>(A, m, p, kp, lower,
                                                                          reinterpret_cast<__nv_bfloat16*>(a_split));
     return launch_status("split_a_kernel");
+}
+
+extern "C" int ag_linear_prepare(const double* A, int32_t m, int32_t p, uint16_t* a_split, void* stream) {
+    return split_a(A, m, p, false, a_split, stream);
+}
+
+extern "C" int ag_whiten_prepare_lower(const double* W, int32_t m, uint16_t* w_split, void* stream) {
+    return split_a(W, m, m, true, w_split, stream);
 }
 
 // workspace of an evaluation: centre [kp], FP64 and as two FP32 parts | ρ₀ [m] | split rows

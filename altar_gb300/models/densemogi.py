@@ -66,7 +66,7 @@ class DenseMogi(Bayesian):
             kp = lib.ag_linear_kpad(m)
             wsplit = torch.empty(m * 3 * kp, dtype=torch.int16, device=DEVICE)
             W = W.contiguous()
-            _native.call("ag_linear_prepare", ptr(W), m, m, ptr(wsplit), stream_handle())
+            _native.call("ag_whiten_prepare_lower", ptr(W), m, ptr(wsplit), stream_handle())
             self._w.append((W, wsplit))
             self.blocks.append(_native.WhitenBlock(W.data_ptr(), wsplit.data_ptr(), col, m))
             col += m

@@ -57,7 +57,7 @@ class CUDA:
                                           upper=False).contiguous()
         kp = _native.load().ag_linear_kpad(m)
         wsplit = torch.empty(m * 3 * kp, dtype=torch.int16, device=DEVICE)
-        _native.call("ag_linear_prepare", ptr(W), m, m, ptr(wsplit), stream_handle())
+        _native.call("ag_whiten_prepare_lower", ptr(W), m, ptr(wsplit), stream_handle())
         self._whiten = (W, wsplit, _native.WhitenBlock(W.data_ptr(), wsplit.data_ptr(), 0, m))
         self._flags = torch.zeros(1, dtype=torch.int32, device=DEVICE)
 

@@ -402,7 +402,8 @@ int ag_linear_llk_fp64(const ag_linear_model* model, const double* theta, int32_
  */
 typedef struct ag_whiten_block {
     const double* w64;        /* [m][m] FP64 W = L⁻¹ */
-    const uint16_t* w_split;  /* [m][3 kpad(m)] BF16 [W_hi | W_hi | W_lo] (ag_linear_prepare) */
+    const uint16_t* w_split;  /* [m][3 kpad(m)] BF16 [W_hi | W_hi | W_lo] (ag_linear_prepare, or
+                                 ag_whiten_prepare_lower for ag_whiten_llk_lower) */
     int32_t col0;             /* first column of the block in the residual rows */
     int32_t m;                /* observations in the block */
 } ag_whiten_block;
@@ -411,8 +412,13 @@ size_t ag_whiten_workspace_bytes(int32_t m, int32_t n);
 /* resid: n rows of ldr FP32 residuals (ag_forward_llk's residual output) */
 int ag_whiten_llk(const ag_whiten_block* block, const float* resid, int32_t ldr, int32_t n, double* llk,
                   void* workspace, size_t workspace_bytes, uint32_t* flags, void* stream);
-/* the same for a lower triangular W (zeros above the diagonal, as L⁻¹ has): the products with those
- * zeros are left out; W's entries above the diagonal are taken as zeros */
+/* build the split BF16 operand of a lower triangular W (m x 3 kpad(m)): as ag_linear_prepare does, with
+ * zeros in place of W's entries above the diagonal, which may hold anything */
+int ag_whiten_prepare_lower(const double* W, int32_t m, uint16_t* w_split, void* stream);
+/* the same for a lower triangular W (as L⁻¹ is): the products with the zeros above its diagonal are left
+ * out.  w_split from ag_whiten_prepare_lower, so that W's entries above the diagonal count as zeros
+ * (w64's are not read); one from ag_linear_prepare serves only if those entries are zeros: 256 columns
+ * of w_split are multiplied at a time, also where the diagonal runs through them. */
 int ag_whiten_llk_lower(const ag_whiten_block* block, const float* resid, int32_t ldr, int32_t n, double* llk,
                         void* workspace, size_t workspace_bytes, uint32_t* flags, void* stream);
 
