@@ -4,7 +4,7 @@ Each forward model exposes a few launch variants (chains per CTA and the
 register budget that sets how many CTAs share an SM, ``ag_forward_variants``).
 ``tune`` times every variant on a sample of the actual problem with CUDA events
 and keeps the fastest; results are cached as JSON keyed by
-(model, observations, chains, GPU name) so later runs skip the trials.
+(model, observations, chains, launch table, GPU name) so later runs skip the trials.
 The cache path is ``$ALTAR_GB300_TUNE_CACHE`` or ``~/.cache/altar_gb300/autotune.json``.
 """
 import json
@@ -13,6 +13,10 @@ import os
 import torch
 
 from . import _native
+
+# what the variants' numbers stand for: raised whenever a variant's launch or kernel changes, so that an
+# entry timed under other ones is not taken (2: packed CDM and Mogi kernels, variant 0 by the number of chains)
+LAUNCH_TABLE = 2
 
 
 def cache_path():
@@ -41,7 +45,7 @@ def _save(table):
 
 
 def key(kind, m, n, nvar):
-    return f"model={kind} m={m} n={n} variants={nvar} gpu={torch.cuda.get_device_name()}"
+    return f"model={kind} m={m} n={n} variants={nvar} table={LAUNCH_TABLE} gpu={torch.cuda.get_device_name()}"
 
 
 def tune(strategy, theta, reps=3, sample=8192, use_cache=True):
