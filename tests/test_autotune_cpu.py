@@ -1,4 +1,5 @@
-"""The autotuner's cache: entries timed under another launch table are not taken (CPU, no kernels)."""
+"""The autotuner's choice and its cache (CPU, no kernels): entries timed under another launch table are
+not taken, and the default is not given up to noise."""
 import json
 import types
 
@@ -60,3 +61,15 @@ def test_entry_of_another_launch_table_is_ignored(monkeypatch, tmp_path):
     # and no longer once the table changes
     monkeypatch.setattr(autotune, "LAUNCH_TABLE", autotune.LAUNCH_TABLE + 1)
     assert autotune.tune(again, theta)["variant"] == 2 and again.calls > 0
+
+
+def test_default_is_kept_against_noise(monkeypatch, tmp_path):
+    """Two variants that are one kernel (14.374 and 14.368 ms, measured): the choice is not their noise."""
+    monkeypatch.setenv("ALTAR_GB300_TUNE_CACHE", str(tmp_path / "autotune.json"))
+    clock = [0.0]
+    _fake_gpu(monkeypatch, clock)
+    theta = torch.zeros(10, 4, dtype=torch.float64)
+    for times, want in (([14.374, 15.0, 14.368], 0), ([14.368, 15.0, 14.374], 0), ([14.4, 14.0, 14.2], 1)):
+        strategy = _Strategy(clock, times)
+        assert autotune.tune(strategy, theta, use_cache=False)["variant"] == want
+        assert strategy.layout.variant == want
