@@ -37,10 +37,11 @@ constexpr int kRevTile = 128;          // observation points per pass
 enum : int { R_POW, R_IPRE, R_A, R_C1, R_CD, R_HS, R_HD, R_KS, R_KD, R_COUNT };
 
 // k R^-5 (or k R^-3) from R².  With i ≈ 1/R and i² rounded, 1 - R² i² (one FMA, exact to its own
-// rounding) is the relative error of i², and so, times 5/2 (3/2), that of the power.
+// rounding) is the relative error of i², and so, times 5/2 (3/2), that of the power.  An infinite R² (a
+// squared distance or depth beyond FP64) gives 0 as the division does, not 0 times that error's NaN.
 __device__ __forceinline__ double inverse_power(double k, double R2, bool cube) {
     const double i = rsqrt(R2), i2 = i * i;
-    const double err = fma(-R2, i2, 1.0);
+    const double err = __double2hiint(R2) >= 0x7ff00000 ? 0.0 : fma(-R2, i2, 1.0);
     const double p = k * (cube ? i2 * i : i2 * i2 * i);
     return fma(p, (cube ? 1.5 : 2.5) * err, p);
 }
