@@ -188,7 +188,6 @@ AG_DEVICE_INLINE double warp_sum(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// bounded mbarrier helpers (shared::cta)
 // First statement of a kernel that launch_after() starts: waits for the kernel before it on the
 // stream to end, its writes visible, then lets the next one's CTAs come in as this one's leave.
 AG_DEVICE_INLINE void after_previous() {
@@ -219,6 +218,7 @@ template <int B> AG_DEVICE_INLINE void cp_async_or_zero(void* dst, const void* s
 AG_DEVICE_INLINE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> AG_DEVICE_INLINE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// bounded mbarrier helpers (shared::cta)
 AG_DEVICE_INLINE void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count));
 }

@@ -18,7 +18,6 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<size_t>(p) % a) == 0; }
 
-// checks a kernel launch and returns the ABI status
 // Launch behind the kernel before it on the stream without waiting for that one's last CTA to leave
 // first (programmatic dependent launch).  The kernel's first statement is after_previous(), so it
 // touches memory only when its predecessor has ended; what it saves is the gap, ~2 µs per launch of
@@ -26,6 +25,8 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<size_t>(
 // prediction (8) 158 -> 141, a stage's schedule, covariance and resampling (8) 275 -> 261, training
 // (8 per batch) 769 -> 753.  Not for the walk's propose, forward and accept kernels: a short run that
 // captures and replays 61 of them per stage took 5.4 ms instead of 4.6.
+// One kernel reads before its wait: mlp_layer_tc_kernel its packed weights.  What writes them has to end two
+// launches back or more, with a kernel in between that waits (split_rows_kernel, in ag_mlp_forward_tc).
 template <class... P, class... A>
 inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchAttribute attr[1];
@@ -40,6 +41,7 @@ inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);   // launch_status() reports its error
 }
+// checks a kernel launch and returns the ABI status
 inline int launch_status(const char* name) { return cuda_status(cudaGetLastError(), name); }
 
 }  // namespace ag

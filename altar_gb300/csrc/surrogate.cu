@@ -667,7 +667,8 @@ mlp_layer_tc_kernel(const __grid_constant__ CUtensorMap map_x,   // n  x K' spli
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     auto aborted = [&]() { return *(volatile int*)&s_abort != 0; };
-    // the weights were packed at least two kernels ago (the rows are split in between)
+    // the weights were packed at least two launches back (the rows are split in between), so they may be
+    // read before the wait
     if (held && threadIdx.x == 0) {
         mbar_arrive_expect_tx(wfull, kblocks / 2 * kMlpW);
         for (int kb = 0; kb < kblocks / 2; ++kb)
@@ -1393,6 +1394,8 @@ extern "C" int ag_mlp_forward_tc(const ag_mlp* net, const float* params, const u
     __nv_bfloat16* buf[2] = {reinterpret_cast<__nv_bfloat16*>(workspace),
                              reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(workspace) + need / 2)};
     const int fi0 = net->sizes[0], kp0 = mlp_kp(fi0);
+    // also what keeps the first layer's early read of wpack behind the packing: it may start once this kernel,
+    // which waits for everything before it, has
     launch_after(split_rows_kernel, nblk((long)n * (kp0 / 8), 256), 256, 0, s, x, n, fi0, kp0, buf[0]);
     rc = launch_status("split_rows_kernel");
     if (rc) return rc;
