@@ -936,9 +936,9 @@ AG_DEVICE_INLINE void rect_quad(const RectQ& Q, const float4* node, int nn, V Xr
 // scalar nodes (79% of slots with the FMA pipe at 65%).  Every element goes through the same
 // operations with the same rounding as in rect_quad: a subtraction is an addition of the
 // negative, which the nodes carry, and the products with -1/(R + d) give -s, -B and -I5, whose
-// signs meet those of W.  32,768 chains x 40,000 stations: 60.2 -> 54.5 ms (one node at a time
-// 56.1, three 56.3, four 57.9; two stations per lane with more warps 59 to 64); issue 58%, FMA pipe
-// 70% busy, now throttled by the pipe's two-cycle instructions.
+// signs meet those of W.  32,768 chains x 40,000 stations: 58.8 -> 54.8 ms (one node at a time
+// 56.1, three 56.3, four 57.9; two stations per lane with more warps 59 to 64); 58% of the issue slots, FMA
+// pipe 68 to 70% busy, now throttled by the pipe's two-cycle instructions.
 struct PackedNode {
     float4 xy;    // -x, -x, -y, -y
     float4 dw;    // d, d, w, w

@@ -609,7 +609,7 @@ def run_dense(args):
         ref -= 0.5 * (z * z).sum(1)
     torch.cuda.synchronize()
     whiten_err = float(((out[sub] - ref).abs() / ref.abs()).max().item())
-    whiten = sum(2.0 * m * m * N for m in sizes)                 # W (r - r̄) per dataset block
+    whiten = sum(float(m) * (m + 1) * N for m in sizes)          # W (r - r̄) per dataset block, W triangular
     pk = peaks()
     peak = float(pk.get("bf16_tflops", 1900.0))
     if rank == 0:
@@ -623,7 +623,7 @@ def run_dense(args):
                        "setup_s": t_setup},
             "roofline": {"bound": "tensor", "achieved": whiten / t / 1e12, "peak": peak, "unit": "TFLOP/s",
                          "frac": whiten / t / 1e12 / peak,
-                         "note": "achieved counts the whitening 2·Σ M_k²·N; the split-BF16 GEMM executes 3x "
+                         "note": "achieved counts the triangular whitening Σ M_k (M_k + 1)·N; the split-BF16 GEMM executes 3x "
                                  "that, and the time includes the Mogi forward launch"},
             "llk_max_rel_err_vs_fp64": {"whitening": whiten_err, "chains": int(sub.numel()),
                                         "reference": "-1/2 |W r|^2 in FP64 (FP64 W = L^-1, the kernel's "
