@@ -962,7 +962,7 @@ def run_ours(args):
                    "population": N * world,
                    "step": "one annealing stage: COV beta + Sigma + resample, 5 Metropolis steps, scaling",
                    "l2": "flushed (256 MB write) between timed iterations",
-                   "graphs": "one CUDA graph per phase (cool, walk, resample)",
+                   "graphs": "one CUDA graph per stage (cool, walk, resample)",
                    "cdm_variant": model.variant, "autotune": model.tuning,
                    "beta_range": [reps[0]["beta"], reps[-1]["beta"]] if reps else None,
                    # proposals outside the prior or above the free surface are rejected without a
